@@ -24,80 +24,138 @@ static __device__ __align__(256) double g_sigma2_scratch[kNoAllocPart];
 std::mutex g_scratch_mu;
 double* g_scratch_ptr[64] = {nullptr};
 
-// Split-k partial sums of sig for a 64-row x 64-segment block: 256 threads, each a 4 x 4 register tile of float64
-// accumulators; per 32-bin step the block's |H|^2 (float64, exact from complex64) and IP tiles go through shared
-// memory (row stride 65 doubles: the transposing stores of 16 consecutive bins hit 16 distinct bank pairs), and the
-// next step's H and IP are loaded into registers while the current one is multiplied.
-constexpr int kSR = 64, kSS = 64, kSK = 32, kSP = kSK * kSR / 256;    // elements of each tile per thread
-__global__ void __launch_bounds__(256) sigma2_partial_kernel(const float2* __restrict__ H, long long ldh, int n,
+// Split-k partial sums of sig for a block of 64 rows x 8 NT segments on the float64 matrix instruction
+// (mma.m8n8k4.f64: products and sums in float64, as an FMA chain). Four warps, each 16 rows (two A fragments) x all
+// 8 NT segments; a chunk is 32 bins. A lane reads its rows' H straight from global memory in fragment order (8 rows x
+// 4 consecutive bins per load, a whole 32-byte sector each) one chunk ahead, forms |H|^2 in float64 (exact from
+// complex64) and feeds it as A; IP goes through shared memory once per chunk, converted to float64 for all four warps
+// (row stride 36 doubles: a fragment read hits 16 distinct bank pairs per half-warp).
+// Templates end at f_ISCO, so most chunks of a row are zero: a warp whose 16 x 32 values are all zero multiplies
+// nothing, unless the chunk's IP holds a value that is not finite (then 0 * inf must give the NaN it always gave).
+// NT is the smallest of 1, 2, 4, 8 that covers the segments: 64-wide blocks for one or a few segments did up to 64
+// times the work. Bound: reading H at few segments, the float64 pipe at many (36.9 TFLOP/s with
+// this instruction, 33.7 with FMAs, whose operands came from shared memory at 2.5 reads per FMA issue slot).
+// 256 templates x 524,289 bins, against the FMA kernel with 64 x 64 blocks that this replaces:
+//   1,790 -> 481 us at 16 segments, 3,970 -> 430 at 4; 1,980 -> 26 for 64 templates x 262,145 bins at one segment.
+constexpr int kSR = 64, kSK = 32, kSB = kSK + 4;
+
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+
+template <int NT>
+__global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __restrict__ H, long long ldh, int n,
                                                              const float* __restrict__ IP, long long ldip, int nseg,
                                                              int kmin, int flen, int kper,
                                                              double* __restrict__ part) {
-    __shared__ double Ps[kSK][kSR + 1];
-    __shared__ double Is[kSK][kSS + 1];
-    const int tid = threadIdx.x;
-    const int tr = tid >> 4, ts = tid & 15;         // rows 4 tr .. 4 tr + 3, segments 4 ts .. 4 ts + 3
-    const int r0 = blockIdx.x * kSR, s0 = blockIdx.y * kSS;
+    __shared__ double Bs[2][8 * NT * kSB];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int fr = lane >> 2, fk = lane & 3;          // fragment row (A) or segment (B), and bin
+    const int r0 = blockIdx.x * kSR + warp * 16, s0 = blockIdx.y * (8 * NT);
     const int ka = kmin + blockIdx.z * kper, kb = min(flen, ka + kper);
-    double acc[4][4];
+    const float2* h[2];
+    bool rok[2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int f = 0; f < 2; ++f) {
+        rok[f] = r0 + 8 * f + fr < n;
+        h[f] = H + (long long)(rok[f] ? r0 + 8 * f + fr : 0) * ldh + fk;
+    }
+    double acc[2][NT][2];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0.0;
-    // thread's load slots: element e = tid + 256 i, (row or segment) = e / kSK, bin = e % kSK (32 consecutive bins
-    // of one row per warp: coalesced)
-    float2 hv[kSP];
-    float iv[kSP];
+    for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) acc[f][j][0] = acc[f][j][1] = 0.0;
+    float2 hv[2][8];
+    float iv[2 * NT];
     auto load = [&](int k0) {
 #pragma unroll
-        for (int i = 0; i < kSP; ++i) {
-            const int e = tid + 256 * i, rr = e / kSK, kk = e % kSK;
-            const int row = r0 + rr, sg = s0 + rr, k = k0 + kk;
-            hv[i] = (row < n && k < kb) ? H[(long long)row * ldh + k] : make_float2(0.f, 0.f);
-            iv[i] = (sg < nseg && k < kb) ? IP[(long long)sg * ldip + k] : 0.f;
+        for (int f = 0; f < 2; ++f)
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                hv[f][e] = (rok[f] && k0 + 4 * e + fk < kb) ? __ldg(h[f] + k0 + 4 * e) : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 2 * NT; ++i) {            // 32 consecutive bins of one segment per warp
+            const int sg = s0 + warp + 4 * i, k = k0 + lane;
+            iv[i] = (sg < nseg && k < kb) ? __ldg(IP + (long long)sg * ldip + k) : 0.f;
         }
     };
     load(ka);
-    for (int k0 = ka; k0 < kb; k0 += kSK) {
-        __syncthreads();
+    int buf = 0;
+    for (int k0 = ka; k0 < kb; k0 += kSK, buf ^= 1) {
+        bool odd = false;
 #pragma unroll
-        for (int i = 0; i < kSP; ++i) {
-            const int e = tid + 256 * i, rr = e / kSK, kk = e % kSK;
-            Ps[kk][rr] = (double)hv[i].x * hv[i].x + (double)hv[i].y * hv[i].y;
-            Is[kk][rr] = (double)iv[i];
+        for (int i = 0; i < 2 * NT; ++i) {
+            Bs[buf][(warp + 4 * i) * kSB + lane] = (double)iv[i];
+            odd |= !(fabsf(iv[i]) <= 3.402823466e+38f);
         }
-        __syncthreads();
+        float2 hc[2][8];
+        bool any = false;
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                hc[f][e] = hv[f][e];
+                any |= hv[f][e].x != 0.f || hv[f][e].y != 0.f;
+            }
+        // the two buffers take turns: a warp that writes one has passed this barrier after everyone's last read of it
+        const int bad = __syncthreads_or(odd);
         if (k0 + kSK < kb) load(k0 + kSK);
-#pragma unroll 4
-        for (int kk = 0; kk < kSK; ++kk) {
-            double p[4], w[4];
+        if (!bad && !__any_sync(0xffffffffu, any)) continue;
 #pragma unroll
-            for (int a = 0; a < 4; ++a) p[a] = Ps[kk][4 * tr + a];
+        for (int e = 0; e < 8; ++e) {
+            double a[2];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) w[b] = Is[kk][4 * ts + b];
+            for (int f = 0; f < 2; ++f)
+                a[f] = (double)hc[f][e].x * hc[f][e].x + (double)hc[f][e].y * hc[f][e].y;
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
-#pragma unroll
-                for (int b = 0; b < 4; ++b) acc[a][b] = fma(p[a], w[b], acc[a][b]);
+            for (int j = 0; j < NT; ++j) {
+                const double b = Bs[buf][(8 * j + fr) * kSB + 4 * e + fk];
+                dmma884(acc[0][j], a[0], b);
+                dmma884(acc[1][j], a[1], b);
+            }
         }
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int f = 0; f < 2; ++f)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int row = r0 + 4 * tr + a, sg = s0 + 4 * ts + b;
-            if (row < n && sg < nseg) part[((long long)blockIdx.z * n + row) * nseg + sg] = acc[a][b];
-        }
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int row = r0 + 8 * f + fr, sg = s0 + 8 * j + 2 * fk + i;
+                if (row < n && sg < nseg) part[((long long)blockIdx.z * n + row) * nseg + sg] = acc[f][j][i];
+            }
 }
 
-__global__ void sigma2_reduce_kernel(const double* __restrict__ part, int nsplit, int n, int nseg, double scale,
-                                     double* __restrict__ sig, long long ldsig) {
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= (long long)n * nseg) return;
+// sig = scale times the sum of the partials: 32 consecutive elements x 16 interleaved runs of splits per block, the
+// runs added in order (the result does not depend on timing)
+__global__ void __launch_bounds__(512) sigma2_reduce_kernel(const double* __restrict__ part, int nsplit, int n,
+                                                            int nseg, double scale, double* __restrict__ sig,
+                                                            long long ldsig) {
+    __shared__ double red[16][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long ne = (long long)n * nseg, e = (long long)blockIdx.x * 32 + lane;
     double s = 0.0;
-    for (int z = 0; z < nsplit; ++z) s += part[(long long)z * n * nseg + e];
-    const long long row = e / nseg, sg = e % nseg;
-    sig[row * ldsig + sg] = scale * s;
+    if (e < ne) {
+#pragma unroll 8
+        for (int z = w; z < nsplit; z += 16) s += part[(long long)z * ne + e];
+    }
+    red[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && e < ne) {
+        s = red[0][lane];
+#pragma unroll
+        for (int i = 1; i < 16; ++i) s += red[i][lane];
+        sig[e / nseg * ldsig + e % nseg] = scale * s;
+    }
+}
+
+// Splits of the k range that fill the device: about eight CTAs of 64 rows per SM, 16 at least (the workspace that the
+// callers sized for the former kernel), 512 at most.
+int sigma2_splits(int n, int nseg) {
+    const long long blocks = cdiv(n, kSR) * cdiv(nseg, 64);
+    return (int)std::max(16ll, std::min(512ll, 8ll * 148 / blocks));
 }
 
 constexpr int kG = 32;   // Gram block: 32 x 32 outputs
@@ -276,20 +334,27 @@ int gwb_sigma2(const float* H, long long ldh, int n, const float* IP, long long 
     GWB_CHECK_ARG(H && IP && part && sig, GWB_ERR_ARG, "sigma2: null pointer");
     GWB_CHECK_ARG(n > 0 && nseg > 0 && flen > kmin && kmin >= 0 && ldsig >= nseg, GWB_ERR_SHAPE,
                   "sigma2: n=%d nseg=%d flen=%d kmin=%d", n, nseg, flen, kmin);
-    const int gx = (int)cdiv(n, kSR), gy = (int)cdiv(nseg, kSS);
-    int nsplit = (int)std::max(1ll, std::min<long long>(64, (4ll * num_sms()) / std::max(1, gx * gy)));
-    nsplit = (int)std::min<long long>(nsplit, part_elems / ((long long)n * nseg));
+    // fewer splits where the workspace holds no more
+    int nsplit = (int)std::min<long long>(sigma2_splits(n, nseg), part_elems / ((long long)n * nseg));
     GWB_CHECK_ARG(nsplit >= 1, GWB_ERR_SHAPE, "sigma2: workspace of %lld doubles is smaller than n*nseg", part_elems);
     const int kper = (int)(cdiv(cdiv(flen - kmin, nsplit), kSK) * kSK);
     nsplit = (int)cdiv(flen - kmin, kper);
     cudaStream_t s = (cudaStream_t)stream;
-    sigma2_partial_kernel<<<dim3(gx, gy, nsplit), 256, 0, s>>>(reinterpret_cast<const float2*>(H), ldh, n, IP, ldip, nseg,
-                                                                kmin, flen, kper, part);
+    const int nt = nseg <= 8 ? 1 : nseg <= 16 ? 2 : nseg <= 32 ? 4 : 8;
+    const dim3 grid((unsigned)cdiv(n, kSR), (unsigned)cdiv(nseg, 8 * nt), nsplit);
+    auto kern = nt == 1 ? sigma2_partial_kernel<1> : nt == 2 ? sigma2_partial_kernel<2>
+                : nt == 4 ? sigma2_partial_kernel<4> : sigma2_partial_kernel<8>;
+    kern<<<grid, 128, 0, s>>>(reinterpret_cast<const float2*>(H), ldh, n, IP, ldip, nseg, kmin, flen, kper, part);
     GWB_LAUNCH_CHECK("sigma2_partial_kernel");
-    const long long ne = (long long)n * nseg;
-    sigma2_reduce_kernel<<<(unsigned)cdiv(ne, 256), 256, 0, s>>>(part, nsplit, n, nseg, 4.0 * df, sig, ldsig);
+    sigma2_reduce_kernel<<<(unsigned)cdiv((long long)n * nseg, 32), 512, 0, s>>>(part, nsplit, n, nseg, 4.0 * df, sig,
+                                                                                ldsig);
     GWB_LAUNCH_CHECK("sigma2_reduce_kernel");
     return GWB_OK;
+}
+
+long long gwb_sigma2_part_elems(int n, int nseg) {
+    if (n <= 0 || nseg <= 0) return -1;
+    return (long long)n * nseg * gwb::sigma2_splits(n, nseg);
 }
 
 int gwb_sigma2_noalloc(const float* H, long long ldh, int n, const float* IP, long long ldip, int nseg, int kmin,

@@ -87,6 +87,7 @@ SIGNATURES = {
     'gwb_search_expand': [_P, _P, _P, _I, _LL, _I, _P, _I, _P, _P, _P, _P],
     'gwb_search_best': [_P, _I, _I, _P, _P],
     'gwb_sigma2': [_P, _LL, _I, _P, _LL, _I, _I, _I, _D, _P, _LL, _P, _LL, _P],
+    'gwb_sigma2_part_elems': [_I, _I],
     'gwb_sigma2_noalloc': [_P, _LL, _I, _P, _LL, _I, _I, _I, _D, _P, _LL, _P],
     'gwb_gram': [_P, _LL, _I, _P, _I, _I, _P, _LL, _P, _P],
     'gwb_eigh_jacobi_sweep': [_P, _P, _P, _I, _I, _I, _D, _D, _P, _P],
@@ -139,6 +140,7 @@ def load():
             f = getattr(lib, name)
             f.argtypes = args
             f.restype = ctypes.c_int
+        lib.gwb_sigma2_part_elems.restype = ctypes.c_longlong
         lib.gwb_consolidate_work_bytes.restype = ctypes.c_longlong
         lib.gwb_bin_sums_work_bytes.restype = ctypes.c_longlong
         lib.gwb_fused_peaks_cplx_work_bytes.restype = ctypes.c_longlong

@@ -282,7 +282,7 @@ class MatchedFilter:
         b = self.bank
         nseg = IP.shape[0]
         sig = torch.empty((b.M, nseg), dtype=torch.float64, device=IP.device)
-        part_elems = b.M * nseg * 16
+        part_elems = _lib.load().gwb_sigma2_part_elems(b.M, nseg)
         part = torch.empty(part_elems, dtype=torch.float64, device=IP.device)
         _lib.call('gwb_sigma2', _lib.ptr(b.H), b.H.stride(0), b.M, _lib.ptr(IP), _lib.row_stride(IP), nseg, b.kmin, b.flen,
                   float(b.df), _lib.ptr(part), part_elems, _lib.ptr(sig), sig.stride(0), _lib.stream_ptr())

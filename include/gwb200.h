@@ -218,7 +218,9 @@ GWB_API int gwb_taylorf2(const double* m1, const double* m2, const double* chi1,
                          const int32_t* kmax, int n, double df, int kmin, int flen, double f_ecc, float* H,
                          long long ldh, void* stream);
 /* Template norms (fp_filter.py:710-714) in float64: sig[i * ldsig + s] = 4 df sum_{k >= kmin} |H_ik|^2 IP_sk.
- * part: workspace of part_elems doubles (>= n * nseg; more allows more k-splits). */
+ * part: workspace of part_elems doubles (>= n * nseg; more allows more k-splits, up to
+ * gwb_sigma2_part_elems(n, nseg), the most it uses; -1 for a bad shape). */
+GWB_API long long gwb_sigma2_part_elems(int n, int nseg);
 GWB_API int gwb_sigma2(const float* H, long long ldh, int n, const float* IP, long long ldip, int nseg, int kmin,
                        int flen, double df, double* part, long long part_elems, double* sig, long long ldsig,
                        void* stream);
