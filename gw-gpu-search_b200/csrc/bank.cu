@@ -26,17 +26,17 @@ double* g_scratch_ptr[64] = {nullptr};
 
 // Split-k partial sums of sig for a block of 64 rows x 8 NT segments on the float64 matrix instruction
 // (mma.m8n8k4.f64: products and sums in float64, as an FMA chain). Four warps, each 16 rows (two A fragments) x all
-// 8 NT segments; a chunk is 32 bins. A lane reads its rows' H straight from global memory in fragment order (8 rows x
-// 4 consecutive bins per load, a whole 32-byte sector each) one chunk ahead, forms |H|^2 in float64 (exact from
-// complex64) and feeds it as A; IP goes through shared memory once per chunk, converted to float64 for all four warps
-// (row stride 36 doubles: a fragment read hits 16 distinct bank pairs per half-warp).
+// 8 NT segments; a chunk is 32 bins. A warp loads its rows' H one chunk ahead, 32 consecutive bins of a row per load
+// (loads in fragment order, 8 rows x 4 bins, reached 2.4 TB/s: 440 us at 16 segments, now 216, 5.0 TB/s), forms |H|^2 in float64 (exact from complex64) and
+// turns it to fragment order through its own shared tile; IP goes through shared memory once per chunk, converted to
+// float64 for all four warps (row stride 36 doubles: a fragment read hits 16 distinct bank pairs per half-warp).
 // Templates end at f_ISCO, so most chunks of a row are zero: a warp whose 16 x 32 values are all zero multiplies
 // nothing, unless the chunk's IP holds a value that is not finite (then 0 * inf must give the NaN it always gave).
 // NT is the smallest of 1, 2, 4, 8 that covers the segments: 64-wide blocks for one or a few segments did up to 64
 // times the work. Bound: reading H at few segments, the float64 pipe at many (36.9 TFLOP/s with
 // this instruction, 33.7 with FMAs, whose operands came from shared memory at 2.5 reads per FMA issue slot).
 // 256 templates x 524,289 bins, against the FMA kernel with 64 x 64 blocks that this replaces:
-//   1,790 -> 481 us at 16 segments, 3,970 -> 430 at 4; 1,980 -> 26 for 64 templates x 262,145 bins at one segment.
+//   1,770 -> 216 us at 16 segments, 3,970 -> 211 at 4; 1,980 -> 26 for 64 templates x 262,145 bins at one segment.
 constexpr int kSR = 64, kSK = 32, kSB = kSK + 4;
 
 __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
@@ -50,31 +50,26 @@ __global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __res
                                                              const float* __restrict__ IP, long long ldip, int nseg,
                                                              int kmin, int flen, int kper,
                                                              double* __restrict__ part) {
-    __shared__ double Bs[2][8 * NT * kSB];
+    extern __shared__ double s2_smem[];              // IP chunks [2][8 NT][kSB], then |H|^2 per warp [4][16][kSB]
+    double (*Bs)[8 * NT * kSB] = reinterpret_cast<double (*)[8 * NT * kSB]>(s2_smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int fr = lane >> 2, fk = lane & 3;          // fragment row (A) or segment (B), and bin
     const int r0 = blockIdx.x * kSR + warp * 16, s0 = blockIdx.y * (8 * NT);
     const int ka = kmin + blockIdx.z * kper, kb = min(flen, ka + kper);
-    const float2* h[2];
-    bool rok[2];
-#pragma unroll
-    for (int f = 0; f < 2; ++f) {
-        rok[f] = r0 + 8 * f + fr < n;
-        h[f] = H + (long long)(rok[f] ? r0 + 8 * f + fr : 0) * ldh + fk;
-    }
+    const float2* h = H + (long long)r0 * ldh + lane;
+    const int nr = min(16, n - r0);                   // rows of this warp (none or fewer at the edge)
+    double* A = s2_smem + 2 * 8 * NT * kSB + warp * 16 * kSB;
     double acc[2][NT][2];
 #pragma unroll
     for (int f = 0; f < 2; ++f)
 #pragma unroll
         for (int j = 0; j < NT; ++j) acc[f][j][0] = acc[f][j][1] = 0.0;
-    float2 hv[2][8];
+    float2 hv[16];
     float iv[2 * NT];
     auto load = [&](int k0) {
 #pragma unroll
-        for (int f = 0; f < 2; ++f)
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-                hv[f][e] = (rok[f] && k0 + 4 * e + fk < kb) ? __ldg(h[f] + k0 + 4 * e) : make_float2(0.f, 0.f);
+        for (int i = 0; i < 16; ++i)
+            hv[i] = (i < nr && k0 + lane < kb) ? __ldg(h + (long long)i * ldh + k0) : make_float2(0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < 2 * NT; ++i) {            // 32 consecutive bins of one segment per warp
             const int sg = s0 + warp + 4 * i, k = k0 + lane;
@@ -90,25 +85,24 @@ __global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __res
             Bs[buf][(warp + 4 * i) * kSB + lane] = (double)iv[i];
             odd |= !(fabsf(iv[i]) <= 3.402823466e+38f);
         }
-        float2 hc[2][8];
         bool any = false;
 #pragma unroll
-        for (int f = 0; f < 2; ++f)
+        for (int i = 0; i < 16; ++i) any |= hv[i].x != 0.f || hv[i].y != 0.f;
+        any = __any_sync(0xffffffffu, any);
+        if (any) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                hc[f][e] = hv[f][e];
-                any |= hv[f][e].x != 0.f || hv[f][e].y != 0.f;
-            }
+            for (int i = 0; i < 16; ++i)
+                A[i * kSB + lane] = (double)hv[i].x * hv[i].x + (double)hv[i].y * hv[i].y;
+        }
         // the two buffers take turns: a warp that writes one has passed this barrier after everyone's last read of it
         const int bad = __syncthreads_or(odd);
         if (k0 + kSK < kb) load(k0 + kSK);
-        if (!bad && !__any_sync(0xffffffffu, any)) continue;
+        if (!bad && !any) continue;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             double a[2];
 #pragma unroll
-            for (int f = 0; f < 2; ++f)
-                a[f] = (double)hc[f][e].x * hc[f][e].x + (double)hc[f][e].y * hc[f][e].y;
+            for (int f = 0; f < 2; ++f) a[f] = any ? A[(8 * f + fr) * kSB + 4 * e + fk] : 0.0;
 #pragma unroll
             for (int j = 0; j < NT; ++j) {
                 const double b = Bs[buf][(8 * j + fr) * kSB + 4 * e + fk];
@@ -116,6 +110,7 @@ __global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __res
                 dmma884(acc[1][j], a[1], b);
             }
         }
+        __syncwarp();                                 // the next chunk's |H|^2 goes over this one's
     }
 #pragma unroll
     for (int f = 0; f < 2; ++f)
@@ -344,7 +339,9 @@ int gwb_sigma2(const float* H, long long ldh, int n, const float* IP, long long 
     const dim3 grid((unsigned)cdiv(n, kSR), (unsigned)cdiv(nseg, 8 * nt), nsplit);
     auto kern = nt == 1 ? sigma2_partial_kernel<1> : nt == 2 ? sigma2_partial_kernel<2>
                 : nt == 4 ? sigma2_partial_kernel<4> : sigma2_partial_kernel<8>;
-    kern<<<grid, 128, 0, s>>>(reinterpret_cast<const float2*>(H), ldh, n, IP, ldip, nseg, kmin, flen, kper, part);
+    const size_t smem = (size_t)(2 * 8 * nt + 4 * 16) * kSB * sizeof(double);
+    GWB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<grid, 128, smem, s>>>(reinterpret_cast<const float2*>(H), ldh, n, IP, ldip, nseg, kmin, flen, kper, part);
     GWB_LAUNCH_CHECK("sigma2_partial_kernel");
     sigma2_reduce_kernel<<<(unsigned)cdiv((long long)n * nseg, 32), 512, 0, s>>>(part, nsplit, n, nseg, 4.0 * df, sig,
                                                                                 ldsig);
