@@ -4,9 +4,14 @@
 // has an fp16 GEMM, so this is the full-precision form that the mixed forms are compared against. CTA = 128 template
 // rows x one output group of `group` 128-sample blocks, walked block by block; 256 threads as 16 x 16, each thread
 // owning 8 rows x 8 samples for re and im (128 accumulators). K is staged through shared memory 16 at a time.
+#include <cooperative_groups.h>
+
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace gwb {
 namespace {
@@ -129,66 +134,105 @@ __global__ void __launch_bounds__(256) simt_absmax_kernel(const float* __restric
     }
 }
 
-// The same product with the operand tiles copied by cp.async through a ring of AS_ST stages, so the loads of the
-// next K tiles overlap the FMAs of this one (the kernel above loads and computes in turn). 16-byte copies: needs K,
-// lda and ldz multiples of 4 and 16-byte aligned operands (the launcher falls back to the kernel above otherwise).
-// Thread (tx, ty) owns rows ty + 16 i (i < 8) and samples 4 tx + j, 64 + 4 tx + j (j < 4): the A reads of a warp
+// The same product, packed and pipelined: the kernel that runs unless gwb_f32_set_async(0) asks for the one above.
+// It is bound by the fp32 pipe (128 FMA lanes per SM; 69 TFLOP/s measured with independent FMAs), and what kept the
+// one-FMA-per-instruction form at 35 TFLOP/s was the issue of everything else beside the FMAs with two warps per
+// scheduler. So:
+//  - FMAs go in pairs (fma.rn.f32x2: two samples of a row per instruction, each rounded as fmaf), which halves the
+//    issue slots they take and leaves the others for shared-memory reads and the duplicated A values;
+//  - operand tiles are copied by cp.async through a ring of AS_ST stages while earlier ones are multiplied (16-byte
+//    copies where K, lda, ldz and the bases allow, else 4-byte ones: the arithmetic is the same);
+//  - CTAs of 128 threads own 64 rows, two per SM, so one's barriers and epilogue pass under the other's FMAs and a
+//    row count is padded to 64, not 128;
+//  - a window is shared out over a cluster of SPL CTAs (each walks its part of the blocks; rank 0 merges the maxima
+//    in block order through distributed shared memory), so that the last wave is a quarter of a window long.
+// Sums run over k in order with one rounding per FMA, so results are bit-identical to the kernel above.
+// Measured, 248 x 192 by 192 x 458,700, 1 s windows: 2,526 -> 1,939 us (45 TFLOP/s); 64 templates x 118 rows of K by
+// 475,136 samples: 855 -> 430 us (half the rows were padding).
+// Thread (tx, ty) owns rows ty + 8 i (i < 8) and samples 4 tx + j, 64 + 4 tx + j (j < 4): the A reads of a warp
 // (two rows, one float4 each) fall in distinct banks, the Z reads are two runs of 256 contiguous bytes.
-constexpr int AS_ST = 3;
-constexpr int AS_STAGE = 3 * BM * BK;            // floats per stage: A re, A im (BM x BK, row-major), Z (BK x BN)
+constexpr int AS_ST = 3, AS_BM = 64, AS_NT = 128, AS_MAXSPL = 4;
+constexpr int AS_STAGE = (2 * AS_BM + BN) * BK;  // floats per stage: A re, A im (AS_BM x BK, row-major), Z (BK x BN)
 
-__device__ __forceinline__ void cp_async16_zfill(float* smem, const float* gmem, int src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(smem)),
-                 "l"(gmem), "r"(src_bytes)
-                 : "memory");
+// N bytes (16 or 4) to shared memory, zero past the first src_bytes
+template <int N>
+__device__ __forceinline__ void cp_async_zfill(float* smem, const float* gmem, int src_bytes) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+    if constexpr (N == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gmem), "r"(src_bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(gmem), "r"(src_bytes) : "memory");
 }
 
-__global__ void __launch_bounds__(256, 1) simt_absmax_async_kernel(
+using pair32 = unsigned long long;               // two floats, the lower one in the low word
+
+__device__ __forceinline__ pair32 dup(float a) {
+    pair32 r;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(a));
+    return r;
+}
+__device__ __forceinline__ void fma2(pair32& c, pair32 a, pair32 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float2 unpack(pair32 p) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+
+template <int SPL, bool VEC>
+__global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
     const float* __restrict__ Are, const float* __restrict__ Aim, long long lda, const float* __restrict__ Z,
     long long ldz, int M, int K, long long Tn, int ntiles, int group, float* __restrict__ V, int32_t* __restrict__ I,
     long long ldv) {
-    static_assert(BM == 128 && BN == 128 && BK == 16, "tile shape");
+    static_assert(BN == 128 && BK == 16 && AS_BM == 64 && AS_NT == 128, "tile shape");
     extern __shared__ __align__(16) float smf[];
+    __shared__ float s_best[AS_BM];
+    __shared__ int s_idx[AS_BM];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * BM;
-    const int o = blockIdx.x;
-    const int t0 = o * group, t1 = min(t0 + group, ntiles);
+    const int m0 = blockIdx.y * AS_BM;
+    const int o = blockIdx.x / SPL, rank = blockIdx.x % SPL;
+    // this CTA's blocks: its share of the window [o group, min(o group + group, ntiles)); the last ranks may have none
+    const int w0 = o * group, w1 = min(w0 + group, ntiles);
+    const int share = (group + SPL - 1) / SPL;
+    const int t0 = min(w0 + rank * share, w1), t1 = min(t0 + share, w1);
     const int nk = (K + BK - 1) / BK;
     const int nsteps = (t1 - t0) * nk;
     auto load = [&](int step) {
         float* sAr = smf + (step % AS_ST) * AS_STAGE;
-        float* sAi = sAr + BM * BK;
-        float* sZ = sAi + BM * BK;
+        float* sAi = sAr + AS_BM * BK;
+        float* sZ = sAi + AS_BM * BK;
         const int t = t0 + step / nk, k0 = (step % nk) * BK;
+        constexpr int E = VEC ? 4 : 1;           // elements per copy
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {            // A: 128 rows x 16 k, four k per copy
-            const int e = tid + 256 * r;
-            const int row = e >> 2, kq = (e & 3) * 4;
+        for (int r = 0; r < AS_BM * BK / E / AS_NT; ++r) {       // A: 64 rows x 16 k
+            const int e = tid + AS_NT * r;
+            const int row = e / (BK / E), kq = e % (BK / E) * E;
             const int gr = m0 + row, gk = k0 + kq;
             const bool ok = gr < M && gk < K;
             const long long off = ok ? (long long)gr * lda + gk : 0;
-            cp_async16_zfill(sAr + row * BK + kq, Are + off, ok ? 16 : 0);
-            cp_async16_zfill(sAi + row * BK + kq, Aim + off, ok ? 16 : 0);
+            cp_async_zfill<4 * E>(sAr + row * BK + kq, Are + off, ok ? 4 * E : 0);
+            cp_async_zfill<4 * E>(sAi + row * BK + kq, Aim + off, ok ? 4 * E : 0);
         }
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {            // Z: 16 k x 128 samples, four samples per copy
-            const int e = tid + 256 * r;
-            const int kk = e >> 5, cq = (e & 31) * 4;
+        for (int r = 0; r < BK * BN / E / AS_NT; ++r) {          // Z: 16 k x 128 samples
+            const int e = tid + AS_NT * r;
+            const int kk = e / (BN / E), cq = e % (BN / E) * E;
             const int gk = k0 + kk;
             const long long gc = (long long)t * BN + cq;
-            const int nb = (gk < K && gc < Tn) ? (int)min(16ll, (Tn - gc) * 4) : 0;
-            cp_async16_zfill(sZ + kk * BN + cq, Z + (nb ? (long long)gk * ldz + gc : 0), nb);
+            const int nb = (gk < K && gc < Tn) ? (int)min((long long)(4 * E), (Tn - gc) * 4) : 0;
+            cp_async_zfill<4 * E>(sZ + kk * BN + cq, Z + (nb ? (long long)gk * ldz + gc : 0), nb);
         }
     };
     float wb[8];
     int wi[8];
-    float ar[8][8], ai[8][8];
+    pair32 ar[8][4], ai[8][4];                   // samples (4 tx, +1), (+2, +3), (64 + 4 tx, +1), (+2, +3)
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        wb[i] = -1.f;
+        wb[i] = -2.f;                            // below every block's maximum (at least -1)
         wi[i] = 0;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ar[i][j] = ai[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) ar[i][j] = ai[i][j] = 0ull;
     }
 #pragma unroll
     for (int s = 0; s < AS_ST - 1; ++s) {
@@ -201,29 +245,29 @@ __global__ void __launch_bounds__(256, 1) simt_absmax_async_kernel(
         if (step + AS_ST - 1 < nsteps) load(step + AS_ST - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* sAr = smf + (step % AS_ST) * AS_STAGE;
-        const float* sAi = sAr + BM * BK;
-        const float* sZ = sAi + BM * BK;
+        const float* sAi = sAr + AS_BM * BK;
+        const float* sZ = sAi + AS_BM * BK;
 #pragma unroll
         for (int kq = 0; kq < BK; kq += 4) {
             float4 a4r[8], a4i[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                a4r[i] = *reinterpret_cast<const float4*>(sAr + (ty + 16 * i) * BK + kq);
-                a4i[i] = *reinterpret_cast<const float4*>(sAi + (ty + 16 * i) * BK + kq);
+                a4r[i] = *reinterpret_cast<const float4*>(sAr + (ty + 8 * i) * BK + kq);
+                a4i[i] = *reinterpret_cast<const float4*>(sAi + (ty + 8 * i) * BK + kq);
             }
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
-                const float4 z0 = *reinterpret_cast<const float4*>(sZ + (kq + kk) * BN + 4 * tx);
-                const float4 z1 = *reinterpret_cast<const float4*>(sZ + (kq + kk) * BN + 64 + 4 * tx);
-                const float z[8] = {z0.x, z0.y, z0.z, z0.w, z1.x, z1.y, z1.z, z1.w};
+                const ulonglong2 z0 = *reinterpret_cast<const ulonglong2*>(sZ + (kq + kk) * BN + 4 * tx);
+                const ulonglong2 z1 = *reinterpret_cast<const ulonglong2*>(sZ + (kq + kk) * BN + 64 + 4 * tx);
+                const pair32 z[4] = {z0.x, z0.y, z1.x, z1.y};
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const float a_r = kk == 0 ? a4r[i].x : kk == 1 ? a4r[i].y : kk == 2 ? a4r[i].z : a4r[i].w;
-                    const float a_i = kk == 0 ? a4i[i].x : kk == 1 ? a4i[i].y : kk == 2 ? a4i[i].z : a4i[i].w;
+                    const pair32 r2 = dup(kk == 0 ? a4r[i].x : kk == 1 ? a4r[i].y : kk == 2 ? a4r[i].z : a4r[i].w);
+                    const pair32 i2 = dup(kk == 0 ? a4i[i].x : kk == 1 ? a4i[i].y : kk == 2 ? a4i[i].z : a4i[i].w);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        ar[i][j] = fmaf(a_r, z[j], ar[i][j]);
-                        ai[i][j] = fmaf(a_i, z[j], ai[i][j]);
+                    for (int j = 0; j < 4; ++j) {
+                        fma2(ar[i][j], r2, z[j]);
+                        fma2(ai[i][j], i2, z[j]);
                     }
                 }
             }
@@ -238,14 +282,20 @@ __global__ void __launch_bounds__(256, 1) simt_absmax_async_kernel(
                 float best = -1.f;
                 int bi = 0;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int cc = (j < 4 ? 4 * tx + j : 64 + 4 * tx + (j - 4));
-                    const float p = (c0 + cc < Tn) ? fmaf(ar[i][j], ar[i][j], ai[i][j] * ai[i][j]) : -1.f;
-                    if (p > best) {
-                        best = p;
+                for (int j = 0; j < 4; ++j) {
+                    const float2 re = unpack(ar[i][j]), im = unpack(ai[i][j]);
+                    const int cc = (j < 2 ? 0 : 64) + 4 * tx + 2 * (j & 1);
+                    const float p0 = (c0 + cc < Tn) ? fmaf(re.x, re.x, im.x * im.x) : -1.f;
+                    const float p1 = (c0 + cc + 1 < Tn) ? fmaf(re.y, re.y, im.y * im.y) : -1.f;
+                    if (p0 > best) {
+                        best = p0;
                         bi = cc;
                     }
-                    ar[i][j] = ai[i][j] = 0.f;
+                    if (p1 > best) {
+                        best = p1;
+                        bi = cc + 1;
+                    }
+                    ar[i][j] = ai[i][j] = 0ull;
                 }
 #pragma unroll
                 for (int off = 8; off > 0; off >>= 1) {
@@ -253,25 +303,74 @@ __global__ void __launch_bounds__(256, 1) simt_absmax_async_kernel(
                     const int oi = __shfl_xor_sync(0xffffffffu, bi, off, 16);
                     better(ob, oi, best, bi);
                 }
-                const int gi = (int)(c0 + bi);
-                if (t == t0 || best > wb[i]) {
+                if (best > wb[i]) {
                     wb[i] = best;
-                    wi[i] = gi;
+                    wi[i] = (int)(c0 + bi);
                 }
             }
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (tx == 0) {
+    if constexpr (SPL > 1) {
+        // rank 0 takes the other ranks' maxima in block order (a later block replaces only where it is larger)
+        if (tx == 0) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                s_best[ty + 8 * i] = wb[i];
+                s_idx[ty + 8 * i] = wi[i];
+            }
+        }
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        if (rank == 0 && tid < AS_BM && m0 + tid < M) {
+            float b = s_best[tid];
+            int bi = s_idx[tid];
+#pragma unroll
+            for (int r = 1; r < SPL; ++r) {
+                const float ob = *cl.map_shared_rank(&s_best[tid], r);
+                const int oi = *cl.map_shared_rank(&s_idx[tid], r);
+                if (ob > b) {
+                    b = ob;
+                    bi = oi;
+                }
+            }
+            V[(long long)(m0 + tid) * ldv + o] = b;
+            I[(long long)(m0 + tid) * ldv + o] = bi;
+        }
+        cl.sync();                               // no CTA leaves while rank 0 may read its shared memory
+    } else if (tx == 0) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int row = m0 + ty + 16 * i;
+            const int row = m0 + ty + 8 * i;
             if (row < M) {
                 V[(long long)row * ldv + o] = wb[i];
                 I[(long long)row * ldv + o] = wi[i];
             }
         }
     }
+}
+
+template <int SPL, bool VEC>
+int launch_packed(const float* Are, const float* Aim, long long lda, const float* Z, long long ldz, int M, int K,
+                  long long Tn, int ntiles, int group, long long nout, float* V, int32_t* I, long long ldv,
+                  cudaStream_t stream) {
+    auto kern = simt_absmax_packed_kernel<SPL, VEC>;
+    const int smem = AS_ST * AS_STAGE * (int)sizeof(float);
+    GWB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nout * SPL), (unsigned)cdiv(M, AS_BM));
+    cfg.blockDim = dim3(AS_NT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = SPL;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = SPL > 1 ? 1 : 0;
+    GWB_CUDA(cudaLaunchKernelEx(&cfg, kern, Are, Aim, lda, Z, ldz, M, K, Tn, ntiles, group, V, I, ldv));
+    GWB_LAUNCH_CHECK("simt_absmax_packed_kernel");
+    return GWB_OK;
 }
 
 std::atomic<int> g_f32_async{1};   // 0: the synchronous kernel only (gwb_f32_set_async)
@@ -299,17 +398,24 @@ extern "C" int gwb_fused_peaks_f32(const float* Are, const float* Aim, long long
     const long long nout = cdiv(ntiles, group);
     GWB_CHECK_ARG(ldv >= nout, GWB_ERR_SHAPE, "fused_peaks_f32: ldv=%lld < outputs per row %lld", ldv, nout);
     GWB_CHECK_ARG(nout < (1ll << 31), GWB_ERR_SHAPE, "fused_peaks_f32: too many outputs");
-    dim3 grid((unsigned)nout, (unsigned)cdiv(M, BM));
-    const bool async = g_f32_async.load() && K % 4 == 0 && lda % 4 == 0 && ldz % 4 == 0 && aligned(Are, 16) &&
-                       aligned(Aim, 16) && aligned(Z, 16);
-    if (async) {
-        const int smem = AS_ST * AS_STAGE * (int)sizeof(float);
-        GWB_CUDA(cudaFuncSetAttribute(simt_absmax_async_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        simt_absmax_async_kernel<<<grid, 256, smem, (cudaStream_t)stream>>>(Are, Aim, lda, Z, ldz, M, K, Tn,
-                                                                            (int)ntiles, group, V, I, ldv);
-        GWB_LAUNCH_CHECK("simt_absmax_async_kernel");
-        return GWB_OK;
+    if (g_f32_async.load() && cdiv(M, AS_BM) <= 65535) {
+        const bool vec = K % 4 == 0 && lda % 4 == 0 && ldz % 4 == 0 && aligned(Are, 16) && aligned(Aim, 16) &&
+                         aligned(Z, 16);
+        // windows are shared out over clusters while whole windows would leave the last of few waves nearly empty
+        // (two CTAs per SM; from 32 waves on it is a thirty-second at most) and a part still holds two blocks
+        const long long items = nout * cdiv(M, AS_BM);
+        const int spl = items >= 32ll * 2 * num_sms() || nout * AS_MAXSPL >= (1ll << 31) ? 1 : group >= 8 ? 4 : group >= 4 ? 2 : 1;
+        auto go = [&](auto v) {
+            constexpr bool VEC = decltype(v)::value;
+            cudaStream_t st = (cudaStream_t)stream;
+            const int nt = (int)ntiles;
+            if (spl == 4) return launch_packed<4, VEC>(Are, Aim, lda, Z, ldz, M, K, Tn, nt, group, nout, V, I, ldv, st);
+            if (spl == 2) return launch_packed<2, VEC>(Are, Aim, lda, Z, ldz, M, K, Tn, nt, group, nout, V, I, ldv, st);
+            return launch_packed<1, VEC>(Are, Aim, lda, Z, ldz, M, K, Tn, nt, group, nout, V, I, ldv, st);
+        };
+        return vec ? go(std::true_type{}) : go(std::false_type{});
     }
+    dim3 grid((unsigned)nout, (unsigned)cdiv(M, BM));
     simt_absmax_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(Are, Aim, lda, Z, ldz, M, K, Tn, (int)ntiles, group, V,
                                                                 I, ldv);
     GWB_LAUNCH_CHECK("simt_absmax_kernel");
