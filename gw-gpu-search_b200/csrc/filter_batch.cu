@@ -143,22 +143,26 @@ int gwb_filter_batch(gwb_handle_t h, const float* x, long long ldx, int nseg, lo
     GWB_TRY(gwb_fft_r2c(h, w.frames, w.F, L, nseg * s.nfr, L, s.nb, st));
     GWB_TRY(gwb_welch_avg(w.F, s.nb, nseg, s.nfr, s.nb, dt, cond->median, median_bias(s.nfr),
                           welch_fac(cond->sr, L), w.psd_w, s.nb, st));
-    GWB_TRY(gwb_interp(w.psd_w, s.nb, nseg, s.nb, 1.0 / (1.0 / cond->sr) / (double)L, s.df, flen, w.psd, flen, st));
+    const double df_w = 1.0 / (1.0 / cond->sr) / (double)L;
+    const float sT = (float)(1.0 / (s.df * (double)n));
     if (cond->inv_len > 0) {
-        // inverse spectrum truncation to inv_len samples (optionally Hann-tapered)
+        // inverse spectrum truncation to inv_len samples (optionally Hann-tapered), then the segment rFFT with
+        // D = stilde / psd and IP = 1 / psd (gpu_stage2)
         if (cond->inv_taper) {
             hann_kernel<<<(unsigned)cdiv(cond->inv_len, 256), 256, 0, st>>>(w.tw, cond->inv_len);
             GWB_LAUNCH_CHECK("hann_kernel");
         }
-        GWB_TRY(gwb_ist_pre(w.psd, flen, nseg, flen, s.kmin, w.inv, flen, st));
+        GWB_TRY(gwb_interp_inv(w.psd_w, s.nb, nseg, s.nb, df_w, s.df, flen, s.kmin, w.inv, flen, st));
         GWB_TRY(gwb_fft_c2r(h, w.inv, w.q, n, nseg, flen, n, st));
         GWB_TRY(gwb_ist_mid(w.q, n, nseg, n, (float)s.df, cond->inv_len, cond->inv_taper ? w.tw : nullptr, st));
         GWB_TRY(gwb_fft_r2c(h, w.q, w.pt, n, nseg, n, flen, st));
-        GWB_TRY(gwb_ist_post(w.pt, flen, nseg, flen, (float)(1.0 / (s.df * (double)n)), w.psd, flen, st));
+        GWB_TRY(gwb_fft_r2c(h, x, w.st, n, nseg, ldx, flen, st));
+        GWB_TRY(gwb_ist_d_ip(w.pt, flen, nseg, flen, sT, w.psd, flen, w.st, flen, s.kmin, dt, D, flen, IP, flen, st));
+    } else {
+        GWB_TRY(gwb_interp(w.psd_w, s.nb, nseg, s.nb, df_w, s.df, flen, w.psd, flen, st));
+        GWB_TRY(gwb_fft_r2c(h, x, w.st, n, nseg, ldx, flen, st));
+        GWB_TRY(gwb_d_ip(w.st, flen, nseg, w.psd, flen, w.pick, flen, s.kmin, dt, D, flen, IP, flen, st));
     }
-    // segment rFFT, D = stilde / psd and IP = 1 / psd (gpu_stage2)
-    GWB_TRY(gwb_fft_r2c(h, x, w.st, n, nseg, ldx, flen, st));
-    GWB_TRY(gwb_d_ip(w.st, flen, nseg, w.psd, flen, w.pick, flen, s.kmin, dt, D, flen, IP, flen, st));
     // the filter step on the conditioned batch
     return gwb_filter_step(tiles, ntiles, H, ldh, M, kmax, nbins, s.kmin, s.df, D, IP, flen, flen, nseg, isw, tlen,
                            flen, cfg, base + head, work_bytes - (head + (base - reinterpret_cast<char*>(work))), cands,

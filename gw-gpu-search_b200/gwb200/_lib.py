@@ -97,6 +97,8 @@ SIGNATURES = {
     'gwb_frames': [_P, _LL, _I, _LL, _LL, _P, _I, _I, _P, _P, _LL, _P],
     'gwb_welch_avg': [_P, _LL, _I, _I, _I, _F, _I, _D, _F, _P, _LL, _P],
     'gwb_interp': [_P, _LL, _I, _I, _D, _D, _I, _P, _LL, _P],
+    'gwb_interp_inv': [_P, _LL, _I, _I, _D, _D, _I, _I, _P, _LL, _P],
+    'gwb_ist_d_ip': [_P, _LL, _I, _I, _F, _P, _LL, _P, _LL, _I, _F, _P, _LL, _P, _LL, _P],
     'gwb_ist_pre': [_P, _LL, _I, _I, _I, _P, _LL, _P],
     'gwb_ist_mid': [_P, _LL, _I, _I, _F, _I, _P, _P],
     'gwb_ist_post': [_P, _LL, _I, _I, _F, _P, _LL, _P],

@@ -523,21 +523,25 @@ class BatchConditioner:
         _lib.call('gwb_welch_avg', _lib.ptr(self.F), self.F.stride(0), nds, self.nfr, L // 2 + 1,
                   float(np.float32(1.0 / self.sr)), int(self.median), float(self.bias), self.fac, _lib.ptr(self.psd_w),
                   self.psd_w.stride(0), s)
-        _lib.call('gwb_interp', _lib.ptr(self.psd_w), self.psd_w.stride(0), nds, L // 2 + 1, float(self.pdf),
-                  float(self.df), flen, _lib.ptr(self.psd), flen, s)
-        self.launches += 3          # this library's kernels; the transforms are cuFFT's
-        P = self.psd
-        if self.mfl:
-            _lib.call('gwb_ist_pre', _lib.ptr(self.psd), flen, nds, flen, self.kmin, _lib.ptr(self.inv), flen, s)
-            _lib.call('gwb_fft_c2r', h, _lib.ptr(self.inv), _lib.ptr(self.q), n, nds, flen, n, s)
-            _lib.call('gwb_ist_mid', _lib.ptr(self.q), n, nds, n, float(np.float32(self.df)), self.mfl,
-                      _lib.ptr(self.tw), s)
-            _lib.call('gwb_fft_r2c', h, _lib.ptr(self.q), _lib.ptr(self.pt), n, nds, n, flen, s)
-            _lib.call('gwb_ist_post', _lib.ptr(self.pt), flen, nds, flen, float(np.float32(1.0 / (self.df * n))),
-                      _lib.ptr(self.psd), flen, s)
-            self.launches += 3
+        self.launches += 2          # this library's kernels; the transforms are cuFFT's
+        nb = L // 2 + 1
+        if not self.mfl:
+            _lib.call('gwb_interp', _lib.ptr(self.psd_w), self.psd_w.stride(0), nds, nb, float(self.pdf),
+                      float(self.df), flen, _lib.ptr(self.psd), flen, s)
+            _lib.call('gwb_fft_r2c', h, _lib.ptr(x), _lib.ptr(self.st), n, nds, n, flen, s)
+            _lib.call('gwb_d_ip', _lib.ptr(self.st), flen, nds, _lib.ptr(self.psd), flen, _lib.ptr(self.pick), flen,
+                      self.kmin, float(np.float32(1.0 / self.sr)), _lib.ptr(self.D), flen, _lib.ptr(self.IP), flen, s)
+            self.launches += 2
+            return self.D, self.IP
+        _lib.call('gwb_interp_inv', _lib.ptr(self.psd_w), self.psd_w.stride(0), nds, nb, float(self.pdf),
+                  float(self.df), flen, self.kmin, _lib.ptr(self.inv), flen, s)
+        _lib.call('gwb_fft_c2r', h, _lib.ptr(self.inv), _lib.ptr(self.q), n, nds, flen, n, s)
+        _lib.call('gwb_ist_mid', _lib.ptr(self.q), n, nds, n, float(np.float32(self.df)), self.mfl, _lib.ptr(self.tw),
+                  s)
+        _lib.call('gwb_fft_r2c', h, _lib.ptr(self.q), _lib.ptr(self.pt), n, nds, n, flen, s)
         _lib.call('gwb_fft_r2c', h, _lib.ptr(x), _lib.ptr(self.st), n, nds, n, flen, s)
-        _lib.call('gwb_d_ip', _lib.ptr(self.st), flen, nds, _lib.ptr(P), flen, _lib.ptr(self.pick), flen, self.kmin,
-                  float(np.float32(1.0 / self.sr)), _lib.ptr(self.D), flen, _lib.ptr(self.IP), flen, s)
-        self.launches += 1
+        _lib.call('gwb_ist_d_ip', _lib.ptr(self.pt), flen, nds, flen, float(np.float32(1.0 / (self.df * n))),
+                  _lib.ptr(self.psd), flen, _lib.ptr(self.st), flen, self.kmin, float(np.float32(1.0 / self.sr)),
+                  _lib.ptr(self.D), flen, _lib.ptr(self.IP), flen, s)
+        self.launches += 3
         return self.D, self.IP

@@ -180,7 +180,14 @@ GWB_API int gwb_interp(const float* psd, long long ldp, int rows, int nold, doub
 /* Inverse spectrum truncation around two real transforms (gpu_prep.inverse_spectrum_truncation, :138-158):
  * pre: out (complex) = sqrt(1/P) for kmin <= k < N/2, else 0;  [C2R of length N = 2 (flen - 1)]
  * mid: q *= df, Hann taper of max_filter_len/2 samples at each end when taper != NULL, zero q[ts:te];  [R2C]
- * post: out = 1 / |X scale|^2. */
+ * post: out = 1 / |X scale|^2.
+ * interp_inv: gwb_interp then pre without the PSD between them (the same values); ist_d_ip: post (into psd) then
+ * gwb_d_ip with segment s on row s, stilde = X_s sscale. */
+GWB_API int gwb_interp_inv(const float* psd, long long ldp, int rows, int nold, double df_old, double df_new, int flen,
+                           int kmin, float* out, long long ldo, void* stream);
+GWB_API int gwb_ist_d_ip(const float* X, long long ldx, int rows, int flen, float scale, float* psd, long long ldp,
+                         const float* stilde, long long ldst, int kmin, float sscale, float* D, long long ldd,
+                         float* IP, long long ldip, void* stream);
 GWB_API int gwb_ist_pre(const float* P, long long ldp, int rows, int flen, int kmin, float* out, long long ldo,
                         void* stream);
 GWB_API int gwb_ist_mid(float* q, long long ldq, int rows, int N, float df, int max_filter_len, const float* taper,
