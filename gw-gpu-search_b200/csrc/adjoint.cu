@@ -9,10 +9,9 @@
 //   chisq = (nb sum_j |z_j|^2 - |z|^2) / sigma^2 over nb equal-power bins (z_j the bin's part of z, edges from the
 //   cumulative |h|^2 IP as the pipeline's, held fixed), dof = 2 nb - 2, newsnr (coinc_rank.py:39-46).
 // |h_k| does not depend on theta (inside [kmin, kmax)), so d sigma = 0 and dz/dtheta_i = 4 df sum_k i dPhi_k/dtheta_i
-// conj(h_k) D_k. dPsi/d(Mc, q, chi1, chi2, e0) comes from forward-mode dual numbers through the phase formula in
-// float64; dPhi/dt_c = 2 pi f, dPhi/dphi_c = -1. The edges are found in the kernel (block scan of |h|^2 IP).
-// One CTA per trigger; each thread takes a contiguous range of bins, so a thread's bin changes a few times only and
-// its per-bin partial sums go to shared memory once per change.
+// conj(h_k) D_k. dPsi/d(Mc, q, chi1, chi2, e0) comes from forward-mode dual numbers through the phase formula (the
+// metric) or its coefficients in f (the gradient) in float64; dPhi/dt_c = 2 pi f, dPhi/dphi_c = -1. The edges are
+// found in the kernel (block scan of |h|^2 IP).
 //
 // The phase metric (the quadratic form of the phase-maximised match, 1 - m ~ dtheta^T g dtheta / 2): with |h|
 // independent of theta, g_ij = Cov_w(dPhi/dtheta_i, dPhi/dtheta_j), w_k = |h_k|^2 IP_k; the phi_c row is zero.
@@ -172,41 +171,106 @@ __device__ __forceinline__ int kmax_of(double Ms, double df, int flen) {
     return (int)min((long long)floor(fisco / df) + 1, (long long)flen - 1);
 }
 
+// ---- SNR and its gradient ----
+// In f alone the phase is linear in ten functions of frequency, whose coefficients hold all of theta: with u = f^(1/3),
+//   Psi(f) = sum_m C_m(theta) phi_m(f),  phi = u^-5, u^-3, u^-2, u^-1, 1, log f, u, u log f, u^2, u^(-34/3).
+// So dPsi/dtheta_p = sum_m dC_m/dtheta_p phi_m, and the sums over bins that the gradient needs are the moments
+// M_m = sum_k q_k phi_m(f_k), one per function (and one of f for t_c), contracted with dC_m/dtheta_p once per
+// chi-squared bin instead of a dual-number phase per (bin, parameter). All phi are products of w = f^(-1/18).
+constexpr int kNF = 10;                  // phase functions
+constexpr int kNM = kNF + 1;             // moments: the phase functions, then f
+constexpr int kOne = 4;                  // phi = 1: the moment is the bin's z
+constexpr int kWarps = kThreads / 32;
+constexpr int kTab = 2048;               // bins whose log f and w are kept from the edge pass
+constexpr int kChunk = kTab / kThreads;  // and the weights per thread that stay in registers
+
+// C_m and its derivatives (Dual) for m = lane; every lane runs the same code with its own power of pi Ms
+__device__ __forceinline__ Dual phase_function_coef(const PhaseCoef& P, int m) {
+    const Dual la = (1.0 / 3.0) * P.lms;                              // log a, v = a u
+    const double expo[kNF] = {-5.0, -3.0, -2.0, -1.0, 0.0, 0.0, 1.0, 1.0, 2.0, -34.0 / 3.0};
+    double ex = 0.0;
+#pragma unroll
+    for (int i = 0; i < kNF; ++i) ex = m == i ? expo[i] : ex;
+    Dual pw;                                                          // a^ex
+    pw.v = exp(ex * la.v);
+#pragma unroll
+    for (int i = 0; i < kNI; ++i) pw.d[i] = pw.v * ex * la.d[i];
+    const Dual p5 = P.p5c * (1.0 + 3.0 * (la - dc(log(0.4082482904638631))));
+    const Dual p6 = P.p6c - (6848.0 / 21.0) * (la + dc(log(4.0)));
+    Dual c = m == 0 ? dc(1.0) : m == 1 ? P.p2 : m == 2 ? P.p3 : m == 3 ? P.p4 : m == 4 ? p5 : m == 5 ? P.p5c
+             : m == 6 ? p6 : m == 7 ? dc(-6848.0 / 63.0) : m == 8 ? P.p7 : P.ecc;
+    return P.pre * pw * c;
+}
+
+// f^(-1/18) from log f; w^42 = f^(-7/3)
+__device__ __forceinline__ double root18(double lf) { return exp(lf * (-1.0 / 18.0)); }
+__device__ __forceinline__ double w_to_73(double w) {
+    const double w3 = w * w * w, iu = w3 * w3, iu3 = iu * iu * iu;
+    return iu3 * iu3 * iu;
+}
+
 // Equal-power edges of w_k = f^-7/3 IP_k over [kmin, k1): edge j = first k whose inclusive cumulative sum exceeds
-// (j / nb) total (the pipeline's edges, offset mode 0). Threads take contiguous ranges; float64 sums, block scan.
+// (j / nb) total (the pipeline's edges, offset mode 0). Threads take contiguous ranges; float64 sums, warp and block
+// scans. A band of at most kTab bins leaves log f and w in tab for the main pass.
 __device__ void block_edges(const float* __restrict__ ip, double df, int kmin, int k1, int nb, int* e, double* tot_out,
-                            double* scan) {
-    const int tid = threadIdx.x;
+                            double* scan, double2* tab) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int len = k1 - kmin, chunk = (len + kThreads - 1) / kThreads;
-    const int a = kmin + tid * chunk, b = min(a + chunk, k1);
-    double s = 0.0;
-    for (int k = a; k < b; ++k) s += pow((double)k * df, -7.0 / 3.0) * (double)ip[k];
-    scan[tid] = s;
-    __syncthreads();
-    if (tid == 0) {
-        double acc = 0.0;
-        for (int t = 0; t < kThreads; ++t) {
-            const double x = scan[t];
-            scan[t] = acc;          // exclusive prefix
-            acc += x;
+    const int a = min(kmin + tid * chunk, k1), b = min(a + chunk, k1);
+    const bool small = len <= kTab;
+    double wk[kChunk], s = 0.0;
+    if (small) {
+#pragma unroll
+        for (int i = 0; i < kChunk; ++i) {
+            wk[i] = 0.0;
+            if (a + i < b) {
+                const double lf = log((double)(a + i) * df), w = root18(lf);
+                tab[a + i - kmin] = make_double2(lf, w);
+                wk[i] = w_to_73(w) * (double)ip[a + i];
+                s += wk[i];
+            }
         }
-        scan[kThreads] = acc;
-        e[0] = kmin;
-        e[nb] = k1;
+    } else {
+        for (int k = a; k < b; ++k) s += w_to_73(root18(log((double)k * df))) * (double)ip[k];
     }
+    double inc = s;                                  // inclusive scan of the threads' sums
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const double v = __shfl_up_sync(0xffffffffu, inc, off);
+        if (lane >= off) inc += v;
+    }
+    if (lane == 31) scan[kThreads + 1 + warp] = inc;
+    for (int j = tid; j <= nb; j += kThreads) e[j] = j == 0 ? kmin : k1;
     __syncthreads();
-    const double tot = scan[kThreads], ex = scan[tid];
+    double base = 0.0;
+    for (int w = 0; w < warp; ++w) base += scan[kThreads + 1 + w];
+    scan[tid + 1] = base + inc;
+    if (tid == 0) scan[0] = 0.0;
+    __syncthreads();
+    const double tot = scan[kThreads], ex = scan[tid], hi = scan[tid + 1];
     for (int j = 1; j < nb; ++j) {
         const double target = (double)j / (double)nb * tot;
-        if (ex <= target && target < ex + s) {
+        if (ex <= target && target < hi) {
             double c = ex;
-            for (int k = a; k < b; ++k) {
-                c += pow((double)k * df, -7.0 / 3.0) * (double)ip[k];
-                if (c > target) {
-                    e[j] = k;
-                    break;
+            int at = b - 1;                          // the last bin's sum is hi (to rounding)
+            if (small) {
+#pragma unroll
+                for (int i = kChunk - 1; i >= 0; --i) {
+                    double ci = ex;
+#pragma unroll
+                    for (int x = 0; x <= i; ++x) ci += wk[x];
+                    if (a + i < b && ci > target) at = a + i;
+                }
+            } else {
+                for (int k = a; k < b; ++k) {
+                    c += w_to_73(root18(log((double)k * df))) * (double)ip[k];
+                    if (c > target) {
+                        at = k;
+                        break;
+                    }
                 }
             }
+            e[j] = at;
         }
     }
     if (tid == 0) *tot_out = tot;
@@ -216,98 +280,165 @@ __device__ void block_edges(const float* __restrict__ ip, double df, int kmin, i
 // out row layout (doubles): snr, newsnr, chisq, sigma2, z_re, z_im, kmax, dsnr[7], dnewsnr[7], dchisq[7]
 constexpr int kOut = 7 + 3 * kNP;
 
+// One CTA per trigger. The band is cut into one contiguous run per warp; a lane's bins are 32 apart (coalesced D and
+// IP), and at every chi-squared edge the warp adds its 22 sums over the lanes (a halving exchange: 31 shuffles of a
+// double, against 110 for 22 trees) and stores them with the edge bin they belong to. Bound: the float64 pipe (log and
+// exp of the edge pass, then about 50 operations per bin). The former kernel took a barrier and a block reduction per
+// chi-squared bin, in which 256 threads share the 20 to 200 bins of 16 s of data, and a dual-number phase with three
+// exp and two pow per frequency bin: 803 -> 203 us for 2,048 triggers of 16 s, float32.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) snr_grad_kernel(const double* __restrict__ params, int n,
-                                                          const float2* __restrict__ D, long long ldd,
-                                                          const float* __restrict__ IP, long long ldip, int flen,
-                                                          double df, int kmin, double f_ecc, int nb,
-                                                          double* __restrict__ out, long long ldout) {
+__global__ void __launch_bounds__(kThreads, 2) snr_grad_kernel(const double* __restrict__ params, int n,
+                                                             const float2* __restrict__ D, long long ldd,
+                                                             const float* __restrict__ IP, long long ldip, int flen,
+                                                             double df, int kmin, double f_ecc, int nb,
+                                                             double* __restrict__ out, long long ldout) {
     const int i = blockIdx.x;
     if (i >= n) return;
-    __shared__ double scan[kThreads + 1];
+    constexpr int kNS = 2 * kNM;
+    constexpr int kSeg = kMaxBins + kWarps;            // (warp, bin) runs: warp + bin never repeats along the band
+    __shared__ double scan[kThreads + 1 + kWarps];
     __shared__ int e[kMaxBins + 1];
     __shared__ double tot;
+    __shared__ double C[kNF][1 + kNI];
+    __shared__ int owner[kSeg];
+    __shared__ double seg[kSeg][kNS];
+    __shared__ double2 tab[kTab];
     __shared__ double acc[kMaxBins][2 + 2 * kNP];      // per bin: z_j (re, im), dz_j (re, im) x 7
-    __shared__ double red[kThreads / 32][2 + 2 * kNP];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const double* th = params + (long long)i * kNP;
-    const PhaseCoef P = phase_coef(th, f_ecc);
-    const double tc = th[5], phic = th[6];
-    const int k1 = kmax_of(P.Ms, df, flen);
+    // the end bin from the same operations as phase_coef's value of Ms
+    const double q1 = 1.0 + th[1], eta = th[1] / (q1 * q1);
+    const int k1 = kmax_of(kMsun * (th[0] * pow(eta, -0.6)), df, flen);
     if (k1 <= kmin + kThreads) {           // no band above kmin (f_ISCO below the low cut): nothing to filter
-        if (threadIdx.x < kOut) out[(long long)i * ldout + threadIdx.x] = 0.0;
+        if (tid < kOut) out[(long long)i * ldout + tid] = 0.0;
         return;
     }
     const float* ip = IP + (long long)i * ldip;
     const float2* d = D + (long long)i * ldd;
-    block_edges(ip, df, kmin, k1, nb, e, &tot, scan);
-    // main pass, bin by bin: threads stride over the bin's range (coalesced D and IP), then a fixed-order block
-    // reduction (warp shuffles, then the warps in order) gives the bin's sums: the result does not depend on timing
-    constexpr int kNS = 2 + 2 * kNP;
-    for (int j = 0; j < nb; ++j) {
-        T s[kNS];
+    if (tid < kSeg) owner[tid] = -1;
+    if (warp == kWarps - 1) {
+        const PhaseCoef P = phase_coef(th, f_ecc);
+        const Dual c = phase_function_coef(P, min(lane, kNF - 1));
+        if (lane < kNF) {
+            C[lane][0] = c.v;
 #pragma unroll
-        for (int x = 0; x < kNS; ++x) s[x] = T(0);
-        for (int k = e[j] + threadIdx.x; k < e[j + 1]; k += kThreads) {
-            const double f = (double)k * df;
-            const Dual ps = psi_at(P, f);
-            double ph = ps.v - 0.25 * kPi + 2.0 * kPi * f * tc - phic;
-            ph -= 2.0 * kPi * rint(ph * (0.5 / kPi));
-            T sn, cs;
-            if constexpr (sizeof(T) == 8) {
-                sincos(ph, &sn, &cs);
-            } else {
-                sincosf((float)ph, &sn, &cs);
-            }
-            const T amp = (T)pow(f, -7.0 / 6.0);
-            const float2 dk = d[k];
-            // q = conj(h) D = amp e^{+i ph} D
-            const T hr = amp * cs, hi = amp * sn;
-            const T qr = hr * (T)dk.x - hi * (T)dk.y, qi = hr * (T)dk.y + hi * (T)dk.x;
-            s[0] += qr;
-            s[1] += qi;
-            // d q / d theta_p = i dPhi_p q
-            T dph[kNP];
-#pragma unroll
-            for (int p = 0; p < kNI; ++p) dph[p] = (T)ps.d[p];
-            dph[5] = (T)(2.0 * kPi * f);
-            dph[6] = T(-1);
-#pragma unroll
-            for (int p = 0; p < kNP; ++p) {
-                s[2 + 2 * p] -= dph[p] * qi;
-                s[3 + 2 * p] += dph[p] * qr;
-            }
+            for (int p = 0; p < kNI; ++p) C[lane][1 + p] = c.d[p];
         }
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-        for (int x = 0; x < kNS; ++x) {
-            double v = (double)s[x];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-            if (lane == 0) red[warp][x] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < kNS) {
-            double v = 0.0;
-            for (int w = 0; w < kThreads / 32; ++w) v += red[w][threadIdx.x];
-            acc[j][threadIdx.x] = v;
-        }
-        __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        const double c4 = 4.0 * df;
-        const double sig2 = c4 * tot;
-        double zr = 0.0, zi = 0.0, dzr[kNP] = {0}, dzi[kNP] = {0}, pw = 0.0, dpw[kNP] = {0};
+    block_edges(ip, df, kmin, k1, nb, e, &tot, scan, tab);   // ends with a barrier
+    {
+        double cv[kNF];
+#pragma unroll
+        for (int m = 0; m < kNF; ++m) cv[m] = C[m][0];
+        cv[kOne] -= 0.25 * kPi + th[6];
+        const double wtc = 2.0 * kPi * th[5];
+        const bool have = k1 - kmin <= kTab;
+        const int run = ((k1 - kmin + kThreads - 1) / kThreads) * 32;    // bins per warp, whole rounds of 32 lanes
+        const int A = min(kmin + warp * run, k1), B = min(A + run, k1);
         for (int j = 0; j < nb; ++j) {
-            const double ar = c4 * acc[j][0], ai = c4 * acc[j][1];
+            const int lo = max(e[j], A), hi = min(e[j + 1], B);
+            if (lo >= hi) continue;                                      // warp-uniform
+            double s[kNS];
+#pragma unroll
+            for (int x = 0; x < kNS; ++x) s[x] = 0.0;
+            for (int k = lo + lane; k < hi; k += 32) {
+                const double f = (double)k * df;
+                double lf, w;
+                if (have) {
+                    const double2 t = tab[k - kmin];
+                    lf = t.x;
+                    w = t.y;
+                } else {
+                    lf = log(f);
+                    w = root18(lf);
+                }
+                const double w2 = w * w, w3 = w2 * w, iu = w3 * w3, iu2 = iu * iu, iu3 = iu2 * iu, iu5 = iu3 * iu2;
+                const double u = f * iu2;
+                const double phi[kNM] = {iu5, iu3, iu2, iu, 1.0, lf, u, u * lf, f * iu, iu5 * iu5 * iu * w2, f};
+                double ph = cv[kOne] + wtc * f;
+#pragma unroll
+                for (int m = 0; m < kNF; ++m)
+                    if (m != kOne) ph = fma(cv[m], phi[m], ph);
+                ph -= 2.0 * kPi * rint(ph * (0.5 / kPi));
+                T sn, cs;
+                if constexpr (sizeof(T) == 8) {
+                    sincos(ph, &sn, &cs);
+                } else {
+                    sincosf((float)ph, &sn, &cs);
+                }
+                const T amp = (T)(iu3 * w3);                             // f^(-7/6)
+                const float2 dk = d[k];
+                // q = conj(h) D = amp e^{+i ph} D
+                const T hr = amp * cs, hi2 = amp * sn;
+                const double qr = (double)(hr * (T)dk.x - hi2 * (T)dk.y), qi = (double)(hr * (T)dk.y + hi2 * (T)dk.x);
+#pragma unroll
+                for (int m = 0; m < kNM; ++m) {
+                    s[2 * m] = fma(qr, phi[m], s[2 * m]);
+                    s[2 * m + 1] = fma(qi, phi[m], s[2 * m + 1]);
+                }
+            }
+            // lane x ends with the warp's sum of s[x]: each exchange halves the values a lane holds
+            double v[16];
+            {
+                const bool up = lane & 16;
+#pragma unroll
+                for (int x = 0; x < 16; ++x) {
+                    const double a = s[x], b = x + 16 < kNS ? s[x + 16 < kNS ? x + 16 : 0] : 0.0;
+                    v[x] = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+                }
+            }
+#pragma unroll
+            for (int h = 8; h >= 1; h >>= 1) {
+                const bool up = lane & h;
+#pragma unroll
+                for (int x = 0; x < h; ++x)
+                    v[x] = (up ? v[x + h] : v[x]) + __shfl_xor_sync(0xffffffffu, up ? v[x] : v[x + h], h);
+            }
+            if (lane < kNS) seg[warp + j][lane] = v[0];
+            if (lane == 0) owner[warp + j] = j;
+        }
+    }
+    __syncthreads();
+    // per (bin, value): the bin's runs in band order, then the contraction with dC / dtheta
+    const double c4 = 4.0 * df;
+    for (int x = tid; x < nb * (1 + kNP); x += kThreads) {
+        const int j = x / (1 + kNP), p = x % (1 + kNP) - 1;
+        double re = 0.0, im = 0.0;
+        for (int w = 0; w < kWarps; ++w) {
+            if (owner[j + w] != j) continue;
+            const double* M = seg[j + w];
+            if (p < 0) {
+                re += M[2 * kOne];
+                im += M[2 * kOne + 1];
+            } else if (p < kNI) {
+#pragma unroll
+                for (int m = 0; m < kNF; ++m) {
+                    re = fma(-C[m][1 + p], M[2 * m + 1], re);
+                    im = fma(C[m][1 + p], M[2 * m], im);
+                }
+            } else {
+                const int m = p == 5 ? kNF : kOne;
+                const double g = p == 5 ? 2.0 * kPi : -1.0;
+                re -= g * M[2 * m + 1];
+                im += g * M[2 * m];
+            }
+        }
+        acc[j][2 * (p + 1)] = c4 * re;
+        acc[j][2 * (p + 1) + 1] = c4 * im;
+    }
+    __syncthreads();
+    if (tid < kNP) {                                   // thread p: the outputs of parameter p (thread 0: the values too)
+        const int p = tid;
+        const double sig2 = c4 * tot;
+        double zr = 0.0, zi = 0.0, pw = 0.0, dzr = 0.0, dzi = 0.0, dpw = 0.0;
+        for (int j = 0; j < nb; ++j) {
+            const double ar = acc[j][0], ai = acc[j][1], br = acc[j][2 + 2 * p], bi = acc[j][3 + 2 * p];
             zr += ar;
             zi += ai;
             pw += ar * ar + ai * ai;
-            for (int p = 0; p < kNP; ++p) {
-                const double br = c4 * acc[j][2 + 2 * p], bi = c4 * acc[j][3 + 2 * p];
-                dzr[p] += br;
-                dzi[p] += bi;
-                dpw[p] += 2.0 * (ar * br + ai * bi);
-            }
+            dzr += br;
+            dzi += bi;
+            dpw += 2.0 * (ar * br + ai * bi);
         }
         const double az = sqrt(zr * zr + zi * zi), sg = sqrt(sig2);
         const double snr = az / sg;
@@ -322,21 +453,21 @@ __global__ void __launch_bounds__(kThreads) snr_grad_kernel(const double* __rest
             ns = snr * g;
         }
         double* o = out + (long long)i * ldout;
-        o[0] = snr;
-        o[1] = ns;
-        o[2] = chisq;
-        o[3] = sig2;
-        o[4] = zr;
-        o[5] = zi;
-        o[6] = (double)k1;
-        for (int p = 0; p < kNP; ++p) {
-            const double dabs = az > 0.0 ? (zr * dzr[p] + zi * dzi[p]) / az : 0.0;
-            const double dsnr = dabs / sg;
-            const double dchi = ((double)nb * dpw[p] - 2.0 * az * dabs) / sig2;
-            o[7 + p] = dsnr;
-            o[7 + kNP + p] = dsnr * g + snr * gp * dchi / (double)dof;
-            o[7 + 2 * kNP + p] = dchi;
+        if (p == 0) {
+            o[0] = snr;
+            o[1] = ns;
+            o[2] = chisq;
+            o[3] = sig2;
+            o[4] = zr;
+            o[5] = zi;
+            o[6] = (double)k1;
         }
+        const double dabs = az > 0.0 ? (zr * dzr + zi * dzi) / az : 0.0;
+        const double dsnr = dabs / sg;
+        const double dchi = ((double)nb * dpw - 2.0 * az * dabs) / sig2;
+        o[7 + p] = dsnr;
+        o[7 + kNP + p] = dsnr * g + snr * gp * dchi / (double)dof;
+        o[7 + 2 * kNP + p] = dchi;
     }
 }
 
