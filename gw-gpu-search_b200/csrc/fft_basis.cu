@@ -465,6 +465,12 @@ __global__ void rowscale_kernel(const float* __restrict__ rowpart, int P, float*
     }
 }
 
+// Where 1 / scale enters pass 2: folded into the step-1 twiddles for the shorter transforms; at the store for N2 = 1024
+// (N = 2^20), where the persistent ring form and the 8- and 16-column kernels all give the same bits of Z. fp8 has one
+// scale per row, always at the store.
+template <int N2, int FORM>
+constexpr bool kFold = N2 != 1024 && FORM != 4;
+
 template <int FORM>
 __device__ __forceinline__ void store_z(void* Zr, void* Zi, void* Zlr, void* Zli, int t, float xr, float xi) {
     if constexpr (FORM == 0) {
@@ -501,9 +507,8 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT) basis_pass2(
     float2* twL = Y + TB * SC;
     const int row = blockIdx.y, t10 = blockIdx.x * TB, tid = threadIdx.x;
     const int stride = N / N2;
-    // 1 / scale: folded into the step-1 twiddles (one rms per call), applied per row at the store for fp8
     const float inv = 1.0f / (FORM == 4 ? scale[row] : *scale);
-    const float tsc = FORM == 4 ? 1.f : inv, zsc = FORM == 4 ? inv : 1.f;
+    const float tsc = kFold<N2, FORM> ? inv : 1.f, zsc = kFold<N2, FORM> ? 1.f : inv;
     for (int m = tid; m < N2; m += NT) {
         const float2 w = tw[m * stride];
         twL[m] = make_float2(w.x * tsc, w.y * tsc);
@@ -543,7 +548,7 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT) basis_pass2(
             const int t = t0 + N1 * (R1 * vv);
             if (t >= 0 && t < Tn) {
                 const float2 z = y[brev(vv, ilog2(R2))];
-                if constexpr (FORM == 4) store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x * zsc, z.y * zsc);
+                if constexpr (!kFold<N2, FORM>) store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x * zsc, z.y * zsc);
                 else store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x, z.y);
             }
         });
@@ -577,8 +582,7 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT, 2) basis_pass2_p(
         cp_async_commit();
     };
     fetch(j0);
-    // 1 / scale folded into the step-1 twiddles; fp8: scale holds one scale per row, applied at the store
-    const float inv0 = FORM == 4 ? 1.f : 1.0f / *scale;
+    const float invs = FORM == 4 ? 1.f : 1.0f / *scale, inv0 = kFold<N2, FORM> ? invs : 1.f;
     for (int e = tid; e < N2; e += NT) {
         const float2 w = tw[(e % R2) * (e / R2) * (N / N2)];
         tw2[e] = make_float2(w.x * inv0, w.y * inv0);
@@ -587,7 +591,7 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT, 2) basis_pass2_p(
     char* zb = static_cast<char*>(Z);
     char* zl = static_cast<char*>(Zlo);
     for (int j = j0; j < j1; ++j) {
-        const float inv = FORM == 4 ? 1.0f / scale[j] : 1.f;
+        const float inv = FORM == 4 ? 1.0f / scale[j] : invs;
         cp_async_wait_all();
         __syncthreads();
         float2 x[R1];
@@ -626,7 +630,7 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT, 2) basis_pass2_p(
                 const int t = t0 + N1 * (R1 * vv);
                 if (t >= 0 && t < Tn) {
                     const float2 z = y[p][brev(vv, ilog2(R2))];
-                    if constexpr (FORM == 4) store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x * inv, z.y * inv);
+                    if constexpr (!kFold<N2, FORM>) store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x * inv, z.y * inv);
                     else store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x, z.y);
                 }
             });
@@ -718,7 +722,7 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
     static_assert(!PAIR || FORM != 4, "fp8 Z is stored per sample");
     extern __shared__ float2 sm[];
     float2* Bt = sm;                              // W tile (two blocks of TB columns), then the exchange tile
-    float2* tw2 = Bt + TBW * SC;                  // tw2[u R2 + b] = e^{2 pi i b u / N2} / scale
+    float2* tw2 = Bt + TBW * SC;                  // tw2[u R2 + b] = e^{2 pi i b u / N2}
     const int tid = threadIdx.x, t10 = blockIdx.x * TBW;
     const int j0 = blockIdx.y * RC, j1 = min(j0 + RC, rows);
     auto fetch = [&](int j) {
@@ -729,12 +733,9 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
         cp_async_commit();
     };
     fetch(j0);
-    // 1 / scale folded into the step-1 twiddles; fp8: scale holds one scale per row, applied at the store
+    // at the store: two products of 60 instructions per sample
     const float inv0 = FORM == 4 ? 1.f : 1.0f / *scale;
-    for (int e = tid; e < N2; e += NT) {
-        const float2 w = tw[(e % R2) * (e / R2) * (N / N2)];
-        tw2[e] = make_float2(w.x * inv0, w.y * inv0);
-    }
+    for (int e = tid; e < N2; e += NT) tw2[e] = tw[(e % R2) * (e / R2) * (N / N2)];
     const int c = (tid & 7) + 8 * ((tid >> 4) & 1);
     const int lo = (tid >> 3) & 1, hi = tid >> 5;
     const int b = lo + 2 * hi;                    // step 1: b < R2
@@ -754,7 +755,7 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
     char* zb = static_cast<char*>(Z);
     char* zl = static_cast<char*>(Zlo);
     for (int j = j0; j < j1; ++j) {
-        const float inv = FORM == 4 ? 1.0f / scale[j] : 1.f;
+        const float inv = FORM == 4 ? 1.0f / scale[j] : inv0;
         cp_async_wait_all();
         __syncthreads();
         float2 x[R1];
@@ -781,7 +782,7 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
                 constexpr int vv = decltype(V)::value;
                 constexpr int K = N1 * R1 * vv / 2;    // pair index of vv (64-bit pairs for fp32: same count)
                 const float2 z = y[brev(vv, ilog2(R2))];
-                ps.template store<K>(z.x, z.y, ph, pl, (vmask >> vv) & 1u);
+                ps.template store<K>(z.x * inv, z.y * inv, ph, pl, (vmask >> vv) & 1u);
             });
         } else {
             const long long re_off = (long long)(row0 + j) * ldz * ES, im_off_b = (long long)(im_off + row0 + j) * ldz * ES;
