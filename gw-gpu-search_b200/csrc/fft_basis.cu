@@ -465,6 +465,37 @@ __global__ void rowscale_kernel(const float* __restrict__ rowpart, int P, float*
     }
 }
 
+// FORM 5 of the pass-2 kernels stores nothing and sums |z|^2 over the analysed samples (unscaled): one double per CTA,
+// added up in a fixed order by power_scale_kernel. The reference's scale is that rms over its first batch of rows.
+constexpr int kPower = 5;
+template <int NT>
+__device__ __forceinline__ void power_partial(double acc, double* __restrict__ partials) {
+    __shared__ double red[NT / 32];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < NT / 32; ++w) s += red[w];
+        partials[(long long)blockIdx.y * gridDim.x + blockIdx.x] = s;
+    }
+}
+__global__ void __launch_bounds__(256) power_scale_kernel(const double* __restrict__ partials, int n, double count,
+                                                          float* __restrict__ scale) {
+    __shared__ double red[8];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < n; i += 256) s += partials[i];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) s += red[w];
+        *scale = (float)sqrt(s / count / 2.0);
+    }
+}
+
 // Where 1 / scale enters pass 2: folded into the step-1 twiddles for the shorter transforms; at the store for N2 = 1024
 // (N = 2^20), where the persistent ring form and the 8- and 16-column kernels all give the same bits of Z. fp8 has one
 // scale per row, always at the store.
@@ -498,7 +529,7 @@ template <int N2, int FORM>
 __global__ void __launch_bounds__(Split<N2, 2>::NT) basis_pass2(
     const float2* __restrict__ W, int N, int N1, const float2* __restrict__ tw, int a0, int Tn,
     const float* __restrict__ scale, void* __restrict__ Z, void* __restrict__ Zlo, long long ldz, int im_off,
-    int row0) {
+    int row0, double* __restrict__ partials) {
     using S = Split<N2, 2>;
     constexpr int R1 = S::R1, R2 = S::R2, NT = S::NT, SB = S::SB, SC = S::SC;
     constexpr int ES = FORM == 1 ? 4 : (FORM == 4 ? 1 : 2);   // bytes per Z element
@@ -507,7 +538,8 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT) basis_pass2(
     float2* twL = Y + TB * SC;
     const int row = blockIdx.y, t10 = blockIdx.x * TB, tid = threadIdx.x;
     const int stride = N / N2;
-    const float inv = 1.0f / (FORM == 4 ? scale[row] : *scale);
+    const float inv = FORM == kPower ? 1.0f : 1.0f / (FORM == 4 ? scale[row] : *scale);
+    float power = 0.f;
     const float tsc = kFold<N2, FORM> ? inv : 1.f, zsc = kFold<N2, FORM> ? 1.f : inv;
     for (int m = tid; m < N2; m += NT) {
         const float2 w = tw[m * stride];
@@ -548,11 +580,13 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT) basis_pass2(
             const int t = t0 + N1 * (R1 * vv);
             if (t >= 0 && t < Tn) {
                 const float2 z = y[brev(vv, ilog2(R2))];
-                if constexpr (!kFold<N2, FORM>) store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x * zsc, z.y * zsc);
+                if constexpr (FORM == kPower) power = fmaf(z.x, z.x, fmaf(z.y, z.y, power));
+                else if constexpr (!kFold<N2, FORM>) store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x * zsc, z.y * zsc);
                 else store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x, z.y);
             }
         });
     }
+    if constexpr (FORM == kPower) power_partial<NT>((double)power, partials);
 }
 
 // pass 2 over row chunks: CTA = (TB consecutive t1, RC consecutive rows). One shared buffer holds the W tile of a row
@@ -713,7 +747,7 @@ template <int N2, int FORM, bool PAIR>
 __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
     const float2* __restrict__ W, int rows, int N, const float2* __restrict__ tw, int a0, int Tn,
     const float* __restrict__ scale, void* __restrict__ Z, void* __restrict__ Zlo, long long ldz, int im_off,
-    int row0) {
+    int row0, double* __restrict__ partials) {
     using S = SplitW<N2>;
     constexpr int R1 = S::R1, R2 = S::R2, NT = S::NT, SB = S::SB, SC = S::SC;
     constexpr int N1 = N2;                        // square split: t = t1 + N1 (u + R1 v)
@@ -734,7 +768,8 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
     };
     fetch(j0);
     // at the store: two products of 60 instructions per sample
-    const float inv0 = FORM == 4 ? 1.f : 1.0f / *scale;
+    const float inv0 = FORM == 4 || FORM == kPower ? 1.f : 1.0f / *scale;
+    double power = 0.0;
     for (int e = tid; e < N2; e += NT) tw2[e] = tw[(e % R2) * (e / R2) * (N / N2)];
     const int c = (tid & 7) + 8 * ((tid >> 4) & 1);
     const int lo = (tid >> 3) & 1, hi = tid >> 5;
@@ -784,6 +819,14 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
                 const float2 z = y[brev(vv, ilog2(R2))];
                 ps.template store<K>(z.x * inv, z.y * inv, ph, pl, (vmask >> vv) & 1u);
             });
+        } else if constexpr (FORM == kPower) {
+            float pj = 0.f;
+            static_for<R2>([&](auto V) {
+                constexpr int vv = decltype(V)::value;
+                const float2 z = y[brev(vv, ilog2(R2))];
+                if ((vmask >> vv) & 1u) pj = fmaf(z.x, z.x, fmaf(z.y, z.y, pj));
+            });
+            power += (double)pj;
         } else {
             const long long re_off = (long long)(row0 + j) * ldz * ES, im_off_b = (long long)(im_off + row0 + j) * ldz * ES;
             void* Zr = zb + re_off;
@@ -799,6 +842,7 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
             });
         }
     }
+    if constexpr (FORM == kPower) power_partial<NT>(power, partials);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -1190,7 +1234,7 @@ int launch_pass2_f(const float2* W, int N, int N1, int rows, const float2* tw, i
     const size_t smem = (size_t)(TB * S::SC + N2) * sizeof(float2);
     auto k = basis_pass2<N2, FORM>;
     GWB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k<<<dim3(N1 / TB, rows), S::NT, smem, s>>>(W, N, N1, tw, a0, Tn, scale, Z, Zlo, ldz, im_off, row0);
+    k<<<dim3(N1 / TB, rows), S::NT, smem, s>>>(W, N, N1, tw, a0, Tn, scale, Z, Zlo, ldz, im_off, row0, nullptr);
     GWB_LAUNCH_CHECK("basis_pass2");
     return GWB_OK;
 }
@@ -1225,7 +1269,7 @@ int launch_pass2_wp(const float2* W, int N, int N1, int rows, const float2* tw, 
     auto k = basis_pass2_w<N2, FORM, PAIR>;
     GWB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<dim3(N1 / TBW, (rows + RC - 1) / RC), S::NT, smem, s>>>(W, rows, N, tw, a0, Tn, scale, Z, Zlo, ldz, im_off,
-                                                                 row0);
+                                                                 row0, nullptr);
     GWB_LAUNCH_CHECK("basis_pass2_w");
     return GWB_OK;
 }
@@ -1277,6 +1321,32 @@ int launch_pass2(int form, const float2* W, int N, int N1, int rows, const float
         case 4: return launch_pass2_f<N2, 4>(W, N, N1, rows, tw, a0, Tn, scale, Z, Zlo, ldz, im_off, row0, s);
         default: return launch_pass2_f<N2, 3>(W, N, N1, rows, tw, a0, Tn, scale, Z, Zlo, ldz, im_off, row0, s);
     }
+}
+
+// scale of `rows` rows of W by their power over the analysed span (npart: doubles available)
+template <int N2>
+int launch_power(const float2* W, int N, int N1, int rows, const float2* tw, int a0, int Tn, double* partials,
+                 long long npart, float* scale, cudaStream_t s) {
+    const dim3 grid = N2 == 1024 ? dim3(N1 / TBW, (rows + RC - 1) / RC) : dim3(N1 / TB, rows);
+    const int n = (int)(grid.x * grid.y);
+    GWB_CHECK_ARG(n <= npart, GWB_ERR_SHAPE, "basis_series: %lld partials, %d needed", npart, n);
+    if constexpr (N2 == 1024) {
+        using S = SplitW<N2>;
+        const size_t smem = (size_t)(TBW * S::SC + N2) * sizeof(float2);
+        auto k = basis_pass2_w<N2, kPower, false>;
+        GWB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k<<<grid, S::NT, smem, s>>>(W, rows, N, tw, a0, Tn, nullptr, nullptr, nullptr, 0, 0, 0, partials);
+    } else {
+        using S = Split<N2, 2>;
+        const size_t smem = (size_t)(TB * S::SC + N2) * sizeof(float2);
+        auto k = basis_pass2<N2, kPower>;
+        GWB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        k<<<grid, S::NT, smem, s>>>(W, N, N1, tw, a0, Tn, nullptr, nullptr, nullptr, 0, 0, 0, partials);
+    }
+    GWB_LAUNCH_CHECK("basis_pass2 (power)");
+    power_scale_kernel<<<1, 256, 0, s>>>(partials, n, (double)rows * (double)Tn, scale);
+    GWB_LAUNCH_CHECK("power_scale_kernel");
+    return GWB_OK;
 }
 
 }  // namespace
@@ -1470,6 +1540,65 @@ int gwb_basis_fused(const float* Vp, long long ldvp, int rows, const float* Dp, 
         if (st) return st;
     }
     return GWB_OK;
+}
+
+int gwb_basis_series(const float* Vh, long long ldv, int rows, const float* D, const float* isw, long long flen,
+                     long long N, const float* tw, float* Vp, float* Dp, float* W, int wrows, long long a0, long long Tn,
+                     int form, void* Z, void* Zlo, long long ldz, int im_off, double* partials, long long npartials,
+                     float* scale, void* stream) {
+    using namespace gwb;
+    GWB_CHECK_ARG(Vh && D && tw && Vp && Dp && W && Z && partials && scale && (form != 2 || Zlo), GWB_ERR_ARG,
+                  "basis_series: null pointer");
+    GWB_CHECK_ARG(form >= 0 && form <= 3, GWB_ERR_ARG, "basis_series: form %d", form);
+    GWB_CHECK_ARG(is_pow2(N) && N >= (1 << 12) && N <= (1 << 20), GWB_ERR_NOT_POW2,
+                  "basis_series: N=%lld must be a power of two in [2^12, 2^20]", N);
+    GWB_CHECK_ARG(rows > 0 && rows < 65536 && wrows > 0 && a0 >= 0 && Tn > 0 && a0 + Tn <= N && ldz >= Tn &&
+                  rows <= im_off, GWB_ERR_SHAPE, "basis_series: rows=%d wrows=%d a0=%lld Tn=%lld", rows, wrows, a0, Tn);
+    const int N1 = 1 << ((log2i(N) + 1) / 2), N2 = (int)(N / N1);
+    const long long ldvp = N / 2 + 2;                      // even: 16-byte aligned rows
+    cudaStream_t s = (cudaStream_t)stream;
+    const float2* t = reinterpret_cast<const float2*>(tw);
+    const float2* v = reinterpret_cast<const float2*>(Vp);
+    const float2* d = reinterpret_cast<const float2*>(Dp);
+    float2* w = reinterpret_cast<float2*>(W);
+    const int n = (int)N, ia0 = (int)a0, iTn = (int)Tn;
+    int st = gwb_fourstep_order(D, flen, 1, isw, flen, N, Dp, ldvp, stream);
+    for (int j0 = 0; st == GWB_OK && j0 < rows; j0 += wrows) {
+        const int nr = std::min(wrows, rows - j0);
+        st = gwb_fourstep_order(Vh + 2 * j0 * ldv, ldv, nr, nullptr, flen, N, Vp, ldvp, stream);
+        if (st) break;
+        switch (N1) {
+            case 64: st = launch_pass1<64>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
+            case 128: st = launch_pass1<128>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
+            case 256: st = launch_pass1<256>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
+            case 512: st = launch_pass1<512>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
+            default: st = launch_pass1_w(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
+        }
+        if (st) break;
+        switch (N2) {
+            case 64:
+                if (j0 == 0) st = launch_power<64>(w, n, N1, nr, t, ia0, iTn, partials, npartials, scale, s);
+                if (!st) st = launch_pass2<64>(form, w, n, N1, nr, t, ia0, iTn, scale, Z, Zlo, ldz, im_off, j0, s);
+                break;
+            case 128:
+                if (j0 == 0) st = launch_power<128>(w, n, N1, nr, t, ia0, iTn, partials, npartials, scale, s);
+                if (!st) st = launch_pass2<128>(form, w, n, N1, nr, t, ia0, iTn, scale, Z, Zlo, ldz, im_off, j0, s);
+                break;
+            case 256:
+                if (j0 == 0) st = launch_power<256>(w, n, N1, nr, t, ia0, iTn, partials, npartials, scale, s);
+                if (!st) st = launch_pass2<256>(form, w, n, N1, nr, t, ia0, iTn, scale, Z, Zlo, ldz, im_off, j0, s);
+                break;
+            case 512:
+                if (j0 == 0) st = launch_power<512>(w, n, N1, nr, t, ia0, iTn, partials, npartials, scale, s);
+                if (!st) st = launch_pass2<512>(form, w, n, N1, nr, t, ia0, iTn, scale, Z, Zlo, ldz, im_off, j0, s);
+                break;
+            default:
+                if (j0 == 0) st = launch_power<1024>(w, n, N1, nr, t, ia0, iTn, partials, npartials, scale, s);
+                if (!st) st = launch_pass2<1024>(form, w, n, N1, nr, t, ia0, iTn, scale, Z, Zlo, ldz, im_off, j0, s);
+                break;
+        }
+    }
+    return st;
 }
 
 }  // extern "C"

@@ -324,6 +324,16 @@ GWB_API int gwb_basis_pass2_columns(int form);
  * (64-bit for fp32) through a lane shuffle, wherever a0, Tn and ldz are even and the planes word-aligned (fp8 and
  * other shapes store per sample); 0 stores every sample separately. Bit-identical results either way. */
 GWB_API int gwb_basis_set_pass2_pairs(int on);
+/* The reference's basis series (fp_filter.py:597-613) from filters and data in natural order: Z rows = Re / Im of the
+ * inverse transform of conj(Vh_j) D isw over [a0, a0 + Tn), divided by the rms of the first min(rows, wrows) rows over
+ * that span (written to scale). Both are reordered (gwb_fourstep_order) and go through the two fused passes in batches
+ * of wrows rows; the first batch's second pass runs once more to sum its power. Vp: wrows x (N / 2 + 2) complex, Dp:
+ * N / 2 + 2, W: wrows x N, partials: wrows x 128 doubles. isw may be NULL (D already divided). form: 0-3 as
+ * gwb_basis_pack. */
+GWB_API int gwb_basis_series(const float* Vh, long long ldv, int rows, const float* D, const float* isw, long long flen,
+                             long long N, const float* tw, float* Vp, float* Dp, float* W, int wrows, long long a0,
+                             long long Tn, int form, void* Z, void* Zlo, long long ldz, int im_off, double* partials,
+                             long long npartials, float* scale, void* stream);
 /* The same basis series for N = 2^20 in one persistent launch that keeps W in L2 (same reference call,
  * fp_filter.py:597-613): rows go in chunks of pc through a ring of nslot slots of W (pc x nslot rows of N complex,
  * 128-byte aligned; wrows = the rows W holds), pass 1 running `look` chunks ahead of pass 2; each W tile's L2 lines
