@@ -184,22 +184,61 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kTab = 2048;               // bins whose log f and w are kept from the edge pass
 constexpr int kChunk = kTab / kThreads;  // and the weights per thread that stay in registers
 
-// C_m and its derivatives (Dual) for m = lane; every lane runs the same code with its own power of pi Ms
-__device__ __forceinline__ Dual phase_function_coef(const PhaseCoef& P, int m) {
-    const Dual la = (1.0 / 3.0) * P.lms;                              // log a, v = a u
-    const double expo[kNF] = {-5.0, -3.0, -2.0, -1.0, 0.0, 0.0, 1.0, 1.0, 2.0, -34.0 / 3.0};
+// C_m and its derivatives for m = lane: pre times a^x times a polynomial in (eta, chi), with every power of pi Ms (and the
+// eccentric term's v0^(19/3)) in one exponential whose exponent is the lane's own; only logarithms of Mc, eta and f_ecc
+// come before it, side by side. (Through pow by pow, the CTA waited for this chain longer than for the sums over bins.)
+__device__ __forceinline__ Dual phase_function_coef(const double* th, double f_ecc, int m) {
+    Dual q = dc(th[1]), c1 = dc(th[2]), c2 = dc(th[3]);
+    q.d[1] = 1.0;
+    c1.d[2] = 1.0;
+    c2.d[3] = 1.0;
+    const Dual one_q = 1.0 + q, iq = dc(1.0) / one_q, qi = q * iq;
+    const Dual eta = qi * iq;
+    // log(pi Ms) = log(pi Msun) + log Mc - 0.6 log eta
+    const double ieta = 1.0 / eta.v;
+    Dual lms = dc(log(kPi * kMsun) + log(th[0]) - 0.6 * log(eta.v));
+    lms.d[0] = 1.0 / th[0];
+    lms.d[1] = -0.6 * ieta * eta.d[1];
+    const Dual la = (1.0 / 3.0) * lms;                                // log a, v = a u
+    // a^x; the eccentric term's a^(-34/3) v0^(19/3) is (pi Ms)^(-34/9 + 19/9) f_ecc^(19/9)
+    const double expo[kNF] = {-5.0, -3.0, -2.0, -1.0, 0.0, 0.0, 1.0, 1.0, 2.0, -5.0};
     double ex = 0.0;
 #pragma unroll
     for (int i = 0; i < kNF; ++i) ex = m == i ? expo[i] : ex;
-    Dual pw;                                                          // a^ex
-    pw.v = exp(ex * la.v);
+    Dual pw;
+    pw.v = exp(ex * la.v + (m == kNF - 1 ? 19.0 / 9.0 * log(f_ecc) : 0.0));
 #pragma unroll
     for (int i = 0; i < kNI; ++i) pw.d[i] = pw.v * ex * la.d[i];
-    const Dual p5 = P.p5c * (1.0 + 3.0 * (la - dc(log(0.4082482904638631))));
-    const Dual p6 = P.p6c - (6848.0 / 21.0) * (la + dc(log(4.0)));
-    Dual c = m == 0 ? dc(1.0) : m == 1 ? P.p2 : m == 2 ? P.p3 : m == 3 ? P.p4 : m == 4 ? p5 : m == 5 ? P.p5c
-             : m == 6 ? p6 : m == 7 ? dc(-6848.0 / 63.0) : m == 8 ? P.p7 : P.ecc;
-    return P.pre * pw * c;
+    const Dual e2 = eta * eta;
+    Dual c;
+    if (m == 1) {
+        c = (20.0 / 9.0) * (743.0 / 336.0 + (11.0 / 4.0) * eta);
+    } else if (m == 2 || m == 3) {
+        const Dual beta = (113.0 / 12.0) * (iq * iq * c1 + qi * qi * c2) + 6.25 * (eta * (c1 + c2));
+        const Dual sigma = (474.0 / 48.0) * (eta * c1 * c2);
+        c = m == 2 ? -16.0 * kPi + 4.0 * beta
+                   : 10.0 * (3058673.0 / 7257600.0 + ((5429.0 / 1008.0) * eta + (617.0 / 144.0) * e2)) - 10.0 * sigma;
+    } else if (m == 4 || m == 5) {
+        c = kPi * (38645.0 / 756.0 + (-65.0 / 9.0) * eta);
+        if (m == 4) c = c * (1.0 + 3.0 * (la - dc(log(0.4082482904638631))));
+    } else if (m == 6) {
+        c = (11583231236531.0 / 4694215680.0 - 640.0 / 3.0 * kPi * kPi - 6848.0 / 21.0 * kEuler) +
+            ((-15737765635.0 / 3048192.0 + 2255.0 / 12.0 * kPi * kPi) * eta + (76055.0 / 1728.0) * e2 +
+             (-127825.0 / 1296.0) * (e2 * eta));
+        c = c - (6848.0 / 21.0) * (la + dc(log(4.0)));
+    } else if (m == 7) {
+        c = dc(-6848.0 / 63.0);
+    } else if (m == 8) {
+        c = kPi * (77096675.0 / 254016.0 + ((378515.0 / 1512.0) * eta + (-74045.0 / 756.0) * e2));
+    } else if (m == 9) {
+        c = dc(-2355.0 / 1462.0 * th[4] * th[4]);
+        c.d[4] = -2355.0 / 731.0 * th[4];
+    } else {
+        c = dc(1.0);
+    }
+    Dual pre = dc(3.0 / 128.0 * ieta);
+    pre.d[1] = -pre.v * ieta * eta.d[1];
+    return pre * pw * c;
 }
 
 // f^(-1/18) from log f; w^42 = f^(-7/3)
@@ -285,7 +324,7 @@ constexpr int kOut = 7 + 3 * kNP;
 // double, against 110 for 22 trees) and stores them with the edge bin they belong to. Bound: the float64 pipe (log and
 // exp of the edge pass, then about 50 operations per bin). The former kernel took a barrier and a block reduction per
 // chi-squared bin, in which 256 threads share the 20 to 200 bins of 16 s of data, and a dual-number phase with three
-// exp and two pow per frequency bin: 803 -> 203 us for 2,048 triggers of 16 s, float32.
+// exp and two pow per frequency bin: 803 -> 194 us for 2,048 triggers of 16 s, float32.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 2) snr_grad_kernel(const double* __restrict__ params, int n,
                                                              const float2* __restrict__ D, long long ldd,
@@ -317,8 +356,7 @@ __global__ void __launch_bounds__(kThreads, 2) snr_grad_kernel(const double* __r
     const float2* d = D + (long long)i * ldd;
     if (tid < kSeg) owner[tid] = -1;
     if (warp == kWarps - 1) {
-        const PhaseCoef P = phase_coef(th, f_ecc);
-        const Dual c = phase_function_coef(P, min(lane, kNF - 1));
+        const Dual c = phase_function_coef(th, f_ecc, min(lane, kNF - 1));
         if (lane < kNF) {
             C[lane][0] = c.v;
 #pragma unroll
@@ -355,10 +393,13 @@ __global__ void __launch_bounds__(kThreads, 2) snr_grad_kernel(const double* __r
                 const double w2 = w * w, w3 = w2 * w, iu = w3 * w3, iu2 = iu * iu, iu3 = iu2 * iu, iu5 = iu3 * iu2;
                 const double u = f * iu2;
                 const double phi[kNM] = {iu5, iu3, iu2, iu, 1.0, lf, u, u * lf, f * iu, iu5 * iu5 * iu * w2, f};
-                double ph = cv[kOne] + wtc * f;
+                double ph = cv[kOne], ph2 = wtc * f;                     // two chains
 #pragma unroll
-                for (int m = 0; m < kNF; ++m)
-                    if (m != kOne) ph = fma(cv[m], phi[m], ph);
+                for (int m = 0; m < kNF; ++m) {
+                    if (m < kOne) ph = fma(cv[m], phi[m], ph);
+                    if (m > kOne) ph2 = fma(cv[m], phi[m], ph2);
+                }
+                ph += ph2;
                 ph -= 2.0 * kPi * rint(ph * (0.5 / kPi));
                 T sn, cs;
                 if constexpr (sizeof(T) == 8) {
