@@ -35,28 +35,28 @@ def plan(rows, samples, seg=0):
     samples = np.asarray(samples, np.int64)
     order = np.lexsort((samples, rows))
     rs, ss = rows[order], samples[order]
-    rows_u, peak_u = np.unique(rs, return_inverse=True)
     n = len(rs)
+    run_start = np.flatnonzero(np.r_[True, rs[1:] != rs[:-1]]) if n else np.zeros(0, np.int64)
+    rows_u = rs[run_start]
+    count = np.diff(np.r_[run_start, n])
     cands = np.zeros(n, CAND)
     cands['row'] = rs
     cands['seg'] = seg
     cands['sample'] = ss
-    cands['unit'] = peak_u
+    cands['unit'] = np.repeat(np.arange(len(rows_u)), count)
     units = np.zeros(len(rows_u), UNIT)
     units['row'] = rows_u
     units['seg'] = seg
-    if n:
-        run_end = np.r_[np.flatnonzero(np.diff(rs)) + 1, n]
-        run_start = np.r_[0, run_end[:-1]]
-        units['first'] = run_start
-        units['count'] = run_end - run_start
-        g = []
-        for u, (a, b) in enumerate(zip(run_start, run_end)):
-            for f in range(a, b, MAX_PEAKS):
-                g.append((u, f, min(MAX_PEAKS, b - f), 0))
-        groups = np.array(g, GROUP)
-    else:
-        groups = np.zeros(0, GROUP)
+    units['first'] = run_start
+    units['count'] = count
+    # a unit's run cut into items of MAX_PEAKS
+    per = -(-count // MAX_PEAKS)
+    u = np.repeat(np.arange(len(rows_u)), per)
+    off = MAX_PEAKS * (np.arange(len(u)) - np.repeat(np.cumsum(per) - per, per))
+    groups = np.zeros(len(u), GROUP)
+    groups['unit'] = u
+    groups['first'] = run_start[u] + off
+    groups['count'] = np.minimum(MAX_PEAKS, count[u] - off)
     return order, rows_u, cands, groups, units
 
 
@@ -92,3 +92,32 @@ def run_sums(cands, groups, units, E, B, nbins_row, H, D, kmin, flen, tlen, sig=
               int(kmin), int(flen), _lib.ptr(slots), _lib.ptr(sig), 0 if sig is None else sig.stride(0), float(df),
               _lib.ptr(out), s)
     return from_dev(out, PEAK, nc)
+
+
+def run_exact(cands, groups, units, H, D, IP, nbins_row, kmax_row, kmin, B, offset_mode, flen, tlen):
+    """run_edges then run_sums for one set of peaks: the records go up in one copy, and the peaks and edges come back in
+    one, so the host waits for the device once. Returns (GwbPeak records, edges (len(units), B + 1) int32), on the
+    host."""
+    dev = H.device
+    nc, ng, nu = len(cands), len(groups), len(units)
+    sizes = [nc * CAND.itemsize, ng * GROUP.itemsize, nu * UNIT.itemsize]     # 16-byte records: aligned parts
+    up = np.empty(sum(sizes), np.uint8)
+    o = 0
+    for rec, nb in zip((cands, groups, units), sizes):
+        up[o:o + nb] = rec.view(np.uint8)
+        o += nb
+    cd, gd, ud = torch.from_numpy(up).to(dev).split(sizes)
+    nchunk = _lib.load().gwb_exact_chunks(int(flen), int(kmin))
+    slots = torch.zeros((nc, nchunk, B, 2), dtype=torch.float32, device=dev)
+    out = torch.empty(nc * PEAK.itemsize + nu * (B + 1) * 4, dtype=torch.uint8, device=dev)
+    E = out[nc * PEAK.itemsize:]
+    s = _lib.stream_ptr(dev)
+    _lib.call('gwb_edges', _lib.ptr(ud), None, nu, _lib.ptr(H), H.stride(0), _lib.ptr(IP), IP.stride(0),
+              _lib.ptr(nbins_row), _lib.ptr(kmax_row), int(kmin), int(B), int(offset_mode), _lib.ptr(E), s)
+    _lib.call('gwb_bin_sums', _lib.ptr(gd), None, ng, _lib.ptr(ud), _lib.ptr(cd), _lib.ptr(E), int(B),
+              _lib.ptr(nbins_row), _lib.ptr(H), H.stride(0), _lib.ptr(D), D.shape[0], int(kmin), int(flen), int(tlen),
+              _lib.ptr(slots), s)
+    _lib.call('gwb_exact_finalize', _lib.ptr(cd), None, nc, _lib.ptr(ud), _lib.ptr(E), int(B), _lib.ptr(nbins_row),
+              int(kmin), int(flen), _lib.ptr(slots), None, 0, 1.0, _lib.ptr(out), s)
+    h = out.cpu().numpy()
+    return h[:nc * PEAK.itemsize].view(PEAK), h[nc * PEAK.itemsize:].view(np.int32).reshape(nu, B + 1)

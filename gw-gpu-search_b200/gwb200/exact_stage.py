@@ -109,15 +109,15 @@ class ExactStage:
         if npk == 0:
             return PeakValues(np.zeros(0, np.complex64), np.zeros(0, np.float32), np.zeros(0))
         order, rows_u, cands, groups, units = _exact.plan(rows, samples)
-        E, B = self._edges_dev(seg, rows_u)
         flen = seg.D.shape[0]
-        pk = _exact.run_sums(cands, groups, units, E, B, self._nb_rows, self.tile.H, seg.D, self.tile.kmin, flen,
-                             seg.tlen)
+        B = int(np.maximum(self.tile.nbins[rows_u], 1).max())
+        pk, Eh = _exact.run_exact(cands, groups, units, self.tile.H, seg.D, seg.IP.reshape(1, -1).contiguous(),
+                                  self._nb_rows, self._kmax_rows, self.tile.kmin, B, 1, flen, seg.tlen)
         z = np.empty(npk, np.complex64)
         pw = np.empty(npk, np.float32)
         z[order] = pk['zr'] + 1j * pk['zi']
         pw[order] = pk['pw']
-        Eh = E.cpu().numpy().astype(np.int64)
+        Eh = Eh.astype(np.int64)
         u_req = np.empty(npk, np.int64)
         u_req[order] = cands['unit']
         return PeakValues(z, pw, _fpeak(Eh[u_req], self.tile.nbins[rows], seg.df))
