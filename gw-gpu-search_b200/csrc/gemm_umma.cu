@@ -10,9 +10,16 @@
 //               resident in shared memory), then streams Z tiles of 128 samples x K through a ring of stages.
 //   warp 1      MMA issuer: one elected thread issues tcgen05.mma (M=128, N=128, K=16 steps) into TMEM. Work item =
 //               (time tile, M block); accumulators for re and im sit in 256 TMEM columns, double buffered (512).
-//   warps 2-9   epilogue: tcgen05.ld of re and im, |z|^2 and running max/argmax in registers. Warps w and w+4 read
-//               the same TMEM lane quarter (rows) and split the 128 columns in halves, then combine through shared
-//               memory. Only (max, index) per row and output group reaches global memory.
+//   warps 2-9   epilogue: two groups of four warps, group g takes the items of accumulator buffer g (every other
+//               item; with two M blocks, always M block g), so a group has two items' time for one and no barrier per
+//               item. A warp reads its 32 rows' re and im by tcgen05.ld, 32 samples at a time, the next 32 in flight
+//               while these are compared; the maximum runs as four chains of eight (one chain of 32 compares waits for
+//               its own latency: it, and not the tensor cores, set the time of an item). Only (max, index) per row and
+//               output group reaches global memory.
+// Work split: gridDim.x CTAs (or, where whole groups would divide unevenly, pairs of CTAs) take contiguous runs of
+// output groups; the two CTAs of a pair (a cluster) halve their run at a tile, and a group cut there is merged through
+// distributed shared memory at the end. 448 windows over 148 CTAs are 3.03 each, 4 at most; over 74 pairs 7 for two.
+// Measured: 256 x 64 split bf16 by 917,504 samples, 1 s windows, 247 -> 209 us; 1,024 x 128 fp16 by 2^20, 636 -> 615.
 // Operands: A is K-major (row = template, K contiguous), Z is MN-major (K rows, samples contiguous); both are staged
 // by TMA with the 128-byte swizzle. No multicast. Every wait is bounded (one second) and records GWB_ERR_TIMEOUT.
 #include "common.cuh"
@@ -35,7 +42,7 @@ struct __align__(64) UmmaArgs {
     int32_t* I;
     long long ldv;
     long long Tn;
-    int M, K, ntiles, group, nout, stages;
+    int M, K, ntiles, group, nout, stages, pair;
     DeviceError* err;
 };
 
@@ -57,16 +64,41 @@ __host__ __device__ inline SmemLayout smem_layout(int na, int nz, int nkc, int K
     L.z_off = 2u * na * nkc * kATileBytes;
     L.stage_bytes = (uint32_t)nz * 2u * (uint32_t)K * 128u;
     L.x_off = L.z_off + (uint32_t)stages * L.stage_bytes;
-    L.bar_off = L.x_off + 2u * 128u * 8u;
+    L.bar_off = L.x_off + 3u * 2u * 128u * 8u;
     L.total = L.bar_off + (uint32_t)(2 * stages + 6) * 8u + 16u;
     return L;
 }
 
-__device__ __forceinline__ void keep_best(float p, int j, float& best, int& bi) {
-    if (p > best) {
-        best = p;
-        bi = j;
+// maximum of |z|^2 over 32 samples and its first index: four chains of eight, merged in order (strictly larger wins, so
+// the first index stays); samples at or past `valid` count as -1
+template <bool FULL>
+__device__ __forceinline__ void best_of_32(const uint32_t (&re)[32], const uint32_t (&im)[32], int valid, int base,
+                                           float& best, int& bi) {
+    float b[4];
+    int x[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        b[c] = -1.f;
+        x[c] = 0;
     }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float r = __uint_as_float(re[8 * c + j]), i = __uint_as_float(im[8 * c + j]);
+            float p = fmaf(r, r, i * i);
+            if (!FULL && 8 * c + j >= valid) p = -1.f;
+            if (p > b[c]) {
+                b[c] = p;
+                x[c] = base + 8 * c + j;
+            }
+        }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (b[c] > best) {
+            best = b[c];
+            bi = x[c];
+        }
 }
 
 template <int FORM>
@@ -79,8 +111,9 @@ __global__ void __launch_bounds__(kThreads, 1) umma_absmax_kernel(const __grid_c
     const SmemLayout L = smem_layout(C::NA, C::NZ, nkc, K, S);
     uint8_t* sA = smem + L.a_off;
     uint8_t* sZ = smem + L.z_off;
-    float* xv = reinterpret_cast<float*>(smem + L.x_off);           // [2][128]
-    int* xi = reinterpret_cast<int*>(smem + L.x_off + 1024);        // [2][128]
+    // maxima that cross warps: [0], [1] the two epilogue groups' (one M block), by window parity; [2] the cut window's
+    float (*xv)[2][128] = reinterpret_cast<float (*)[2][128]>(smem + L.x_off);
+    int (*xi)[2][128] = reinterpret_cast<int (*)[2][128]>(smem + L.x_off + 3072);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L.bar_off);
     uint64_t* full = bars;
     uint64_t* empty = bars + S;
@@ -94,12 +127,19 @@ __global__ void __launch_bounds__(kThreads, 1) umma_absmax_kernel(const __grid_c
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * 256;
     const int MBe = min(2, (args.M - m0 + 127) / 128);
-    const long long o0 = (long long)blockIdx.x * args.nout / gridDim.x;
-    const long long o1 = (long long)(blockIdx.x + 1) * args.nout / gridDim.x;
-    const int t_begin = (int)(o0 * args.group);
-    const int t_end = (int)min(o1 * (long long)args.group, (long long)args.ntiles);
+    const int pair = args.pair, rank = pair ? (int)(blockIdx.x & 1) : 0;
+    const int runs = (int)gridDim.x >> pair, run = (int)blockIdx.x >> pair;
+    const long long o0 = (long long)run * args.nout / runs;
+    const long long o1 = (long long)(run + 1) * args.nout / runs;
+    const int r_begin = (int)(o0 * args.group);
+    const int r_end = (int)min(o1 * (long long)args.group, (long long)args.ntiles);
+    const int r_mid = r_begin + (r_end - r_begin + 1) / 2;            // where a pair's run is cut
+    const int t_begin = rank ? r_mid : r_begin, t_end = pair && !rank ? r_mid : r_end;
     const int ntl = t_end - t_begin;
-    if (ntl <= 0 || MBe <= 0) return;   // uniform across the CTA
+    // the cut falls inside a group: rank 1 hands its part's maximum to rank 0
+    const bool cut = pair && r_mid < r_end && r_mid % args.group != 0;
+    if (!pair && (ntl <= 0 || MBe <= 0)) return;   // uniform across the CTA
+    const bool live = ntl > 0 && MBe > 0;          // a pair's CTA without tiles still meets the other at the end
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < S; ++s) {
@@ -108,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_absmax_kernel(const __grid_c
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
-            mbar_init(&tempty[b], kEpiWarps);
+            mbar_init(&tempty[b], kEpiWarps / 2);
         }
         mbar_init(barA, 1);
         mbar_init(done, 1);
@@ -124,7 +164,8 @@ __global__ void __launch_bounds__(kThreads, 1) umma_absmax_kernel(const __grid_c
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    if (warp == 0) {
+    if (!live) {
+    } else if (warp == 0) {
         // ---------------- TMA producer ----------------
         if (lane == 0) {
             for (int a = 0; a < C::NA; ++a) prefetch_tmap(&args.tA[a]);
@@ -194,14 +235,18 @@ __global__ void __launch_bounds__(kThreads, 1) umma_absmax_kernel(const __grid_c
                             // products: (A hi, Z hi), (A hi, Z lo), (A lo, Z hi)
                             const int a = (pr == 2 ? 2 : 0) + ri;
                             const int z = (pr == 1) ? 1 : 0;
-                            for (int k16 = 0; k16 < K / 16; ++k16) {
-                                const uint32_t aaddr =
-                                    a_base + ((mb * C::NA + a) * nkc + (k16 >> 2)) * kATileBytes + (k16 & 3) * 32;
-                                const uint32_t baddr = z_base + s * L.stage_bytes + (z * 2) * K * 128 + k16 * 2048;
-                                const uint64_t adesc = smem_desc(aaddr, 16, 1024, 2);
-                                const uint64_t bdesc = smem_desc(baddr, (uint32_t)K * 128u, 1024, 2);
-                                umma_f16(d, adesc, bdesc, idesc, acc);
-                                acc = 1;
+                            // descriptors advance by K steps of 16: 32 bytes of a 64-wide A box, 2048 of Z
+                            uint64_t ad = smem_desc(a_base + (mb * C::NA + a) * nkc * kATileBytes, 16, 1024, 2);
+                            uint64_t bd = smem_desc(z_base + s * L.stage_bytes + (z * 2) * K * 128, (uint32_t)K * 128u,
+                                                    1024, 2);
+                            for (int kc = 0; kc < nkc; ++kc) {
+#pragma unroll
+                                for (int k16 = 0; k16 < 4; ++k16) {
+                                    umma_f16(d, ad + k16 * (32 >> 4), bd + k16 * (2048 >> 4), idesc, acc);
+                                    acc = 1;
+                                }
+                                ad += kATileBytes >> 4;
+                                bd += 4 * 2048 >> 4;
                             }
                         }
                     }
@@ -215,94 +260,149 @@ __global__ void __launch_bounds__(kThreads, 1) umma_absmax_kernel(const __grid_c
         __syncwarp();
     } else {
         // ---------------- epilogue ----------------
-        const int ew = warp - 2, q = warp & 3, hh = ew >> 2;
+        const int q = warp & 3, g = (warp - 2) >> 2;
         const int rl = 32 * q + lane;
-        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-        float wb0 = -1.f, wb1 = -1.f;
-        int wi0 = 0, wi1 = 0;
-        for (int i = 0; i < ntl; ++i) {
-            const int t = t_begin + i;
-            const long long col0 = (long long)t * kTile;
-            const bool full_tile = col0 + kTile <= args.Tn;
-#pragma unroll
-            for (int mb = 0; mb < 2; ++mb) {
-                if (mb >= MBe) break;
-                const int j = i * MBe + mb, b = j & 1;
-                const uint32_t u = (uint32_t)(j >> 1);
-                float best = -1.f;
-                int bi = 0;
-                if (*abort_flag || !mbar_wait_bounded(&tfull[b], u & 1)) {
-                    record_error(args.err, GWB_ERR_TIMEOUT, 105, blockIdx.x, i);
-                    *abort_flag = 1;
-                } else {
-                    tc_fence_after();
-#pragma unroll
-                    for (int c = 0; c < 64; c += 32) {
-                        uint32_t re[32], im[32];
-                        tmem_ld_32x32b_x32(lane_base + (uint32_t)(b * 256 + hh * 64 + c), re);
-                        tmem_ld_32x32b_x32(lane_base + (uint32_t)(b * 256 + 128 + hh * 64 + c), im);
-                        tmem_ld_wait();
-                        // tie every value to the wait so no use is scheduled above it
-#pragma unroll
-                        for (int jj = 0; jj < 32; ++jj) asm volatile("" : "+r"(re[jj]), "+r"(im[jj]));
-                        const int cb = hh * 64 + c;
-                        float lb = -1.f;
-                        int lj = 0;
-                        if (full_tile) {
-#pragma unroll
-                            for (int jj = 0; jj < 32; ++jj) {
-                                const float xr = __uint_as_float(re[jj]), xi_ = __uint_as_float(im[jj]);
-                                keep_best(fmaf(xr, xr, xi_ * xi_), jj, lb, lj);
-                            }
-                        } else {
-                            const int valid = (int)min((long long)32, max(0ll, args.Tn - (col0 + cb)));
-#pragma unroll
-                            for (int jj = 0; jj < 32; ++jj) {
-                                const float xr = __uint_as_float(re[jj]), xi_ = __uint_as_float(im[jj]);
-                                keep_best(jj < valid ? fmaf(xr, xr, xi_ * xi_) : -1.f, jj, lb, lj);
-                            }
-                        }
-                        if (lb > best) {
-                            best = lb;
-                            bi = cb + lj;
-                        }
-                    }
-                }
+        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(g * 256);
+        const int G = args.group;
+        // maximum of item j (tile t): waits for the accumulators, frees them once they are in registers
+        auto item = [&](int j, int t, float& best, int& bi) {
+            best = -1.f;
+            bi = 0;
+            if (*abort_flag || !mbar_wait_bounded(&tfull[g], (uint32_t)((j >> 1) & 1))) {
+                record_error(args.err, GWB_ERR_TIMEOUT, 105, blockIdx.x, j);
+                *abort_flag = 1;
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&tempty[b]);
-                if (hh == 1) {
-                    xv[(j & 1) * 128 + rl] = best;
-                    xi[(j & 1) * 128 + rl] = bi;
+                if (lane == 0) mbar_arrive(&tempty[g]);
+                return;
+            }
+            tc_fence_after();
+            const long long left = args.Tn - (long long)t * kTile;     // samples of the tile inside the row
+            uint32_t re[2][32], im[2][32];
+            tmem_ld_32x32b_x32(lane_base, re[0]);
+            tmem_ld_32x32b_x32(lane_base + 128, im[0]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                tmem_ld_wait();
+                // tie every value to the wait so no use is scheduled above it
+#pragma unroll
+                for (int jj = 0; jj < 32; ++jj) asm volatile("" : "+r"(re[c & 1][jj]), "+r"(im[c & 1][jj]));
+                if (c < 3) {
+                    tmem_ld_32x32b_x32(lane_base + 32 * (c + 1), re[(c + 1) & 1]);
+                    tmem_ld_32x32b_x32(lane_base + 128 + 32 * (c + 1), im[(c + 1) & 1]);
+                } else {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty[g]);
                 }
-                named_bar_sync(1, 32 * kEpiWarps);
-                if (hh == 0) {
-                    const float ob = xv[(j & 1) * 128 + rl];
-                    const int oi = xi[(j & 1) * 128 + rl];
-                    if (ob > best) {
-                        best = ob;
-                        bi = oi;
-                    }
-                    const int gi = (int)(col0 + bi);
-                    const bool first = (t % args.group) == 0;
-                    const bool last = ((t + 1) % args.group) == 0 || t == args.ntiles - 1;
-                    float& wb = (mb == 0) ? wb0 : wb1;
-                    int& wi = (mb == 0) ? wi0 : wi1;
-                    if (first || best > wb) {
+                if (left >= kTile)
+                    best_of_32<true>(re[c & 1], im[c & 1], 32, 32 * c, best, bi);
+                else
+                    best_of_32<false>(re[c & 1], im[c & 1], (int)min(32ll, max(0ll, left - 32 * c)), 32 * c, best, bi);
+            }
+            bi += t * kTile;
+        };
+        // the maximum (wb, wi) of the part of group o that this CTA holds, of M block mb: rank 1's part of a cut group
+        // goes to shared memory, rank 0 keeps its own in registers (returns true), all others go out
+        auto put = [&](int o, int mb, float wb, int wi) {
+            if (cut && o == r_mid / G) {
+                if (rank == 0) return true;
+                xv[2][mb][rl] = wb;
+                xi[2][mb][rl] = wi;
+                return false;
+            }
+            const int row = m0 + mb * 128 + rl;
+            if (row < args.M) {
+                args.V[(long long)row * args.ldv + o] = wb;
+                args.I[(long long)row * args.ldv + o] = wi;
+            }
+            return false;
+        };
+        float wb = -2.f;                                   // below any tile's maximum (at least -1)
+        int wi = 0;
+        bool held = false;                                 // (wb, wi) is rank 0's part of the cut group
+        if (MBe == 2) {                                    // group g: M block g of every tile
+            for (int i = 0; i < ntl; ++i) {
+                const int t = t_begin + i;
+                float best;
+                int bi;
+                item(2 * i + g, t, best, bi);
+                if (best > wb) {
+                    wb = best;
+                    wi = bi;
+                }
+                if ((t + 1) % G == 0 || t + 1 == t_end) {
+                    held = put(t / G, g, wb, wi);
+                    if (!held) wb = -2.f;
+                }
+            }
+        } else if (G == 1) {                               // one M block, every tile an output: tiles by parity
+            for (int i = g; i < ntl; i += 2) {
+                float best;
+                int bi;
+                item(i, t_begin + i, best, bi);
+                put(t_begin + i, 0, best, bi);
+            }
+        } else {                                           // one M block: the two groups meet at every output
+            int par = 0;
+            for (int t = t_begin; t < t_end; par ^= 1) {
+                const int o = t / G, te = min((o + 1) * G, t_end);
+                wb = -2.f;
+                wi = 0;
+                for (; t < te; ++t) {
+                    const int i = t - t_begin;
+                    if ((i & 1) != g) continue;
+                    float best;
+                    int bi;
+                    item(i, t, best, bi);
+                    if (best > wb) {
                         wb = best;
-                        wi = gi;
+                        wi = bi;
                     }
-                    if (last) {
-                        const int row = m0 + mb * 128 + rl;
-                        if (row < args.M) {
-                            const long long o = t / args.group;
-                            args.V[(long long)row * args.ldv + o] = wb;
-                            args.I[(long long)row * args.ldv + o] = wi;
-                        }
+                }
+                if (g == 1) {
+                    xv[par][0][rl] = wb;
+                    xi[par][0][rl] = wi;
+                }
+                named_bar_sync(1, 32 * kEpiWarps);         // the slots take turns: written again two outputs on
+                if (g == 0) {
+                    const float ob = xv[par][0][rl];
+                    const int oi = xi[par][0][rl];
+                    if (ob > wb || (ob == wb && oi < wi)) {
+                        wb = ob;
+                        wi = oi;
                     }
+                    held = put(o, 0, wb, wi);
                 }
             }
         }
+        if (cut) {
+            // rank 1's part lies after rank 0's: it replaces only where it is larger
+            cluster_sync_all();
+            if (held) {
+                const int mb = MBe == 2 ? g : 0;
+                float ob;
+                int oi;
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(ob) : "r"(mapa_shared(smem_u32(&xv[2][mb][rl]), 1)));
+                asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(oi) : "r"(mapa_shared(smem_u32(&xi[2][mb][rl]), 1)));
+                if (ob > wb) {
+                    wb = ob;
+                    wi = oi;
+                }
+                const int row = m0 + mb * 128 + rl;
+                if (row < args.M) {
+                    args.V[(long long)row * args.ldv + r_mid / G] = wb;
+                    args.I[(long long)row * args.ldv + r_mid / G] = wi;
+                }
+            }
+        }
+    }
+    if (cut) {
+        // every thread of both CTAs: the epilogue warps met once above (rank 1's part is in shared memory); all meet
+        // again here, so that rank 1 does not leave while its shared memory may be read
+        if (!live || warp < 2) cluster_sync_all();
+        __syncwarp();
+        cluster_sync_all();
     }
     __syncthreads();
     if (warp == 1) {
@@ -370,9 +470,23 @@ int launch_umma(const uint16_t* const* A, const uint16_t* const* Zp, long long l
 
     auto kern = umma_absmax_kernel<FORM>;
     GWB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int gx = (int)std::max(1ll, std::min(nout, (long long)std::max(1, num_sms() / mgroups)));
-    dim3 grid(gx, mgroups);
-    kern<<<grid, kThreads, smem, stream>>>(args);
+    int gx = (int)std::max(1ll, std::min(nout, (long long)std::max(1, num_sms() / mgroups)));
+    // pairs of CTAs where whole groups of several tiles would divide unevenly (a CTA would hold 16 or fewer): the run
+    // with the most groups then holds at most half a group more than the mean per CTA, not a whole one
+    args.pair = group > 1 && gx > 1 && nout <= 16ll * gx && nout % gx != 0;
+    if (args.pair) gx &= ~1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(gx, mgroups);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = args.pair ? 1 : 0;
+    GWB_CUDA(cudaLaunchKernelEx(&cfg, kern, args));
     GWB_LAUNCH_CHECK("umma_absmax_kernel");
     return GWB_OK;
 }
