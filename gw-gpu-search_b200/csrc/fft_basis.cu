@@ -42,9 +42,20 @@ __global__ void twiddle_kernel(float2* tw, long long N) {
 
 // P[j][k2 H + k1] = X[j][N2 k1 + k2] (times isw) for k1 < H = N1 / 2, k2 < N2, and P[j][N / 2] = X[j][N / 2]; zero
 // where k >= flen. 32 x 32 tiles through shared memory.
+// last_nz (may be null): the largest k of any row whose value is not zero (NaN counts); last_bad (may be null): per row
+// the largest k whose value is not finite. Both are raised by atomicMax: the caller sets them (to -1). ENDS: either is
+// wanted (the looks cost 40% of the copy).
+template <bool ENDS>
 __global__ void fourstep_order_kernel(const float2* __restrict__ X, long long ldx, const float* __restrict__ isw,
-                                      long long flen, int N2, int H, float2* __restrict__ P, long long ldp) {
+                                      long long flen, int N2, int H, float2* __restrict__ P, long long ldp,
+                                      int* __restrict__ last_nz, int* __restrict__ last_bad) {
     __shared__ float2 tile[32][33];
+    int nz = -1, bad = -1;
+    auto look = [&](float2 v, long long k) {
+        if constexpr (!ENDS) return;
+        if (v.x != 0.f || v.y != 0.f) nz = (int)k;
+        if (!isfinite(v.x) || !isfinite(v.y)) bad = (int)k;
+    };
     const int j = blockIdx.z;
     const int k20 = blockIdx.x * 32, k10 = blockIdx.y * 32;
     const float2* x = X + (long long)j * ldx;
@@ -60,6 +71,7 @@ __global__ void fourstep_order_kernel(const float2* __restrict__ X, long long ld
             }
         }
         tile[i][threadIdx.x] = v;
+        look(v, k);                                // k rises with i
     }
     __syncthreads();
     for (int i = threadIdx.y; i < 32; i += blockDim.y)
@@ -72,6 +84,15 @@ __global__ void fourstep_order_kernel(const float2* __restrict__ X, long long ld
             if (isw) v = make_float2(v.x * isw[k], v.y * isw[k]);
         }
         p[k] = v;
+        look(v, k);
+    }
+    if constexpr (!ENDS) return;
+    nz = __reduce_max_sync(0xffffffffu, nz);
+    bad = __reduce_max_sync(0xffffffffu, bad);
+    if (threadIdx.x == 0) {
+        // most warps find the word already at or above theirs
+        if (last_nz && nz > *(volatile int*)last_nz) atomicMax(last_nz, nz);
+        if (last_bad && bad > *(volatile int*)(last_bad + j)) atomicMax(last_bad + j, bad);
     }
 }
 
@@ -188,6 +209,30 @@ __device__ __forceinline__ void dft_reg_upper_zero(float2 (&x)[R]) {
     });
 }
 
+// dft_reg for inputs that are zero from x[Q] on (Q a power of two): while a stage's half h is at least Q, its butterflies
+// have a zero partner and reduce to a copy and a rotation of the Q live inputs of each block. Same output as dft_reg on
+// those inputs (up to the sign of exact zeros).
+template <int Q, int R>
+__device__ __forceinline__ void dft_reg_zero_from(float2 (&x)[R]) {
+    static_for<ilog2(R)>([&](auto S) {
+        constexpr int h = R >> (decltype(S)::value + 1);
+        static_for<R / (2 * h)>([&](auto B) {
+            constexpr int base = decltype(B)::value * 2 * h;
+            static_for<(h < Q ? h : Q)>([&](auto J) {
+                constexpr int j = decltype(J)::value;
+                const float2 a = x[base + j];
+                if constexpr (h >= Q) {
+                    x[base + j + h] = rot<j, 2 * h>(a);
+                } else {
+                    const float2 b = x[base + j + h];
+                    x[base + j] = make_float2(a.x + b.x, a.y + b.y);
+                    x[base + j + h] = rot<j, 2 * h>(make_float2(a.x - b.x, a.y - b.y));
+                }
+            });
+        });
+    });
+}
+
 // Two-level split of a DFT of length L over TB columns. Shared buffer Y[c][b][u] at c * SC + b * SB + u (float2):
 // SB = 1 (mod 16 eight-byte words) and SC = SCM (mod 16), chosen per pass so that each half-warp of a 64-bit access
 // hits 16 distinct bank pairs.
@@ -253,12 +298,21 @@ constexpr int RC = 8;   // rows per pass-1 CTA of the warp-per-column form
 // shared memory (cp.async) while the current row is transformed. No CTA barrier after the set-up, so the warps of a
 // CTA drift apart and one warp's copies overlap another's arithmetic. Scale partials: one per (row chunk, column),
 // summed in a fixed order by the last warp to finish.
+// Band: the basis filters of a tile end at its templates' last f_ISCO, so q is zero from bin kend on and only the first
+// A of a column's 16 runs of 32 bins are live (k1 < 32 A holds every k < kend): the others are neither loaded nor
+// multiplied, and the first DFT starts from A inputs. The outputs are those of the full kernel bit for bit (up to the
+// sign of exact zeros) as long as D is finite from kend on; where it is not (*last_bad >= kend), 0 * D puts a NaN into
+// every output, and so does this kernel. 122 rows of 2^20 at A = 1: 315 -> 240 us (W's
+// store is 157 at the measured copy rate).
+template <int N2, int A>
 __global__ void __launch_bounds__(256, 2) basis_pass1_w(
-    const float2* __restrict__ Vp, long long ldvp, int rows, const float2* __restrict__ Dp, int N, int N2,
+    const float2* __restrict__ Vp, long long ldvp, int rows, const float2* __restrict__ Dp,
     const float2* __restrict__ tw, float2* __restrict__ W, int nfirst, double* __restrict__ partials,
-    unsigned int* __restrict__ ticket, float* __restrict__ scale_out, float* __restrict__ rowpart) {
-    constexpr int N1 = 1024, R = 32, H = N1 / 2, NW = 8, YS = R * (R + 1);
+    unsigned int* __restrict__ ticket, float* __restrict__ scale_out, float* __restrict__ rowpart, int kend,
+    const int* __restrict__ last_bad) {
+    constexpr int N1 = 1024, N = N1 * N2, R = 32, H = N1 / 2, NW = 8, YS = R * (R + 1);
     constexpr int WS = YS + R + H;                          // per warp: Y tile, TH, basis-filter segment
+    static_assert(A >= 1 && A <= R / 2, "live runs");
     extern __shared__ float2 sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float2* tw2 = sm;                                       // tw2[u 32 + b] = e^{2 pi i b u / N1}
@@ -267,19 +321,23 @@ __global__ void __launch_bounds__(256, 2) basis_pass1_w(
     float2* Vs = THw + R;                                   // Vp[row][k2 H .. k2 H + H)
     const int k2 = blockIdx.x * NW + warp;
     const int j0 = blockIdx.y * RC, j1 = min(j0 + RC, rows);
-    const int mask = N - 1;
-    auto fetch = [&](int j) {                               // 4 KB: 8 x 16 bytes per lane
+    constexpr int mask = N - 1;
+    auto fetch = [&](int j) {                               // 256 A bytes (4 KB at A = 16: 8 x 16 bytes per lane)
         const char* g = reinterpret_cast<const char*>(Vp + (long long)j * ldvp + k2 * H);
         char* d = reinterpret_cast<char*>(Vs);
+        if (A > 1 || lane < 16) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) cp_async16(d + i * 512 + lane * 16, g + i * 512 + lane * 16);
+            for (int i = 0; i < (A + 1) / 2; ++i) cp_async16(d + i * 512 + lane * 16, g + i * 512 + lane * 16);
+        }
         cp_async_commit();
     };
     fetch(j0);
-    float2 dk[R / 2];
+    float2 dk[A];
 #pragma unroll
-    for (int a = 0; a < R / 2; ++a) dk[a] = __ldg(Dp + k2 * H + R * a + lane);
+    for (int a = 0; a < A; ++a) dk[a] = __ldg(Dp + k2 * H + R * a + lane);
     const float2 dN = Dp[N / 2];
+    const bool poison = A < R / 2 && last_bad && *last_bad >= kend;
+    if (poison) dk[0] = make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
     for (int e = threadIdx.x; e < N1; e += NW * 32) tw2[e] = tw[(e % R) * (e / R) * (N / N1)];
     THw[lane] = tw[(k2 * (R * lane)) & mask];
     const float2 tl = tw[(k2 * lane) & mask];               // e^{2 pi i k2 u / N}, u = lane
@@ -291,16 +349,16 @@ __global__ void __launch_bounds__(256, 2) basis_pass1_w(
         __syncwarp();
         float2 x[R];
 #pragma unroll
-        for (int a = 0; a < R / 2; ++a) x[a] = Vs[R * a + lane];
+        for (int a = 0; a < A; ++a) x[a] = Vs[R * a + lane];
         __syncwarp();
         if (j + 1 < j1) fetch(j + 1);
 #pragma unroll
-        for (int a = 0; a < R / 2; ++a) {
+        for (int a = 0; a < A; ++a) {
             const float2 av = x[a];
             x[a] = make_float2(fmaf(av.x, dk[a].x, av.y * dk[a].y), fmaf(av.x, dk[a].y, -(av.y * dk[a].x)));
         }
-        x[R / 2] = make_float2(0.f, 0.f);
-        if (k2 == 0 && lane == 0) {                         // the bin N / 2
+        if constexpr (A == R / 2) x[R / 2] = make_float2(0.f, 0.f);
+        if (A == R / 2 && k2 == 0 && lane == 0) {           // the bin N / 2
             const float2 av = Vp[(long long)j * ldvp + N / 2];
             x[R / 2] = make_float2(fmaf(av.x, dN.x, av.y * dN.y), fmaf(av.x, dN.y, -(av.y * dN.x)));
         }
@@ -308,7 +366,7 @@ __global__ void __launch_bounds__(256, 2) basis_pass1_w(
         if (j < nf || rowpart) {
             float part = 0.f;
 #pragma unroll
-            for (int a = 0; a <= R / 2; ++a) part = fmaf(x[a].x, x[a].x, fmaf(x[a].y, x[a].y, part));
+            for (int a = 0; a <= (A == R / 2 ? A : A - 1); ++a) part = fmaf(x[a].x, x[a].x, fmaf(x[a].y, x[a].y, part));
             if (j < nf) acc += (double)part;
             if (rowpart) {                                  // per-row sums of |q|^2: rowpart[j][k2]
                 float ps = part;
@@ -317,7 +375,8 @@ __global__ void __launch_bounds__(256, 2) basis_pass1_w(
                 if (lane == 0) rowpart[(long long)j * N2 + k2] = ps;
             }
         }
-        dft_reg_upper_zero<R>(x);                           // q is zero for k1 > N1 / 2
+        if constexpr (A == R / 2) dft_reg_upper_zero<R>(x); // q is zero for k1 > N1 / 2
+        else dft_reg_zero_from<A, R>(x);
         static_for<R>([&](auto U) {
             constexpr int u = decltype(U)::value;
             Yw[lane * (R + 1) + u] = cmul(x[brev(u, ilog2(R))], tw2[u * R + lane]);
@@ -1202,15 +1261,32 @@ int launch_persist(const PersistArgs& a, cudaStream_t s) {
     return GWB_OK;
 }
 
-int launch_pass1_w(const float2* Vp, long long ldvp, int rows, const float2* Dp, int N, int N2, const float2* tw,
-                   float2* W, int nfirst, double* partials, unsigned* ticket, float* scale_out, float* rowpart,
-                   cudaStream_t s) {
+template <int N2, int A>
+int launch_pass1_wa(const float2* Vp, long long ldvp, int rows, const float2* Dp, const float2* tw, float2* W, int nfirst,
+                    double* partials, unsigned* ticket, float* scale_out, float* rowpart, int kend, const int* last_bad,
+                    cudaStream_t s) {
     const size_t smem = (size_t)(1024 + 8 * (32 * 33 + 32 + 512)) * sizeof(float2);
-    GWB_CUDA(cudaFuncSetAttribute(basis_pass1_w, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    basis_pass1_w<<<dim3(N2 / 8, (rows + RC - 1) / RC), 256, smem, s>>>(Vp, ldvp, rows, Dp, N, N2, tw, W, nfirst,
-                                                                         partials, ticket, scale_out, rowpart);
+    auto k = basis_pass1_w<N2, A>;
+    GWB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k<<<dim3(N2 / 8, (rows + RC - 1) / RC), 256, smem, s>>>(Vp, ldvp, rows, Dp, tw, W, nfirst, partials, ticket,
+                                                             scale_out, rowpart, kend, last_bad);
     GWB_LAUNCH_CHECK("basis_pass1_w");
     return GWB_OK;
+}
+
+// N1 = 1024: N2 is 512 or 1024. kend: Vp is zero from this bin on (N / 2 + 1: no limit)
+int launch_pass1_w(const float2* Vp, long long ldvp, int rows, const float2* Dp, int N2, const float2* tw, float2* W,
+                   int nfirst, double* partials, unsigned* ticket, float* scale_out, float* rowpart, int kend,
+                   const int* last_bad, cudaStream_t s) {
+    const int runs = kend > 512 * N2 ? 16 : ((kend + N2 - 1) / N2 + 31) / 32;
+    auto go = [&](auto n2) {
+        constexpr int M = decltype(n2)::value;
+#define GWB_P1(A) launch_pass1_wa<M, A>(Vp, ldvp, rows, Dp, tw, W, nfirst, partials, ticket, scale_out, rowpart, kend, \
+                                        last_bad, s)
+        return runs <= 1 ? GWB_P1(1) : runs <= 2 ? GWB_P1(2) : runs <= 4 ? GWB_P1(4) : runs <= 8 ? GWB_P1(8) : GWB_P1(16);
+#undef GWB_P1
+    };
+    return N2 == 512 ? go(ic<512>{}) : go(ic<1024>{});
 }
 
 template <int N1>
@@ -1365,6 +1441,11 @@ int gwb_fft_twiddles(long long N, float* tw, void* stream) {
 
 int gwb_fourstep_order(const float* X, long long ldx, int rows, const float* isw, long long flen, long long N,
                        float* P, long long ldp, void* stream) {
+    return gwb_fourstep_order_ends(X, ldx, rows, isw, flen, N, P, ldp, nullptr, nullptr, stream);
+}
+
+int gwb_fourstep_order_ends(const float* X, long long ldx, int rows, const float* isw, long long flen, long long N,
+                            float* P, long long ldp, int32_t* last_nz, int32_t* last_bad, void* stream) {
     using namespace gwb;
     GWB_CHECK_ARG(X && P, GWB_ERR_ARG, "fourstep_order: null pointer");
     GWB_CHECK_ARG(is_pow2(N) && N >= (1 << 12) && N <= (1 << 20), GWB_ERR_NOT_POW2,
@@ -1373,8 +1454,12 @@ int gwb_fourstep_order(const float* X, long long ldx, int rows, const float* isw
                   GWB_ERR_SHAPE, "fourstep_order: rows=%d flen=%lld N=%lld ldx=%lld ldp=%lld", rows, flen, N, ldx, ldp);
     const int p = log2i(N);
     const int N1 = 1 << ((p + 1) / 2), N2 = (int)(N / N1);
-    fourstep_order_kernel<<<dim3(N2 / 32, N1 / 64, rows), dim3(32, 8), 0, (cudaStream_t)stream>>>(
-        reinterpret_cast<const float2*>(X), ldx, isw, flen, N2, N1 / 2, reinterpret_cast<float2*>(P), ldp);
+    if (last_nz) GWB_CUDA(cudaMemsetAsync(last_nz, 0xff, sizeof(int32_t), (cudaStream_t)stream));
+    if (last_bad) GWB_CUDA(cudaMemsetAsync(last_bad, 0xff, sizeof(int32_t) * rows, (cudaStream_t)stream));
+    auto kern = last_nz || last_bad ? fourstep_order_kernel<true> : fourstep_order_kernel<false>;
+    kern<<<dim3(N2 / 32, N1 / 64, rows), dim3(32, 8), 0, (cudaStream_t)stream>>>(
+        reinterpret_cast<const float2*>(X), ldx, isw, flen, N2, N1 / 2, reinterpret_cast<float2*>(P), ldp, last_nz,
+        last_bad);
     GWB_LAUNCH_CHECK("fourstep_order_kernel");
     return GWB_OK;
 }
@@ -1480,7 +1565,19 @@ int gwb_basis_fused(const float* Vp, long long ldvp, int rows, const float* Dp, 
                     int wrows, long long a0, long long Tn, int form, void* Z, void* Zlo, long long ldz, int im_off,
                     int row0, int nfirst, double* partials, long long npartials, uint32_t* ticket, float* scale,
                     float* rowscale, float* rowpart, long long rowpart_elems, void* stream) {
+    return gwb_basis_fused_band(Vp, ldvp, rows, Dp, N, tw, W, wrows, a0, Tn, form, Z, Zlo, ldz, im_off, row0, nfirst,
+                                partials, npartials, ticket, scale, rowscale, rowpart, rowpart_elems, N / 2 + 1,
+                                nullptr, stream);
+}
+
+int gwb_basis_fused_band(const float* Vp, long long ldvp, int rows, const float* Dp, long long N, const float* tw,
+                         float* W, int wrows, long long a0, long long Tn, int form, void* Z, void* Zlo, long long ldz,
+                         int im_off, int row0, int nfirst, double* partials, long long npartials, uint32_t* ticket,
+                         float* scale, float* rowscale, float* rowpart, long long rowpart_elems, long long kend64,
+                         const int32_t* last_bad, void* stream) {
     using namespace gwb;
+    GWB_CHECK_ARG(kend64 >= 0, GWB_ERR_SHAPE, "basis_fused: kend=%lld", kend64);
+    const int kend = (int)std::min(kend64, N / 2 + 1);
     GWB_CHECK_ARG(Vp && Dp && tw && W && Z && scale && (form != 2 || Zlo), GWB_ERR_ARG, "basis_fused: null pointer");
     GWB_CHECK_ARG(form >= 0 && form <= 4, GWB_ERR_ARG, "basis_fused: form %d", form);
     GWB_CHECK_ARG(is_pow2(N) && N >= (1 << 12) && N <= (1 << 20), GWB_ERR_NOT_POW2,
@@ -1520,7 +1617,7 @@ int gwb_basis_fused(const float* Vp, long long ldvp, int rows, const float* Dp, 
             case 128: st = launch_pass1<128>(v, ldvp, nr, d, n, N2, t, w, nfb, partials, tk, scale, rp, s); break;
             case 256: st = launch_pass1<256>(v, ldvp, nr, d, n, N2, t, w, nfb, partials, tk, scale, rp, s); break;
             case 512: st = launch_pass1<512>(v, ldvp, nr, d, n, N2, t, w, nfb, partials, tk, scale, rp, s); break;
-            default: st = launch_pass1_w(v, ldvp, nr, d, n, N2, t, w, nfb, partials, tk, scale, rp, s); break;
+            default: st = launch_pass1_w(v, ldvp, nr, d, N2, t, w, nfb, partials, tk, scale, rp, kend, last_bad, s); break;
         }
         if (st) return st;
         const float* sc = scale;
@@ -1572,7 +1669,7 @@ int gwb_basis_series(const float* Vh, long long ldv, int rows, const float* D, c
             case 128: st = launch_pass1<128>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
             case 256: st = launch_pass1<256>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
             case 512: st = launch_pass1<512>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
-            default: st = launch_pass1_w(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
+            default: st = launch_pass1_w(v, ldvp, nr, d, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, n / 2 + 1, nullptr, s); break;
         }
         if (st) break;
         switch (N2) {

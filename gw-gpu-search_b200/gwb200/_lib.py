@@ -52,6 +52,9 @@ SIGNATURES = {
     'gwb_fourstep_order': [_P, _LL, _I, _P, _LL, _LL, _P, _LL, _P],
     'gwb_basis_fused': [_P, _LL, _I, _P, _LL, _P, _P, _I, _LL, _LL, _I, _P, _P, _LL, _I, _I, _I, _P, _LL, _P, _P, _P,
                         _P, _LL, _P],
+    'gwb_fourstep_order_ends': [_P, _LL, _I, _P, _LL, _LL, _P, _LL, _P, _P, _P],
+    'gwb_basis_fused_band': [_P, _LL, _I, _P, _LL, _P, _P, _I, _LL, _LL, _I, _P, _P, _LL, _I, _I, _I, _P, _LL, _P, _P,
+                             _P, _P, _LL, _LL, _P, _P],
     'gwb_basis_fused_ring': [_P, _LL, _I, _P, _LL, _P, _P, _I, _LL, _LL, _I, _P, _P, _LL, _I, _I, _P, _LL, _P, _P, _P,
                              _LL, _P, _LL, _P],
     'gwb_basis_series': [_P, _LL, _I, _P, _P, _LL, _LL, _P, _P, _P, _P, _I, _LL, _LL, _I, _P, _P, _LL, _I, _P, _LL, _P, _P],

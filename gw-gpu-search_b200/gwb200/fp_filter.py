@@ -144,18 +144,19 @@ def twiddles(N, device='cuda'):
 FUSED_MIN, FUSED_MAX = 1 << 12, 1 << 20     # transform lengths of the fused basis series
 
 
-def fourstep_order(X, N, isw=None, out=None):
+def fourstep_order(X, N, isw=None, out=None, last_nz=None, last_bad=None):
     """Rows of a half spectrum (rows, flen) complex64 in the four-step order of a length-N transform: P[j, k2 (N1/2) +
     k1] = X[j, N2 k1 + k2] (times isw), P[j, N/2] = X[j, N/2] (gwb_fourstep_order); the input layout of the fused
-    basis series."""
+    basis series. last_nz (1,) and last_bad (rows,), int32: filled with the last bin of any row that is not zero, and
+    each row's last bin that is not finite (-1: none)."""
     _lib.require_cuda(X)
     X2 = X if X.dim() == 2 else X[None]
     rows, flen = X2.shape
     if out is None:
         # rows padded to an even length: 16-byte aligned rows for the fused pass's asynchronous copies
         out = torch.empty((rows, N // 2 + 2), dtype=torch.complex64, device=X.device)[:, :N // 2 + 1]
-    _lib.call('gwb_fourstep_order', _lib.ptr(X2), _lib.row_stride(X2), rows, _lib.ptr(isw), flen, int(N),
-              _lib.ptr(out), _lib.row_stride(out), _lib.stream_ptr(X.device))
+    _lib.call('gwb_fourstep_order_ends', _lib.ptr(X2), _lib.row_stride(X2), rows, _lib.ptr(isw), flen, int(N),
+              _lib.ptr(out), _lib.row_stride(out), _lib.ptr(last_nz), _lib.ptr(last_bad), _lib.stream_ptr(X.device))
     return out if X.dim() == 2 else out[0]
 
 
@@ -191,11 +192,12 @@ class FusedBasisWorkspace:
         self.rowpart = torch.empty((rows if self.ring else self.wrows) * n2, dtype=torch.float32, device=device)
 
 
-def basis_series_fused(ws, Vp, Dp, a0, Tn, Z, Zlo=None, form='f16', im_off=None):
+def basis_series_fused(ws, Vp, Dp, a0, Tn, Z, Zlo=None, form='f16', im_off=None, kend=None, last_bad=None):
     """Same Z as basis_series_into in two fused passes (gwb_basis_fused), from the basis filters Vp (r, tlen/2 + 1) and
     one segment's D isw Dp (tlen/2 + 1,), both in four-step order (fourstep_order). The scale is the whole-series rms
     of the first min(RB, wrows) rows by Parseval instead of the analysed-span rms (it cancels between Z and A).
-    Returns the device scale; for form 'fp8' Z row j holds z_j / ws.rowscale[j] in e4m3 instead."""
+    Returns the device scale; for form 'fp8' Z row j holds z_j / ws.rowscale[j] in e4m3 instead. kend: Vp is zero from
+    this bin on, with last_bad (device int32) the data's last non-finite bin (gwb_basis_fused_band)."""
     r = Vp.shape[0]
     assert r <= ws.rows and Vp.shape[1] >= ws.tlen // 2 + 1 and Dp.numel() >= ws.tlen // 2 + 1
     im_off = r if im_off is None else im_off
@@ -206,11 +208,11 @@ def basis_series_fused(ws, Vp, Dp, a0, Tn, Z, Zlo=None, form='f16', im_off=None)
                   0, _lib.ptr(ws.partials), ws.partials.numel(), _lib.ptr(ws.scale), _lib.ptr(ws.rowscale),
                   _lib.ptr(ws.rowpart), ws.rowpart.numel(), _lib.ptr(ws.sync), ws.sync.numel(), _lib.stream_ptr())
         return ws.scale
-    _lib.call('gwb_basis_fused', _lib.ptr(Vp), Vp.stride(0), r, _lib.ptr(Dp), ws.tlen, _lib.ptr(ws.tw),
+    _lib.call('gwb_basis_fused_band', _lib.ptr(Vp), Vp.stride(0), r, _lib.ptr(Dp), ws.tlen, _lib.ptr(ws.tw),
               _lib.ptr(ws.W), ws.wrows, int(a0), int(Tn), FORMS[form], _lib.ptr(Z), _lib.ptr(Zlo), Z.stride(0),
               int(im_off), 0, min(ws.nfirst, r), _lib.ptr(ws.partials), ws.partials.numel(), _lib.ptr(ws.ticket),
               _lib.ptr(ws.scale), _lib.ptr(ws.rowscale), _lib.ptr(ws.rowpart), ws.rowpart.numel(),
-              _lib.stream_ptr())
+              ws.tlen // 2 + 1 if kend is None else int(kend), _lib.ptr(last_bad), _lib.stream_ptr())
     return ws.scale
 
 

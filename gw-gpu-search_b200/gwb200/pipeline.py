@@ -122,7 +122,11 @@ class MatchedFilter:
             self.fws = fp_filter.FusedBasisWorkspace(tlen, bank.flen, rmax, device, wrows=bt.get('wrows'),
                                                      ring=bt.get('ring'))
             # basis filters in the four-step order of the transform, once per tile; D isw per step (self.Dp)
-            self.vp = [fp_filter.fourstep_order(s['Vh'], tlen) for s in bank.svd]
+            # and, read from the filters themselves, the bin from which each tile's are zero (its last f_ISCO)
+            ends = torch.empty(len(bank.svd), dtype=torch.int32, device=device)
+            self.vp = [fp_filter.fourstep_order(s['Vh'], tlen, last_nz=ends[t:t + 1]) for t, s in enumerate(bank.svd)]
+            self.kend = [int(e) + 1 for e in ends.cpu()]
+            self.last_bad = None
             self.Dp = None
         else:
             self.ws = fp_filter.BasisWorkspace(tlen, bank.flen, fp_filter.RB, device)
@@ -240,7 +244,8 @@ class MatchedFilter:
         im_off = Kh if self.compact else r
         if self.fused:
             scale = fp_filter.basis_series_fused(self.fws, self.vp[t], self.Dp[seg], self.a0, self.Tn, self.Z,
-                                                 self.Zlo, self.form, im_off=im_off)
+                                                 self.Zlo, self.form, im_off=im_off, kend=self.kend[t],
+                                                 last_bad=None if self.last_bad is None else self.last_bad[seg:seg + 1])
         else:
             scale = fp_filter.basis_series_into(self.ws, sv['Vh'], D[seg], isw, self.a0, self.Tn, self.Z,
                                                 self.Zlo, self.form, im_off=im_off)
@@ -357,7 +362,8 @@ class MatchedFilter:
             # every segment's D isw in four-step order, shared by all tiles
             if self.Dp is None or self.Dp.shape[0] != D.shape[0]:
                 self.Dp = torch.empty((D.shape[0], self.tlen // 2 + 1), dtype=torch.complex64, device=D.device)
-            fp_filter.fourstep_order(D, self.tlen, isw, out=self.Dp)
+                self.last_bad = torch.empty(D.shape[0], dtype=torch.int32, device=D.device)
+            fp_filter.fourstep_order(D, self.tlen, isw, out=self.Dp, last_bad=self.last_bad)
             self.kernel_launches += 1
         if prof is not None:
             e_f[1].record()

@@ -306,6 +306,11 @@ GWB_API int gwb_fft_twiddles(long long N, float* tw, void* stream);
  * P[j][N/2] = X[j][N/2] isw[N/2], zero where k >= flen (isw NULL: no weight). ldp >= N/2 + 1. */
 GWB_API int gwb_fourstep_order(const float* X, long long ldx, int rows, const float* isw, long long flen, long long N,
                                float* P, long long ldp, void* stream);
+/* gwb_fourstep_order that also tells where the rows end: last_nz (1 int, or NULL) = the largest k of any row whose value
+ * is not zero, last_bad (rows ints, or NULL) = per row the largest k whose value is not finite; -1 where there is none. */
+GWB_API int gwb_fourstep_order_ends(const float* X, long long ldx, int rows, const float* isw, long long flen,
+                                    long long N, float* P, long long ldp, int32_t* last_nz, int32_t* last_bad,
+                                    void* stream);
 /* form 4 (fp8 e4m3, the screening form; no reference counterpart): each basis row j gets its own scale,
  * rowscale[j] = (rms of one component of its series) / 16 from the row's |q|^2 sums (Parseval), and Z rows hold
  * z_j / rowscale[j] in e4m3 (saturating). rowscale: rows floats (out); rowpart: workspace of min(rows, wrows) x P
@@ -314,6 +319,15 @@ GWB_API int gwb_basis_fused(const float* Vp, long long ldvp, int rows, const flo
                             float* W, int wrows, long long a0, long long Tn, int form, void* Z, void* Zlo, long long ldz,
                             int im_off, int row0, int nfirst, double* partials, long long npartials, uint32_t* ticket,
                             float* scale, float* rowscale, float* rowpart, long long rowpart_elems, void* stream);
+/* gwb_basis_fused for basis filters that are zero from bin kend on (last_nz + 1 of gwb_fourstep_order_ends): at N = 2^19
+ * and 2^20 the first pass neither loads nor transforms what lies past it. Same Z bits (up to the sign of zeros).
+ * last_bad (device int, or NULL): the data's last non-finite bin; at or past kend it makes every output NaN, as 0 * inf
+ * does without the limit. */
+GWB_API int gwb_basis_fused_band(const float* Vp, long long ldvp, int rows, const float* Dp, long long N,
+                                 const float* tw, float* W, int wrows, long long a0, long long Tn, int form, void* Z,
+                                 void* Zlo, long long ldz, int im_off, int row0, int nfirst, double* partials,
+                                 long long npartials, uint32_t* ticket, float* scale, float* rowscale, float* rowpart,
+                                 long long rowpart_elems, long long kend, const int32_t* last_bad, void* stream);
 /* Columns of the transform per pass-2 CTA of gwb_basis_fused at N = 2^20, process-wide per Z form (0-4 as
  * gwb_basis_fused's `form`; -1 sets every form): 16 (default; a CTA writes runs of 16 consecutive Z samples: whole
  * 32-byte sectors for 16-bit Z, one 512-thread CTA per SM) or 8 (runs of 8, twice the L2 write requests).
