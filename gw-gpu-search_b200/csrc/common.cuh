@@ -118,6 +118,21 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     }
 }
 
+// A value that is the same in every lane, as such to the compiler: what is derived from it can live in uniform registers.
+__device__ __forceinline__ int warp_uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+
+// One lane of a converged warp (the same lane at every call of the warp).
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+// mbar_wait_bounded by a whole warp: the same answer in every lane
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // TMA. No TMA or bulk load in this library uses cluster multicast; the only multicast is umma_commit_pair's
 // tcgen05.commit, an mbarrier arrive on the two CTAs of one CTA pair on the same GPU.

@@ -19,7 +19,8 @@
 // Work split: gridDim.x CTAs (or, where whole groups would divide unevenly, pairs of CTAs) take contiguous runs of
 // output groups; the two CTAs of a pair (a cluster) halve their run at a tile, and a group cut there is merged through
 // distributed shared memory at the end. 448 windows over 148 CTAs are 3.03 each, 4 at most; over 74 pairs 7 for two.
-// Measured: 256 x 64 split bf16 by 917,504 samples, 1 s windows, 247 -> 209 us; 1,024 x 128 fp16 by 2^20, 636 -> 615.
+// Measured with the warp-wide issue loop below: 256 x 64 split bf16 by 917,504 samples, 1 s windows, 247 -> 159 us a call
+// (209 with a one-lane loop; kernel 141, 1,282 TFLOP/s issued); 1,024 x 128 fp16 by 2^20, 636 -> 511 (615; 1,266).
 // Operands: A is K-major (row = template, K contiguous), Z is MN-major (K rows, samples contiguous); both are staged
 // by TMA with the 128-byte swizzle. No multicast. Every wait is bounded (one second) and records GWB_ERR_TIMEOUT.
 #include "common.cuh"
@@ -124,7 +125,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_absmax_kernel(const __grid_c
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * 256;
     const int MBe = min(2, (args.M - m0 + 127) / 128);
     const int pair = args.pair, rank = pair ? (int)(blockIdx.x & 1) : 0;
@@ -201,62 +202,76 @@ __global__ void __launch_bounds__(kThreads, 1) umma_absmax_kernel(const __grid_c
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t idesc = instr_desc(128, 128, C::FMT, C::FMT, 0, 1);
-            const uint32_t a_base = smem_u32(sA), z_base = smem_u32(sZ);
-            bool ok = mbar_wait_bounded(barA, 0);
+        // The whole warp runs the loop and one elected lane issues: descriptors, TMEM addresses and loop state are then
+        // warp-uniform and stay in the uniform registers that tcgen05.mma reads (in a one-lane branch each operand of
+        // each MMA was moved there first, and the issue loop, not the MMAs, set the time of a tile).
+        const bool el = elect_lane();
+        const uint32_t tm = (uint32_t)warp_uniform((int)tmem);
+        const uint32_t idesc = instr_desc(128, 128, C::FMT, C::FMT, 0, 1);
+        const uint32_t a_base = smem_u32(sA), z_base = smem_u32(sZ);
+        bool ok = mbar_wait_warp(barA, 0);
+        if (!ok) {
+            record_error(args.err, GWB_ERR_TIMEOUT, 102, blockIdx.x, 0);
+            *abort_flag = 1;
+        }
+        tc_fence_after();
+        int s = 0;
+        uint32_t ph = 0;                                   // stage and its phase
+        for (int i = 0; i < ntl && ok; ++i) {
+            ok = __all_sync(0xffffffffu, *abort_flag == 0) && mbar_wait_warp(&full[s], ph);
             if (!ok) {
-                record_error(args.err, GWB_ERR_TIMEOUT, 102, blockIdx.x, 0);
+                record_error(args.err, GWB_ERR_TIMEOUT, 103, blockIdx.x, i);
                 *abort_flag = 1;
+                break;
             }
             tc_fence_after();
-            for (int i = 0; i < ntl && ok; ++i) {
-                const int s = i % S;
-                if (*abort_flag || !mbar_wait_bounded(&full[s], (uint32_t)((i / S) & 1))) {
-                    record_error(args.err, GWB_ERR_TIMEOUT, 103, blockIdx.x, i);
+            for (int mb = 0; mb < MBe; ++mb) {
+                const int j = i * MBe + mb, b = j & 1;
+                ok = mbar_wait_warp(&tempty[b], (uint32_t)(((j >> 1) & 1) ^ 1));
+                if (!ok) {
+                    record_error(args.err, GWB_ERR_TIMEOUT, 104, blockIdx.x, i);
                     *abort_flag = 1;
                     break;
                 }
                 tc_fence_after();
-                for (int mb = 0; mb < MBe; ++mb) {
-                    const int j = i * MBe + mb, b = j & 1;
-                    const uint32_t u = (uint32_t)(j >> 1);
-                    if (!mbar_wait_bounded(&tempty[b], (u & 1) ^ 1)) {
-                        record_error(args.err, GWB_ERR_TIMEOUT, 104, blockIdx.x, i);
-                        *abort_flag = 1;
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    for (int ri = 0; ri < 2; ++ri) {
-                        const uint32_t d = tmem + (uint32_t)(b * 256 + ri * 128);
-                        uint32_t acc = 0;
-                        for (int pr = 0; pr < C::NPROD; ++pr) {
-                            // products: (A hi, Z hi), (A hi, Z lo), (A lo, Z hi)
-                            const int a = (pr == 2 ? 2 : 0) + ri;
-                            const int z = (pr == 1) ? 1 : 0;
-                            // descriptors advance by K steps of 16: 32 bytes of a 64-wide A box, 2048 of Z
-                            uint64_t ad = smem_desc(a_base + (mb * C::NA + a) * nkc * kATileBytes, 16, 1024, 2);
-                            uint64_t bd = smem_desc(z_base + s * L.stage_bytes + (z * 2) * K * 128, (uint32_t)K * 128u,
-                                                    1024, 2);
-                            for (int kc = 0; kc < nkc; ++kc) {
+                for (int ri = 0; ri < 2; ++ri) {
+                    const uint32_t d = tm + (uint32_t)(b * 256 + ri * 128);
+                    uint32_t acc = 0;
 #pragma unroll
-                                for (int k16 = 0; k16 < 4; ++k16) {
-                                    umma_f16(d, ad + k16 * (32 >> 4), bd + k16 * (2048 >> 4), idesc, acc);
-                                    acc = 1;
-                                }
-                                ad += kATileBytes >> 4;
-                                bd += 4 * 2048 >> 4;
+                    for (int pr = 0; pr < C::NPROD; ++pr) {
+                        // products: (A hi, Z hi), (A hi, Z lo), (A lo, Z hi)
+                        const int a = (pr == 2 ? 2 : 0) + ri;
+                        const int z = (pr == 1) ? 1 : 0;
+                        // descriptors advance by K steps of 16: 32 bytes of a 64-wide A box, 2048 of Z
+                        uint64_t ad = smem_desc(a_base + (mb * C::NA + a) * nkc * kATileBytes, 16, 1024, 2);
+                        uint64_t bd = smem_desc(z_base + s * L.stage_bytes + (z * 2) * K * 128, (uint32_t)K * 128u, 1024,
+                                                2);
+                        for (int kc = 0; kc < nkc; ++kc) {
+                            if (el) {
+                                umma_f16(d, ad, bd, idesc, acc);
+                                umma_f16(d, ad + (32 >> 4), bd + (2048 >> 4), idesc, 1);
+                                umma_f16(d, ad + (64 >> 4), bd + (4096 >> 4), idesc, 1);
+                                umma_f16(d, ad + (96 >> 4), bd + (6144 >> 4), idesc, 1);
                             }
+                            acc = 1;
+                            ad += kATileBytes >> 4;
+                            bd += 4 * 2048 >> 4;
                         }
                     }
-                    umma_commit(&tfull[b]);
                 }
-                umma_commit(&empty[s]);
+                if (el) umma_commit(&tfull[b]);
             }
-            umma_commit(done);
-            mbar_wait_bounded(done, 0);
+            if (!ok) break;
+            if (el) umma_commit(&empty[s]);
+            if (++s == S) {
+                s = 0;
+                ph ^= 1;
+            }
         }
+        __syncwarp();
+        if (el) umma_commit(done);
+        __syncwarp();
+        mbar_wait_bounded(done, 0);
         __syncwarp();
     } else {
         // ---------------- epilogue ----------------
