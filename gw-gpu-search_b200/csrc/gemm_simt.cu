@@ -140,19 +140,21 @@ __global__ void __launch_bounds__(256) simt_absmax_kernel(const float* __restric
 // scheduler. So:
 //  - FMAs go in pairs (fma.rn.f32x2: two samples of a row per instruction, each rounded as fmaf), which halves the
 //    issue slots they take and leaves the others for shared-memory reads and the duplicated A values;
-//  - operand tiles are copied by cp.async through a ring of AS_ST stages while earlier ones are multiplied (16-byte
-//    copies where K, lda, ldz and the bases allow, else 4-byte ones: the arithmetic is the same);
+//  - operand tiles are copied by cp.async through a ring of AS_ST stages while earlier ones are multiplied (Z in 16-byte
+//    copies where ldz and the base allow, else 4-byte ones: the arithmetic is the same);
 //  - CTAs of 128 threads own 64 rows, two per SM, so one's barriers and epilogue pass under the other's FMAs and a
 //    row count is padded to 64, not 128;
 //  - a window is shared out over a cluster of SPL CTAs (each walks its part of the blocks; rank 0 merges the maxima
 //    in block order through distributed shared memory), so that the last wave is a quarter of a window long.
 // Sums run over k in order with one rounding per FMA, so results are bit-identical to the kernel above.
-// Measured, 248 x 192 by 192 x 458,700, 1 s windows: 2,526 -> 1,939 us (45 TFLOP/s); 64 templates x 118 rows of K by
-// 475,136 samples: 855 -> 430 us (half the rows were padding).
-// Thread (tx, ty) owns rows ty + 8 i (i < 8) and samples 4 tx + j, 64 + 4 tx + j (j < 4): the A reads of a warp
-// (two rows, one float4 each) fall in distinct banks, the Z reads are two runs of 256 contiguous bytes.
+// Measured, 248 x 192 by 192 x 458,700, 1 s windows: 2,526 -> 1,759 us (49.7 TFLOP/s; 1,935 with pairs along samples, 16
+// duplicated A values per k); 64 templates x 118 rows of K by 475,136 samples: 855 -> 338 us (half the rows were padding).
+// Pairs run along rows: A lies k-major in shared memory (4-byte copies), so a pair of rows is one register pair as read,
+// and only the 8 samples of a k are duplicated, not 16 A values. Thread (tx, ty) owns rows 8 ty .. 8 ty + 7 and samples
+// 4 tx + j, 64 + 4 tx + j (j < 4): a warp's A reads are two broadcast float4, its Z reads two runs of 256 bytes.
 constexpr int AS_ST = 3, AS_BM = 64, AS_NT = 128, AS_MAXSPL = 4;
-constexpr int AS_STAGE = (2 * AS_BM + BN) * BK;  // floats per stage: A re, A im (AS_BM x BK, row-major), Z (BK x BN)
+constexpr int AS_LD = AS_BM + 4;                 // floats per k of an A tile (k-major; rows on 16-byte boundaries)
+constexpr int AS_STAGE = (2 * AS_LD + BN) * BK;  // floats per stage: A re, A im (BK x AS_LD), Z (BK x BN)
 
 // N bytes (16 or 4) to shared memory, zero past the first src_bytes
 template <int N>
@@ -200,19 +202,19 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
     const int nsteps = (t1 - t0) * nk;
     auto load = [&](int step) {
         float* sAr = smf + (step % AS_ST) * AS_STAGE;
-        float* sAi = sAr + AS_BM * BK;
-        float* sZ = sAi + AS_BM * BK;
+        float* sAi = sAr + AS_LD * BK;
+        float* sZ = sAi + AS_LD * BK;
         const int t = t0 + step / nk, k0 = (step % nk) * BK;
         constexpr int E = VEC ? 4 : 1;           // elements per copy
 #pragma unroll
-        for (int r = 0; r < AS_BM * BK / E / AS_NT; ++r) {       // A: 64 rows x 16 k
+        for (int r = 0; r < AS_BM * BK / AS_NT; ++r) {           // A: 64 rows x 16 k, transposed
             const int e = tid + AS_NT * r;
-            const int row = e / (BK / E), kq = e % (BK / E) * E;
-            const int gr = m0 + row, gk = k0 + kq;
+            const int row = e / BK, kk = e % BK;
+            const int gr = m0 + row, gk = k0 + kk;
             const bool ok = gr < M && gk < K;
             const long long off = ok ? (long long)gr * lda + gk : 0;
-            cp_async_zfill<4 * E>(sAr + row * BK + kq, Are + off, ok ? 4 * E : 0);
-            cp_async_zfill<4 * E>(sAi + row * BK + kq, Aim + off, ok ? 4 * E : 0);
+            cp_async_zfill<4>(sAr + kk * AS_LD + row, Are + off, ok ? 4 : 0);
+            cp_async_zfill<4>(sAi + kk * AS_LD + row, Aim + off, ok ? 4 : 0);
         }
 #pragma unroll
         for (int r = 0; r < BK * BN / E / AS_NT; ++r) {          // Z: 16 k x 128 samples
@@ -226,14 +228,16 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
     };
     float wb[8];
     int wi[8];
-    pair32 ar[8][4], ai[8][4];                   // samples (4 tx, +1), (+2, +3), (64 + 4 tx, +1), (+2, +3)
+    pair32 ar[4][8], ai[4][8];                   // rows (2 i, 2 i + 1), samples 4 tx + j, 64 + 4 tx + j
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         wb[i] = -2.f;                            // below every block's maximum (at least -1)
         wi[i] = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) ar[i][j] = ai[i][j] = 0ull;
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ar[i][j] = ai[i][j] = 0ull;
 #pragma unroll
     for (int s = 0; s < AS_ST - 1; ++s) {
         if (s < nsteps) load(s);
@@ -245,30 +249,23 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
         if (step + AS_ST - 1 < nsteps) load(step + AS_ST - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const float* sAr = smf + (step % AS_ST) * AS_STAGE;
-        const float* sAi = sAr + AS_BM * BK;
-        const float* sZ = sAi + AS_BM * BK;
+        const float* sAi = sAr + AS_LD * BK;
+        const float* sZ = sAi + AS_LD * BK;
 #pragma unroll
-        for (int kq = 0; kq < BK; kq += 4) {
-            float4 a4r[8], a4i[8];
+        for (int kk = 0; kk < BK; ++kk) {
+            const float4 z0 = *reinterpret_cast<const float4*>(sZ + kk * BN + 4 * tx);
+            const float4 z1 = *reinterpret_cast<const float4*>(sZ + kk * BN + 64 + 4 * tx);
+            const pair32 z[8] = {dup(z0.x), dup(z0.y), dup(z0.z), dup(z0.w), dup(z1.x), dup(z1.y), dup(z1.z), dup(z1.w)};
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                a4r[i] = *reinterpret_cast<const float4*>(sAr + (ty + 8 * i) * BK + kq);
-                a4i[i] = *reinterpret_cast<const float4*>(sAi + (ty + 8 * i) * BK + kq);
-            }
+            for (int h = 0; h < 2; ++h) {
+                const ulonglong2 r2 = *reinterpret_cast<const ulonglong2*>(sAr + kk * AS_LD + 8 * ty + 4 * h);
+                const ulonglong2 i2 = *reinterpret_cast<const ulonglong2*>(sAi + kk * AS_LD + 8 * ty + 4 * h);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-                const ulonglong2 z0 = *reinterpret_cast<const ulonglong2*>(sZ + (kq + kk) * BN + 4 * tx);
-                const ulonglong2 z1 = *reinterpret_cast<const ulonglong2*>(sZ + (kq + kk) * BN + 64 + 4 * tx);
-                const pair32 z[4] = {z0.x, z0.y, z1.x, z1.y};
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const pair32 r2 = dup(kk == 0 ? a4r[i].x : kk == 1 ? a4r[i].y : kk == 2 ? a4r[i].z : a4r[i].w);
-                    const pair32 i2 = dup(kk == 0 ? a4i[i].x : kk == 1 ? a4i[i].y : kk == 2 ? a4i[i].z : a4i[i].w);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        fma2(ar[i][j], r2, z[j]);
-                        fma2(ai[i][j], i2, z[j]);
-                    }
+                for (int j = 0; j < 8; ++j) {
+                    fma2(ar[2 * h][j], r2.x, z[j]);
+                    fma2(ar[2 * h + 1][j], r2.y, z[j]);
+                    fma2(ai[2 * h][j], i2.x, z[j]);
+                    fma2(ai[2 * h + 1][j], i2.y, z[j]);
                 }
             }
         }
@@ -282,20 +279,15 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
                 float best = -1.f;
                 int bi = 0;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 re = unpack(ar[i][j]), im = unpack(ai[i][j]);
-                    const int cc = (j < 2 ? 0 : 64) + 4 * tx + 2 * (j & 1);
-                    const float p0 = (c0 + cc < Tn) ? fmaf(re.x, re.x, im.x * im.x) : -1.f;
-                    const float p1 = (c0 + cc + 1 < Tn) ? fmaf(re.y, re.y, im.y * im.y) : -1.f;
-                    if (p0 > best) {
-                        best = p0;
+                for (int j = 0; j < 8; ++j) {
+                    const float2 re = unpack(ar[i / 2][j]), im = unpack(ai[i / 2][j]);
+                    const float xr = i & 1 ? re.y : re.x, xi = i & 1 ? im.y : im.x;
+                    const int cc = (j < 4 ? 4 * tx + j : 64 + 4 * tx + (j - 4));
+                    const float p = (c0 + cc < Tn) ? fmaf(xr, xr, xi * xi) : -1.f;
+                    if (p > best) {
+                        best = p;
                         bi = cc;
                     }
-                    if (p1 > best) {
-                        best = p1;
-                        bi = cc + 1;
-                    }
-                    ar[i][j] = ai[i][j] = 0ull;
                 }
 #pragma unroll
                 for (int off = 8; off > 0; off >>= 1) {
@@ -308,6 +300,10 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
                     wi[i] = (int)(c0 + bi);
                 }
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) ar[i][j] = ai[i][j] = 0ull;
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -316,8 +312,8 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
         if (tx == 0) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                s_best[ty + 8 * i] = wb[i];
-                s_idx[ty + 8 * i] = wi[i];
+                s_best[8 * ty + i] = wb[i];
+                s_idx[8 * ty + i] = wi[i];
             }
         }
         cg::cluster_group cl = cg::this_cluster();
@@ -341,7 +337,7 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
     } else if (tx == 0) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int row = m0 + ty + 8 * i;
+            const int row = m0 + 8 * ty + i;
             if (row < M) {
                 V[(long long)row * ldv + o] = wb[i];
                 I[(long long)row * ldv + o] = wi[i];
@@ -399,8 +395,7 @@ extern "C" int gwb_fused_peaks_f32(const float* Are, const float* Aim, long long
     GWB_CHECK_ARG(ldv >= nout, GWB_ERR_SHAPE, "fused_peaks_f32: ldv=%lld < outputs per row %lld", ldv, nout);
     GWB_CHECK_ARG(nout < (1ll << 31), GWB_ERR_SHAPE, "fused_peaks_f32: too many outputs");
     if (g_f32_async.load() && cdiv(M, AS_BM) <= 65535) {
-        const bool vec = K % 4 == 0 && lda % 4 == 0 && ldz % 4 == 0 && aligned(Are, 16) && aligned(Aim, 16) &&
-                         aligned(Z, 16);
+        const bool vec = ldz % 4 == 0 && aligned(Z, 16);        // 16-byte copies of Z
         // windows are shared out over clusters while whole windows would leave the last of few waves nearly empty
         // (two CTAs per SM; from 32 waves on it is a thirty-second at most) and a part still holds two blocks
         const long long items = nout * cdiv(M, AS_BM);
