@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int m0 = blockIdx.y * 128 * MB;
     const int MBe = min(MB, (args.M - m0 + 127) / 128);
     int t_begin, t_end;
@@ -202,11 +202,15 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        // the whole warp runs the loop and one elected lane issues, so that descriptors, TMEM addresses and loop state stay
+        // in the uniform registers that tcgen05.mma reads
+        {
+            const bool el = elect_lane();
+            const uint32_t tm = (uint32_t)warp_uniform((int)tmem);
             const uint32_t idesc = instr_desc(128, 128, C::FMT, C::FMT, 0, 1);
             const uint32_t idesc_neg = idesc | (1u << 13);     // negate A
             const uint32_t a_base = smem_u32(sA), z_base = smem_u32(sZ);
-            bool ok = mbar_wait_bounded(barA, 0);
+            bool ok = mbar_wait_warp(barA, 0);
             if (!ok) {
                 record_error(args.err, GWB_ERR_TIMEOUT, 202, blockIdx.x, 0);
                 *abort_flag = 1;
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
             auto issue = [&](int kc, int mb, int b, uint32_t st) {
                 if constexpr (C::NPROD == 1) {
                     constexpr int MAXS = 4;                      // K steps per chunk: KC / KSTEP (64/16, 128/32)
-                    const uint32_t dre = tmem + (uint32_t)(b * 256), dim = dre + 128;
+                    const uint32_t dre = tm + (uint32_t)(b * 256), dim = dre + 128;
                     const int nsteps = min(KC, Kh - kc * KC) / C::KSTEP;
                     const uint32_t abase = a_base + mb * L.a_tiles * kATile;
                     // base descriptors of the chunk plus byte offsets >> 4 (the start-address field, bits 0-13;
@@ -243,6 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                     for (int sk = 0; sk < MAXS; ++sk) {
                         if (sk >= nsteps) break;
                         const uint32_t acc = (kc > 0 || sk > 0) ? 1u : 0u;
+                        if (!el) continue;
                         if constexpr (C::F8) {
                             umma_f8(dre, dAre[sk], dZre[sk], idesc, acc);
                             umma_f8(dre, dAim[sk], dZim[sk], idesc_neg, 1u);
@@ -256,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                         }
                     }
                 } else {
-                    const uint32_t dre = tmem + (uint32_t)(b * 256), dim = dre + 128;
+                    const uint32_t dre = tm + (uint32_t)(b * 256), dim = dre + 128;
                     const int nsteps = min(KC, Kh - kc * KC) / C::KSTEP;
                     for (int sk = 0; sk < nsteps; ++sk) {
                         const int k = kc * KC + sk * C::KSTEP;
@@ -288,6 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                             const uint64_t dZre = smem_desc(zre, (uint32_t)KC * 128u, 1024, 2);
                             const uint64_t dZim = smem_desc(zim, (uint32_t)KC * 128u, 1024, 2);
                             const uint32_t acc = (kc > 0 || sk > 0 || pr > 0) ? 1u : 0u;
+                            if (!el) continue;
                             if constexpr (C::F8) {
                                 umma_f8(dre, dAre, dZre, idesc, acc);
                                 umma_f8(dre, dAim, dZim, idesc_neg, 1u);
@@ -306,7 +312,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
             // this item's accumulators must have been read out by the epilogue
             auto wait_tempty = [&](int i, int j) {
                 const uint32_t u = (uint32_t)(j >> 1);
-                if (!mbar_wait_bounded(&tempty[j & 1], (u & 1) ^ 1)) {
+                if (!mbar_wait_warp(&tempty[j & 1], (u & 1) ^ 1)) {
                     record_error(args.err, GWB_ERR_TIMEOUT, 204, blockIdx.x, i);
                     *abort_flag = 1;
                     return false;
@@ -315,7 +321,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                 return true;
             };
             auto wait_full = [&](int f) {
-                if (*abort_flag || !mbar_wait_bounded(&full[f % S], (uint32_t)((f / S) & 1))) {
+                if (!__all_sync(0xffffffffu, *abort_flag == 0) || !mbar_wait_warp(&full[f % S], (uint32_t)((f / S) & 1))) {
                     record_error(args.err, GWB_ERR_TIMEOUT, 203, blockIdx.x, f);
                     *abort_flag = 1;
                     return false;
@@ -336,9 +342,9 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                             if (mb == 0 && !(ok = wait_full(f))) break;
                             if (kc == 0 && !(ok = wait_tempty(i, j))) break;
                             issue(kc, mb, j & 1, z_base + (f % S) * L.stage_bytes);
-                            if (mb == MBe - 1) umma_commit(&empty[f % S]);
+                            if (mb == MBe - 1 && el) umma_commit(&empty[f % S]);
                         }
-                        if (ok) umma_commit(&tfull[j & 1]);
+                        if (ok && el) umma_commit(&tfull[j & 1]);
                     }
                 } else {
                     for (int kc = 0; kc < nkc && ok; ++kc) {
@@ -349,13 +355,15 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                             if (kc == 0 && !(ok = wait_tempty(i, j))) break;
                             issue(kc, mb, j & 1, z_base + (f % S) * L.stage_bytes);
                         }
-                        umma_commit(&empty[f % S]);
+                        if (el) umma_commit(&empty[f % S]);
                     }
-                    if (ok)
+                    if (ok && el)
                         for (int mb = 0; mb < MBe; ++mb) umma_commit(&tfull[(i * MBe + mb) & 1]);
                 }
             }
-            umma_commit(done);
+            __syncwarp();
+            if (el) umma_commit(done);
+            __syncwarp();
             mbar_wait_bounded(done, 0);
         }
         __syncwarp();
@@ -533,8 +541,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_ctarank();
+    const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const uint32_t rank = (uint32_t)warp_uniform((int)cluster_ctarank());
     const bool leader = rank == 0;
     // a timeout in either CTA stops both: the flag is set here and in the peer (through its shared::cluster address)
     const uint32_t peer_abort = mapa_shared(smem_u32((const void*)abort_flag), rank ^ 1u);
@@ -621,7 +629,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
         }
     } else if (ntl > 0 && warp == 1) {
-        if (lane == 0 && leader) {
+        // the leader's whole warp runs the loop and one elected lane issues (as in the one-CTA kernel)
+        if (leader) {
+            const bool el = elect_lane();
+            const uint32_t tm = (uint32_t)warp_uniform((int)tmem);
             const uint32_t idesc = instr_desc(256, 128, C::FMT, C::FMT, 0, 1);
             const uint32_t idesc_neg = idesc | (1u << 13);  // negate A
             const int order = args.order;
@@ -629,7 +640,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             // descriptors of the resident A copies at K column 0 (the split forms add offsets to them)
             uint64_t ad0[2];
             for (int h = 0; h < 2; ++h) ad0[h] = smem_desc(a_base + (h < nres ? h : 0) * L.a_tiles * kATile, 16, 1024, 2);
-            bool ok = mbar_wait_bounded(barA, 0);
+            bool ok = mbar_wait_warp(barA, 0);
             if (!ok) {
                 record_error(args.err, GWB_ERR_TIMEOUT, 212, tr, 0);
                 abort_pair();
@@ -638,17 +649,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             for (int i = 0; i < ntl && ok; ++i) {
                 const int b = i & 1;
                 const uint32_t u = (uint32_t)(i >> 1);
-                if (!mbar_wait_bounded(&tempty[b], (u & 1) ^ 1)) {
+                if (!mbar_wait_warp(&tempty[b], (u & 1) ^ 1)) {
                     record_error(args.err, GWB_ERR_TIMEOUT, 214, tr, i);
                     abort_pair();
                     ok = false;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t dre = tmem + (uint32_t)(b * 256), dim = dre + 128;
+                const uint32_t dre = tm + (uint32_t)(b * 256), dim = dre + 128;
                 for (int kc = 0; kc < nkc && ok; ++kc) {
                     const int f = i * nkc + kc;
-                    if (*abort_flag || !mbar_wait_bounded(&full[f % S], (uint32_t)((f / S) & 1))) {
+                    if (!__all_sync(0xffffffffu, *abort_flag == 0) ||
+                        !mbar_wait_warp(&full[f % S], (uint32_t)((f / S) & 1))) {
                         record_error(args.err, GWB_ERR_TIMEOUT, 213, tr, f);
                         abort_pair();
                         ok = false;
@@ -670,31 +682,42 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         auto acc0 = [&](int sk) { return (kc > 0 || sk > 0) ? 1u : 0u; };
                         if (order == 1) {            // per K step, grouped by A half
                             for (int sk = 0; sk < nsteps; ++sk) {
-                                umma_f16_pair(dre, dA(sk, 0), dZ(sk, 0), idesc, acc0(sk));
-                                umma_f16_pair(dim, dA(sk, 0), dZ(sk, 1), idesc, acc0(sk));
-                                umma_f16_pair(dre, dA(sk, 1), dZ(sk, 1), idesc_neg, 1u);
-                                umma_f16_pair(dim, dA(sk, 1), dZ(sk, 0), idesc, 1u);
+                                const uint64_t ar = dA(sk, 0), ai = dA(sk, 1), zr = dZ(sk, 0), zi = dZ(sk, 1);
+                                const uint32_t acc = acc0(sk);
+                                if (el) {
+                                    umma_f16_pair(dre, ar, zr, idesc, acc);
+                                    umma_f16_pair(dim, ar, zi, idesc, acc);
+                                    umma_f16_pair(dre, ai, zi, idesc_neg, 1u);
+                                    umma_f16_pair(dim, ai, zr, idesc, 1u);
+                                }
                             }
                         } else if (order == 2) {     // the chunk's real-part MMAs, then its imaginary-part MMAs
-                            for (int sk = 0; sk < nsteps; ++sk) {
-                                umma_f16_pair(dre, dA(sk, 0), dZ(sk, 0), idesc, acc0(sk));
-                                umma_f16_pair(dre, dA(sk, 1), dZ(sk, 1), idesc_neg, 1u);
-                            }
-                            for (int sk = 0; sk < nsteps; ++sk) {
-                                umma_f16_pair(dim, dA(sk, 0), dZ(sk, 1), idesc, acc0(sk));
-                                umma_f16_pair(dim, dA(sk, 1), dZ(sk, 0), idesc, 1u);
-                            }
+                            for (int im = 0; im < 2; ++im)
+                                for (int sk = 0; sk < nsteps; ++sk) {
+                                    const uint64_t ar = dA(sk, 0), ai = dA(sk, 1), z0 = dZ(sk, im), z1 = dZ(sk, im ^ 1);
+                                    const uint32_t acc = acc0(sk), d = im ? dim : dre;
+                                    if (el) {
+                                        umma_f16_pair(d, ar, z0, idesc, acc);
+                                        umma_f16_pair(d, ai, z1, im ? idesc : idesc_neg, 1u);
+                                    }
+                                }
                         } else if (order == 3) {     // one product at a time over the chunk's K steps
-                            for (int sk = 0; sk < nsteps; ++sk) umma_f16_pair(dre, dA(sk, 0), dZ(sk, 0), idesc, acc0(sk));
-                            for (int sk = 0; sk < nsteps; ++sk) umma_f16_pair(dre, dA(sk, 1), dZ(sk, 1), idesc_neg, 1u);
-                            for (int sk = 0; sk < nsteps; ++sk) umma_f16_pair(dim, dA(sk, 0), dZ(sk, 1), idesc, acc0(sk));
-                            for (int sk = 0; sk < nsteps; ++sk) umma_f16_pair(dim, dA(sk, 1), dZ(sk, 0), idesc, 1u);
+                            for (int pr = 0; pr < 4; ++pr)
+                                for (int sk = 0; sk < nsteps; ++sk) {
+                                    const uint64_t ad = dA(sk, pr & 1), zd = dZ(sk, pr == 1 || pr == 2);
+                                    const uint32_t acc = pr & 1 ? 1u : acc0(sk);
+                                    if (el) umma_f16_pair(pr < 2 ? dre : dim, ad, zd, pr == 1 ? idesc_neg : idesc, acc);
+                                }
                         } else {                     // per K step: re += ReA ReZ, re -= ImA ImZ, im += ImA ReZ, += ReA ImZ
                             for (int sk = 0; sk < nsteps; ++sk) {
-                                umma_f16_pair(dre, dA(sk, 0), dZ(sk, 0), idesc, acc0(sk));
-                                umma_f16_pair(dre, dA(sk, 1), dZ(sk, 1), idesc_neg, 1u);
-                                umma_f16_pair(dim, dA(sk, 1), dZ(sk, 0), idesc, acc0(sk));
-                                umma_f16_pair(dim, dA(sk, 0), dZ(sk, 1), idesc, 1u);
+                                const uint64_t ar = dA(sk, 0), ai = dA(sk, 1), zr = dZ(sk, 0), zi = dZ(sk, 1);
+                                const uint32_t acc = acc0(sk);
+                                if (el) {
+                                    umma_f16_pair(dre, ar, zr, idesc, acc);
+                                    umma_f16_pair(dre, ai, zi, idesc_neg, 1u);
+                                    umma_f16_pair(dim, ai, zr, idesc, acc);
+                                    umma_f16_pair(dim, ar, zi, idesc, 1u);
+                                }
                             }
                         }
                     } else {
@@ -743,6 +766,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
                             for (int sk = 0; sk < MAXS; ++sk) {
                                 if (s0 + sk >= nsteps) break;
+                                if (!el) continue;
 #pragma unroll
                                 for (int pr = 0; pr < C::NPROD; ++pr) {
                                     const uint32_t acc = (kc > 0 || s0 + sk > 0 || pr > 0) ? 1u : 0u;
@@ -754,11 +778,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                             }
                         }
                     }
-                    umma_commit_pair(&empty[f % S]);
+                    if (el) umma_commit_pair(&empty[f % S]);
                 }
-                if (ok) umma_commit_pair(&tfull[b]);
+                if (ok && el) umma_commit_pair(&tfull[b]);
             }
-            umma_commit_pair(done);
+            __syncwarp();
+            if (el) umma_commit_pair(done);
         }
         __syncwarp();
         if (lane == 0 && !mbar_wait_bounded(done, 0)) {   // every MMA of the pair has completed
