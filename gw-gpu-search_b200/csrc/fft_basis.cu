@@ -817,7 +817,8 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
     float2* Bt = sm;                              // W tile (two blocks of TB columns), then the exchange tile
     float2* tw2 = Bt + TBW * SC;                  // tw2[u R2 + b] = e^{2 pi i b u / N2}
     const int tid = threadIdx.x, t10 = blockIdx.x * TBW;
-    const int j0 = blockIdx.y * RC, j1 = min(j0 + RC, rows);
+    // the last rows first: they are what the first pass left in L2 (128 rows, fp16: 340 -> 331 us)
+    const int j0 = (gridDim.y - 1 - blockIdx.y) * RC, j1 = min(j0 + RC, rows);
     auto fetch = [&](int j) {
         const char* g = reinterpret_cast<const char*>(W + (long long)j * N + (long long)blockIdx.x * (N2 * TBW));
         char* d = reinterpret_cast<char*>(Bt);
