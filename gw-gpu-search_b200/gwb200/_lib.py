@@ -174,13 +174,14 @@ def call(name, *args):
 
 
 def stream_ptr(device=None):
-    """The caller's current torch stream as the void* the C ABI takes."""
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+    """The caller's current torch stream as the void* the C ABI takes (an integer: no stream object per launch)."""
+    i = None if device is None else device if isinstance(device, int) else torch.device(device).index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
 
 def ptr(t):
     """Device pointer of a tensor (None -> NULL)."""
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def row_stride(t):
