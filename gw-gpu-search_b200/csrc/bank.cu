@@ -36,7 +36,8 @@ double* g_scratch_ptr[64] = {nullptr};
 // times the work. Bound: reading H at few segments, the float64 pipe at many (36.9 TFLOP/s with
 // this instruction, 33.7 with FMAs, whose operands came from shared memory at 2.5 reads per FMA issue slot).
 // 256 templates x 524,289 bins, against the FMA kernel with 64 x 64 blocks that this replaces:
-//   1,770 -> 216 us at 16 segments, 3,970 -> 211 at 4; 1,980 -> 26 for 64 templates x 262,145 bins at one segment.
+//   1,770 -> 215 us at 16 segments, 3,970 -> 211 at 4; 1,980 -> 26 for 64 templates x 262,145 bins at one segment; with
+//   the rows' ends known (kmax) 30 us at 4 segments and 15 at one.
 constexpr int kSR = 64, kSK = 32, kSB = kSK + 4;
 
 __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
@@ -48,17 +49,32 @@ __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
 template <int NT>
 __global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __restrict__ H, long long ldh, int n,
                                                              const float* __restrict__ IP, long long ldip, int nseg,
-                                                             int kmin, int flen, int kper,
+                                                             int kmin, int flen,
+                                                             const int32_t* __restrict__ kmax,
                                                              double* __restrict__ part) {
     extern __shared__ double s2_smem[];              // IP chunks [2][8 NT][kSB], then |H|^2 per warp [4][16][kSB]
     double (*Bs)[8 * NT * kSB] = reinterpret_cast<double (*)[8 * NT * kSB]>(s2_smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int fr = lane >> 2, fk = lane & 3;          // fragment row (A) or segment (B), and bin
     const int r0 = blockIdx.x * kSR + warp * 16, s0 = blockIdx.y * (8 * NT);
-    const int ka = kmin + blockIdx.z * kper, kb = min(flen, ka + kper);
+    // chunks of 32 bins are dealt out in turn: with contiguous ranges the few splits that cover a short band held it all
+    const int ka = kmin + (int)blockIdx.z * kSK, kstep = (int)gridDim.z * kSK, kb = flen;
     const float2* h = H + (long long)r0 * ldh + lane;
     const int nr = min(16, n - r0);                   // rows of this warp (none or fewer at the edge)
     double* A = s2_smem + 2 * 8 * NT * kSB + warp * 16 * kSB;
+    // the rows are zero from kmax on: past the block's last end nothing is multiplied, and IP is only looked at for values
+    // that are not finite, which make the segment's norms NaN (0 * inf)
+    __shared__ int s_kh, s_bad[8 * NT];
+    int kc = kb;                                      // end of the chunks that are multiplied
+    if (kmax) {
+        if (tid == 0) s_kh = 0;
+        for (int i = tid; i < 8 * NT; i += 128) s_bad[i] = 0;
+        __syncthreads();
+        const int kw = __reduce_max_sync(0xffffffffu, lane < nr ? kmax[r0 + lane] : 0);
+        if (lane == 0) atomicMax(&s_kh, kw);
+        __syncthreads();
+        kc = min(kb, kmin + (max(s_kh - kmin, 0) + kSK - 1) / kSK * kSK);      // whole chunks
+    }
     double acc[2][NT][2];
 #pragma unroll
     for (int f = 0; f < 2; ++f)
@@ -69,16 +85,17 @@ __global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __res
     auto load = [&](int k0) {
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-            hv[i] = (i < nr && k0 + lane < kb) ? __ldg(h + (long long)i * ldh + k0) : make_float2(0.f, 0.f);
+            hv[i] = (i < nr && k0 + lane < kc) ? __ldg(h + (long long)i * ldh + k0) : make_float2(0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < 2 * NT; ++i) {            // 32 consecutive bins of one segment per warp
             const int sg = s0 + warp + 4 * i, k = k0 + lane;
-            iv[i] = (sg < nseg && k < kb) ? __ldg(IP + (long long)sg * ldip + k) : 0.f;
+            iv[i] = (sg < nseg && k < kc) ? __ldg(IP + (long long)sg * ldip + k) : 0.f;
         }
     };
-    load(ka);
+    if (ka < kc) load(ka);
     int buf = 0;
-    for (int k0 = ka; k0 < kb; k0 += kSK, buf ^= 1) {
+    int k0 = ka;
+    for (; k0 < kc; k0 += kstep, buf ^= 1) {
         bool odd = false;
 #pragma unroll
         for (int i = 0; i < 2 * NT; ++i) {
@@ -96,7 +113,7 @@ __global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __res
         }
         // the two buffers take turns: a warp that writes one has passed this barrier after everyone's last read of it
         const int bad = __syncthreads_or(odd);
-        if (k0 + kSK < kb) load(k0 + kSK);
+        if (k0 + kstep < kc) load(k0 + kstep);
         if (!bad && !any) continue;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -112,6 +129,20 @@ __global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __res
         }
         __syncwarp();                                 // the next chunk's |H|^2 goes over this one's
     }
+    if (kmax) {
+#pragma unroll
+        for (int i = 0; i < 2 * NT; ++i) {
+            const int sg = s0 + warp + 4 * i;
+            bool odd = false;
+            if (sg < nseg) {
+                const float* p = IP + (long long)sg * ldip;
+#pragma unroll 8
+                for (int k = k0 + lane; k < kb; k += kstep) odd |= !(fabsf(__ldg(p + k)) <= 3.402823466e+38f);
+            }
+            if (odd) s_bad[warp + 4 * i] = 1;
+        }
+        __syncthreads();
+    }
 #pragma unroll
     for (int f = 0; f < 2; ++f)
 #pragma unroll
@@ -119,7 +150,9 @@ __global__ void __launch_bounds__(128) sigma2_partial_kernel(const float2* __res
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
                 const int row = r0 + 8 * f + fr, sg = s0 + 8 * j + 2 * fk + i;
-                if (row < n && sg < nseg) part[((long long)blockIdx.z * n + row) * nseg + sg] = acc[f][j][i];
+                if (row < n && sg < nseg)
+                    part[((long long)blockIdx.z * n + row) * nseg + sg] =
+                        kmax && s_bad[sg - s0] ? __longlong_as_double(0x7ff8000000000000ll) : acc[f][j][i];
             }
 }
 
@@ -325,6 +358,12 @@ extern "C" {
 
 int gwb_sigma2(const float* H, long long ldh, int n, const float* IP, long long ldip, int nseg, int kmin, int flen,
                double df, double* part, long long part_elems, double* sig, long long ldsig, void* stream) {
+    return gwb_sigma2_band(H, ldh, n, nullptr, IP, ldip, nseg, kmin, flen, df, part, part_elems, sig, ldsig, stream);
+}
+
+int gwb_sigma2_band(const float* H, long long ldh, int n, const int32_t* kmax, const float* IP, long long ldip, int nseg,
+                    int kmin, int flen, double df, double* part, long long part_elems, double* sig, long long ldsig,
+                    void* stream) {
     using namespace gwb;
     GWB_CHECK_ARG(H && IP && part && sig, GWB_ERR_ARG, "sigma2: null pointer");
     GWB_CHECK_ARG(n > 0 && nseg > 0 && flen > kmin && kmin >= 0 && ldsig >= nseg, GWB_ERR_SHAPE,
@@ -332,8 +371,7 @@ int gwb_sigma2(const float* H, long long ldh, int n, const float* IP, long long 
     // fewer splits where the workspace holds no more
     int nsplit = (int)std::min<long long>(sigma2_splits(n, nseg), part_elems / ((long long)n * nseg));
     GWB_CHECK_ARG(nsplit >= 1, GWB_ERR_SHAPE, "sigma2: workspace of %lld doubles is smaller than n*nseg", part_elems);
-    const int kper = (int)(cdiv(cdiv(flen - kmin, nsplit), kSK) * kSK);
-    nsplit = (int)cdiv(flen - kmin, kper);
+    nsplit = (int)std::min<long long>(nsplit, cdiv(flen - kmin, kSK));
     cudaStream_t s = (cudaStream_t)stream;
     const int nt = nseg <= 8 ? 1 : nseg <= 16 ? 2 : nseg <= 32 ? 4 : 8;
     const dim3 grid((unsigned)cdiv(n, kSR), (unsigned)cdiv(nseg, 8 * nt), nsplit);
@@ -341,7 +379,7 @@ int gwb_sigma2(const float* H, long long ldh, int n, const float* IP, long long 
                 : nt == 4 ? sigma2_partial_kernel<4> : sigma2_partial_kernel<8>;
     const size_t smem = (size_t)(2 * 8 * nt + 4 * 16) * kSB * sizeof(double);
     GWB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<grid, 128, smem, s>>>(reinterpret_cast<const float2*>(H), ldh, n, IP, ldip, nseg, kmin, flen, kper, part);
+    kern<<<grid, 128, smem, s>>>(reinterpret_cast<const float2*>(H), ldh, n, IP, ldip, nseg, kmin, flen, kmax, part);
     GWB_LAUNCH_CHECK("sigma2_partial_kernel");
     sigma2_reduce_kernel<<<(unsigned)cdiv((long long)n * nseg, 32), 512, 0, s>>>(part, nsplit, n, nseg, 4.0 * df, sig,
                                                                                 ldsig);

@@ -289,8 +289,8 @@ class MatchedFilter:
         sig = torch.empty((b.M, nseg), dtype=torch.float64, device=IP.device)
         part_elems = _lib.load().gwb_sigma2_part_elems(b.M, nseg)
         part = torch.empty(part_elems, dtype=torch.float64, device=IP.device)
-        _lib.call('gwb_sigma2', _lib.ptr(b.H), b.H.stride(0), b.M, _lib.ptr(IP), _lib.row_stride(IP), nseg, b.kmin, b.flen,
-                  float(b.df), _lib.ptr(part), part_elems, _lib.ptr(sig), sig.stride(0), _lib.stream_ptr())
+        _lib.call('gwb_sigma2_band', _lib.ptr(b.H), b.H.stride(0), b.M, _lib.ptr(b.kmax), _lib.ptr(IP),
+                  _lib.row_stride(IP), nseg, b.kmin, b.flen, float(b.df), _lib.ptr(part), part_elems, _lib.ptr(sig), sig.stride(0), _lib.stream_ptr())
         self.kernel_launches += 2
         return sig
 

@@ -231,6 +231,11 @@ GWB_API long long gwb_sigma2_part_elems(int n, int nseg);
 GWB_API int gwb_sigma2(const float* H, long long ldh, int n, const float* IP, long long ldip, int nseg, int kmin,
                        int flen, double df, double* part, long long part_elems, double* sig, long long ldsig,
                        void* stream);
+/* gwb_sigma2 for templates that are zero from bin kmax[row] on (n ints, or NULL): the same norms without reading the
+ * zeros. */
+GWB_API int gwb_sigma2_band(const float* H, long long ldh, int n, const int32_t* kmax, const float* IP, long long ldip,
+                            int nseg, int kmin, int flen, double df, double* part, long long part_elems, double* sig,
+                            long long ldsig, void* stream);
 /* Template norms as gwb_sigma2, for callers that must not allocate device memory: no counterpart in the reference.
  * Some callers cannot let a library call cudaMalloc: a host program (for example a Go or Java service over the C ABI)
  * whose own pool owns every byte of device memory, code that runs between stream-capture begin and end, where an

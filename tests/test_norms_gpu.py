@@ -34,3 +34,31 @@ def test_sigma2_non_finite_inverse_psd():
     sig, _ = fp_filter.sigma2(torch.from_numpy(H).cuda(), torch.from_numpy(IP).cuda(), 1.0, 0)
     s = sig.cpu().numpy()
     assert np.all(s[:, 0] == 360.0) and np.isnan(s[:, 1:]).all()
+
+
+def _band(H, kmax, IP, df, kmin):
+    from gwb200 import _lib
+    n, nseg = H.shape[0], IP.shape[0]
+    part = torch.empty(_lib.load().gwb_sigma2_part_elems(n, nseg), dtype=torch.float64, device='cuda')
+    sig = torch.empty((n, nseg), dtype=torch.float64, device='cuda')
+    _lib.call('gwb_sigma2_band', _lib.ptr(H), H.stride(0), n, _lib.ptr(kmax), _lib.ptr(IP), _lib.row_stride(IP), nseg, kmin,
+              H.shape[1], df, _lib.ptr(part), part.numel(), _lib.ptr(sig), nseg, _lib.stream_ptr())
+    return sig
+
+
+@pytest.mark.parametrize('n,nseg,flen,kmin', [(1, 1, 4097, 40), (65, 9, 30001, 3), (130, 33, 9000, 500), (40, 70, 5000, 0)])
+def test_sigma2_of_rows_with_ends(n, nseg, flen, kmin):
+    rng = np.random.default_rng(n + nseg)
+    H = (rng.standard_normal((n, flen)) + 1j * rng.standard_normal((n, flen))).astype(np.complex64)
+    kmax = rng.integers(kmin + 1, flen, n).astype(np.int32)
+    kmax[n // 2] = kmin                                          # a row of zeros
+    for i in range(n):
+        H[i, kmax[i]:] = 0
+    IP = rng.uniform(0.1, 2.0, (nseg, flen)).astype(np.float32)
+    Hd, kd, IPd = torch.from_numpy(H).cuda(), torch.from_numpy(kmax).cuda(), torch.from_numpy(IP).cuda()
+    ref = 2.0 * (np.abs(H[:, kmin:].astype(np.complex128)) ** 2) @ IP[:, kmin:].astype(np.float64).T
+    np.testing.assert_allclose(_band(Hd, kd, IPd, 0.5, kmin).cpu().numpy(), ref, rtol=1e-12)
+    IPd[nseg - 1, flen - 1] = float('inf')                       # past every end: 0 * inf
+    s = _band(Hd, kd, IPd, 0.5, kmin).cpu().numpy()
+    assert np.isnan(s[:, nseg - 1]).all()
+    np.testing.assert_allclose(s[:, :nseg - 1], ref[:, :nseg - 1], rtol=1e-12)
