@@ -180,9 +180,9 @@ __device__ __forceinline__ int kmax_of(double Ms, double df, int flen) {
 constexpr int kNF = 10;                  // phase functions
 constexpr int kNM = kNF + 1;             // moments: the phase functions, then f
 constexpr int kOne = 4;                  // phi = 1: the moment is the bin's z
-constexpr int kWarps = kThreads / 32;
-constexpr int kTab = 2048;               // bins whose log f and w are kept from the edge pass
-constexpr int kChunk = kTab / kThreads;  // and the weights per thread that stay in registers
+constexpr int kGT = 256;                 // threads per trigger of snr_grad_kernel
+constexpr int kWarps = kGT / 32;
+constexpr int kTab = 6016;               // bins from kmin on whose log f and w a CTA keeps for all its triggers (94 KB)
 
 // C_m and its derivatives for m = lane: pre times a^x times a polynomial in (eta, chi), with every power of pi Ms (and the
 // eccentric term's v0^(19/3)) in one exponential whose exponent is the lane's own; only logarithms of Mc, eta and f_ecc
@@ -248,68 +248,59 @@ __device__ __forceinline__ double w_to_73(double w) {
     return iu3 * iu3 * iu;
 }
 
+__device__ __forceinline__ double2 log_root(const double2* tab, int kmin, int k, double df) {
+    if (k - kmin < kTab) return tab[k - kmin];
+    const double lf = log((double)k * df);
+    return make_double2(lf, root18(lf));
+}
+
 // Equal-power edges of w_k = f^-7/3 IP_k over [kmin, k1): edge j = first k whose inclusive cumulative sum exceeds
 // (j / nb) total (the pipeline's edges, offset mode 0). Threads take contiguous ranges; float64 sums, warp and block
-// scans. A band of at most kTab bins leaves log f and w in tab for the main pass.
+// scans, and one walk per thread over its range that sets the edges inside it.
 __device__ void block_edges(const float* __restrict__ ip, double df, int kmin, int k1, int nb, int* e, double* tot_out,
-                            double* scan, double2* tab) {
+                            double* scan, const double2* tab) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int len = k1 - kmin, chunk = (len + kThreads - 1) / kThreads;
+    const int len = k1 - kmin, chunk = (len + kGT - 1) / kGT;
     const int a = min(kmin + tid * chunk, k1), b = min(a + chunk, k1);
-    const bool small = len <= kTab;
-    double wk[kChunk], s = 0.0;
-    if (small) {
-#pragma unroll
-        for (int i = 0; i < kChunk; ++i) {
-            wk[i] = 0.0;
-            if (a + i < b) {
-                const double lf = log((double)(a + i) * df), w = root18(lf);
-                tab[a + i - kmin] = make_double2(lf, w);
-                wk[i] = w_to_73(w) * (double)ip[a + i];
-                s += wk[i];
-            }
-        }
-    } else {
-        for (int k = a; k < b; ++k) s += w_to_73(root18(log((double)k * df))) * (double)ip[k];
-    }
+    auto weight = [&](int k) { return w_to_73(log_root(tab, kmin, k, df).y) * (double)ip[k]; };
+    double s = 0.0;
+#pragma unroll 4
+    for (int k = a; k < b; ++k) s += weight(k);
     double inc = s;                                  // inclusive scan of the threads' sums
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
         const double v = __shfl_up_sync(0xffffffffu, inc, off);
         if (lane >= off) inc += v;
     }
-    if (lane == 31) scan[kThreads + 1 + warp] = inc;
-    for (int j = tid; j <= nb; j += kThreads) e[j] = j == 0 ? kmin : k1;
+    if (lane == 31) scan[kGT + 1 + warp] = inc;
+    for (int j = tid; j <= nb; j += kGT) e[j] = j == 0 ? kmin : k1;
     __syncthreads();
     double base = 0.0;
-    for (int w = 0; w < warp; ++w) base += scan[kThreads + 1 + w];
+#pragma unroll
+    for (int w = 0; w < kWarps - 1; ++w) base += w < warp ? scan[kGT + 1 + w] : 0.0;
     scan[tid + 1] = base + inc;
     if (tid == 0) scan[0] = 0.0;
     __syncthreads();
-    const double tot = scan[kThreads], ex = scan[tid], hi = scan[tid + 1];
-    for (int j = 1; j < nb; ++j) {
-        const double target = (double)j / (double)nb * tot;
-        if (ex <= target && target < hi) {
+    const double tot = scan[kGT], ex = scan[tid], hi = scan[tid + 1];
+    if (tot > 0.0) {                                 // (not for a NaN)
+        // the edges j with ex <= (j / nb) tot < hi
+        auto target = [&](int j) { return (double)j / (double)nb * tot; };
+        int j = max(1, (int)(ex / tot * (double)nb) - 1);
+        while (j < nb && target(j) < ex) ++j;
+        double t = j < nb ? target(j) : hi;
+        if (t < hi) {
             double c = ex;
-            int at = b - 1;                          // the last bin's sum is hi (to rounding)
-            if (small) {
-#pragma unroll
-                for (int i = kChunk - 1; i >= 0; --i) {
-                    double ci = ex;
-#pragma unroll
-                    for (int x = 0; x <= i; ++x) ci += wk[x];
-                    if (a + i < b && ci > target) at = a + i;
-                }
-            } else {
-                for (int k = a; k < b; ++k) {
-                    c += w_to_73(root18(log((double)k * df))) * (double)ip[k];
-                    if (c > target) {
-                        at = k;
-                        break;
-                    }
+            for (int k = a; k < b; ++k) {
+                c += weight(k);
+                while (t < hi && c > t) {
+                    e[j] = k;
+                    t = ++j < nb ? target(j) : hi;
                 }
             }
-            e[j] = at;
+            while (t < hi) {                         // the range's last sum is hi, to rounding
+                e[j] = b - 1;
+                t = ++j < nb ? target(j) : hi;
+            }
         }
     }
     if (tid == 0) *tot_out = tot;
@@ -319,196 +310,209 @@ __device__ void block_edges(const float* __restrict__ ip, double df, int kmin, i
 // out row layout (doubles): snr, newsnr, chisq, sigma2, z_re, z_im, kmax, dsnr[7], dnewsnr[7], dchisq[7]
 constexpr int kOut = 7 + 3 * kNP;
 
-// One CTA per trigger. The band is cut into one contiguous run per warp; a lane's bins are 32 apart (coalesced D and
-// IP), and at every chi-squared edge the warp adds its 22 sums over the lanes (a halving exchange: 31 shuffles of a
-// double, against 110 for 22 trees) and stores them with the edge bin they belong to. Bound: the float64 pipe (log and
-// exp of the edge pass, then about 50 operations per bin). The former kernel took a barrier and a block reduction per
-// chi-squared bin, in which 256 threads share the 20 to 200 bins of 16 s of data, and a dual-number phase with three
-// exp and two pow per frequency bin: 803 -> 194 us for 2,048 triggers of 16 s, float32.
+// CTAs of eight warps, two per SM, stay for all their triggers (blockIdx.x, + gridDim.x, ...), so that log f and
+// f^(-1/18) of the first kTab bins are computed once per CTA, as far as the longest band of its triggers. Per trigger, the
+// band is cut into one contiguous run per warp; a lane's bins are 32 apart (coalesced D and IP), and at every chi-squared
+// edge the warp adds its 22 sums over the lanes (a halving exchange: 31 shuffles of a double, against 110 for 22 trees)
+// and stores them with the edge bin they belong to. Bound: the chain of a trigger (coefficients, edges, runs, final sums)
+// with two of them per SM, and the float64 pipe. The former kernel took a barrier and a block reduction per chi-squared
+// bin, in which 256 threads share the 20 to 200 bins of 16 s of data, and a dual-number phase with three exp and two pow
+// per frequency bin: 803 us for 2,048 triggers of 16 s, float32, now 159. (A CTA per trigger without the table 194, four
+// warps per trigger and four CTAs per SM 192, a warp per trigger 291: it waits for the longest band.)
 template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) snr_grad_kernel(const double* __restrict__ params, int n,
+__global__ void __launch_bounds__(kGT, 2) snr_grad_kernel(const double* __restrict__ params, int n,
                                                              const float2* __restrict__ D, long long ldd,
                                                              const float* __restrict__ IP, long long ldip, int flen,
                                                              double df, int kmin, double f_ecc, int nb,
                                                              double* __restrict__ out, long long ldout) {
-    const int i = blockIdx.x;
-    if (i >= n) return;
     constexpr int kNS = 2 * kNM;
     constexpr int kSeg = kMaxBins + kWarps;            // (warp, bin) runs: warp + bin never repeats along the band
-    __shared__ double scan[kThreads + 1 + kWarps];
+    __shared__ double scan[kGT + 1 + kWarps];
     __shared__ int e[kMaxBins + 1];
     __shared__ double tot;
     __shared__ double C[kNF][1 + kNI];
     __shared__ int owner[kSeg];
     __shared__ double seg[kSeg][kNS];
-    __shared__ double2 tab[kTab];
+    extern __shared__ double2 tab[];                   // kTab
+    __shared__ int s_top;                              // the longest band of this CTA's triggers
     __shared__ double acc[kMaxBins][2 + 2 * kNP];      // per bin: z_j (re, im), dz_j (re, im) x 7
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const double* th = params + (long long)i * kNP;
-    // the end bin from the same operations as phase_coef's value of Ms
-    const double q1 = 1.0 + th[1], eta = th[1] / (q1 * q1);
-    const int k1 = kmax_of(kMsun * (th[0] * pow(eta, -0.6)), df, flen);
-    if (k1 <= kmin + kThreads) {           // no band above kmin (f_ISCO below the low cut): nothing to filter
-        if (tid < kOut) out[(long long)i * ldout + tid] = 0.0;
-        return;
-    }
-    const float* ip = IP + (long long)i * ldip;
-    const float2* d = D + (long long)i * ldd;
-    if (tid < kSeg) owner[tid] = -1;
-    if (warp == kWarps - 1) {
-        const Dual c = phase_function_coef(th, f_ecc, min(lane, kNF - 1));
-        if (lane < kNF) {
-            C[lane][0] = c.v;
-#pragma unroll
-            for (int p = 0; p < kNI; ++p) C[lane][1 + p] = c.d[p];
-        }
-    }
-    block_edges(ip, df, kmin, k1, nb, e, &tot, scan, tab);   // ends with a barrier
-    {
-        double cv[kNF];
-#pragma unroll
-        for (int m = 0; m < kNF; ++m) cv[m] = C[m][0];
-        cv[kOne] -= 0.25 * kPi + th[6];
-        const double wtc = 2.0 * kPi * th[5];
-        const bool have = k1 - kmin <= kTab;
-        const int run = ((k1 - kmin + kThreads - 1) / kThreads) * 32;    // bins per warp, whole rounds of 32 lanes
-        const int A = min(kmin + warp * run, k1), B = min(A + run, k1);
-        for (int j = 0; j < nb; ++j) {
-            const int lo = max(e[j], A), hi = min(e[j + 1], B);
-            if (lo >= hi) continue;                                      // warp-uniform
-            double s[kNS];
-#pragma unroll
-            for (int x = 0; x < kNS; ++x) s[x] = 0.0;
-            for (int k = lo + lane; k < hi; k += 32) {
-                const double f = (double)k * df;
-                double lf, w;
-                if (have) {
-                    const double2 t = tab[k - kmin];
-                    lf = t.x;
-                    w = t.y;
-                } else {
-                    lf = log(f);
-                    w = root18(lf);
-                }
-                const double w2 = w * w, w3 = w2 * w, iu = w3 * w3, iu2 = iu * iu, iu3 = iu2 * iu, iu5 = iu3 * iu2;
-                const double u = f * iu2;
-                const double phi[kNM] = {iu5, iu3, iu2, iu, 1.0, lf, u, u * lf, f * iu, iu5 * iu5 * iu * w2, f};
-                double ph = cv[kOne], ph2 = wtc * f;                     // two chains
-#pragma unroll
-                for (int m = 0; m < kNF; ++m) {
-                    if (m < kOne) ph = fma(cv[m], phi[m], ph);
-                    if (m > kOne) ph2 = fma(cv[m], phi[m], ph2);
-                }
-                ph += ph2;
-                ph -= 2.0 * kPi * rint(ph * (0.5 / kPi));
-                T sn, cs;
-                if constexpr (sizeof(T) == 8) {
-                    sincos(ph, &sn, &cs);
-                } else {
-                    sincosf((float)ph, &sn, &cs);
-                }
-                const T amp = (T)(iu3 * w3);                             // f^(-7/6)
-                const float2 dk = d[k];
-                // q = conj(h) D = amp e^{+i ph} D
-                const T hr = amp * cs, hi2 = amp * sn;
-                const double qr = (double)(hr * (T)dk.x - hi2 * (T)dk.y), qi = (double)(hr * (T)dk.y + hi2 * (T)dk.x);
-#pragma unroll
-                for (int m = 0; m < kNM; ++m) {
-                    s[2 * m] = fma(qr, phi[m], s[2 * m]);
-                    s[2 * m + 1] = fma(qi, phi[m], s[2 * m + 1]);
-                }
-            }
-            // lane x ends with the warp's sum of s[x]: each exchange halves the values a lane holds
-            double v[16];
-            {
-                const bool up = lane & 16;
-#pragma unroll
-                for (int x = 0; x < 16; ++x) {
-                    const double a = s[x], b = x + 16 < kNS ? s[x + 16 < kNS ? x + 16 : 0] : 0.0;
-                    v[x] = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
-                }
-            }
-#pragma unroll
-            for (int h = 8; h >= 1; h >>= 1) {
-                const bool up = lane & h;
-#pragma unroll
-                for (int x = 0; x < h; ++x)
-                    v[x] = (up ? v[x + h] : v[x]) + __shfl_xor_sync(0xffffffffu, up ? v[x] : v[x + h], h);
-            }
-            if (lane < kNS) seg[warp + j][lane] = v[0];
-            if (lane == 0) owner[warp + j] = j;
-        }
+    if (tid == 0) s_top = 0;
+    __syncthreads();
+    for (int i = blockIdx.x + tid * (int)gridDim.x; i < n; i += kGT * (int)gridDim.x) {
+        const double* th = params + (long long)i * kNP;
+        const double q1 = 1.0 + th[1], eta = th[1] / (q1 * q1);
+        atomicMax(&s_top, kmax_of(kMsun * (th[0] * pow(eta, -0.6)), df, flen));
     }
     __syncthreads();
-    // per (bin, value): the bin's runs in band order, then the contraction with dC / dtheta
-    const double c4 = 4.0 * df;
-    for (int x = tid; x < nb * (1 + kNP); x += kThreads) {
-        const int j = x / (1 + kNP), p = x % (1 + kNP) - 1;
-        double re = 0.0, im = 0.0;
-        for (int w = 0; w < kWarps; ++w) {
-            if (owner[j + w] != j) continue;
-            const double* M = seg[j + w];
-            if (p < 0) {
-                re += M[2 * kOne];
-                im += M[2 * kOne + 1];
-            } else if (p < kNI) {
-#pragma unroll
-                for (int m = 0; m < kNF; ++m) {
-                    re = fma(-C[m][1 + p], M[2 * m + 1], re);
-                    im = fma(C[m][1 + p], M[2 * m], im);
-                }
-            } else {
-                const int m = p == 5 ? kNF : kOne;
-                const double g = p == 5 ? 2.0 * kPi : -1.0;
-                re -= g * M[2 * m + 1];
-                im += g * M[2 * m];
-            }
-        }
-        acc[j][2 * (p + 1)] = c4 * re;
-        acc[j][2 * (p + 1) + 1] = c4 * im;
+    for (int k = tid; k < min(kTab, s_top - kmin); k += kGT) {
+        const double lf = log((double)(kmin + k) * df);
+        tab[k] = make_double2(lf, root18(lf));
     }
     __syncthreads();
-    if (tid < kNP) {                                   // thread p: the outputs of parameter p (thread 0: the values too)
-        const int p = tid;
-        const double sig2 = c4 * tot;
-        double zr = 0.0, zi = 0.0, pw = 0.0, dzr = 0.0, dzi = 0.0, dpw = 0.0;
-        for (int j = 0; j < nb; ++j) {
-            const double ar = acc[j][0], ai = acc[j][1], br = acc[j][2 + 2 * p], bi = acc[j][3 + 2 * p];
-            zr += ar;
-            zi += ai;
-            pw += ar * ar + ai * ai;
-            dzr += br;
-            dzi += bi;
-            dpw += 2.0 * (ar * br + ai * bi);
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const double* th = params + (long long)i * kNP;
+        // the end bin from the same operations as phase_coef's value of Ms
+        const double q1 = 1.0 + th[1], eta = th[1] / (q1 * q1);
+        const int k1 = kmax_of(kMsun * (th[0] * pow(eta, -0.6)), df, flen);
+        if (k1 <= kmin + 256) {           // no band above kmin (f_ISCO below the low cut): nothing to filter
+            if (tid < kOut) out[(long long)i * ldout + tid] = 0.0;
+            continue;
         }
-        const double az = sqrt(zr * zr + zi * zi), sg = sqrt(sig2);
-        const double snr = az / sg;
-        const double chisq = ((double)nb * pw - az * az) / sig2;
-        const int dof = 2 * nb - 2;
-        const double rc = chisq / (double)dof;
-        double ns = snr, g = 1.0, gp = 0.0;
-        if (rc > 1.0) {
-            const double base = (1.0 + rc * rc * rc) / 2.0;
-            g = pow(base, -1.0 / 6.0);
-            gp = -1.0 / 6.0 * pow(base, -7.0 / 6.0) * 1.5 * rc * rc;   // d g / d rc
-            ns = snr * g;
+        const float* ip = IP + (long long)i * ldip;
+        const float2* d = D + (long long)i * ldd;
+        if (tid < kSeg) owner[tid] = -1;
+        if (warp == kWarps - 1) {
+            const Dual c = phase_function_coef(th, f_ecc, min(lane, kNF - 1));
+            if (lane < kNF) {
+                C[lane][0] = c.v;
+#pragma unroll
+                for (int p = 0; p < kNI; ++p) C[lane][1 + p] = c.d[p];
+            }
         }
-        double* o = out + (long long)i * ldout;
-        if (p == 0) {
-            o[0] = snr;
-            o[1] = ns;
-            o[2] = chisq;
-            o[3] = sig2;
-            o[4] = zr;
-            o[5] = zi;
-            o[6] = (double)k1;
+        block_edges(ip, df, kmin, k1, nb, e, &tot, scan, tab);   // ends with a barrier
+        {
+            double cv[kNF];
+#pragma unroll
+            for (int m = 0; m < kNF; ++m) cv[m] = C[m][0];
+            cv[kOne] -= 0.25 * kPi + th[6];
+            const double wtc = 2.0 * kPi * th[5];
+            const int run = ((k1 - kmin + kGT - 1) / kGT) * 32;    // bins per warp, whole rounds of 32 lanes
+            const int A = min(kmin + warp * run, k1), B = min(A + run, k1);
+            for (int j = 0; j < nb; ++j) {
+                const int lo = max(e[j], A), hi = min(e[j + 1], B);
+                if (lo >= hi) continue;                                      // warp-uniform
+                double s[kNS];
+#pragma unroll
+                for (int x = 0; x < kNS; ++x) s[x] = 0.0;
+                float2 dn = lo + lane < hi ? d[lo + lane] : make_float2(0.f, 0.f);
+                for (int k = lo + lane; k < hi; k += 32) {
+                    const float2 dk = dn;
+                    if (k + 32 < hi) dn = d[k + 32];
+                    const double f = (double)k * df;
+                    const double2 t = log_root(tab, kmin, k, df);
+                    const double lf = t.x, w = t.y;
+                    const double w2 = w * w, w3 = w2 * w, iu = w3 * w3, iu2 = iu * iu, iu3 = iu2 * iu, iu5 = iu3 * iu2;
+                    const double u = f * iu2;
+                    const double phi[kNM] = {iu5, iu3, iu2, iu, 1.0, lf, u, u * lf, f * iu, iu5 * iu5 * iu * w2, f};
+                    double ph = cv[kOne], ph2 = wtc * f;                     // two chains
+#pragma unroll
+                    for (int m = 0; m < kNF; ++m) {
+                        if (m < kOne) ph = fma(cv[m], phi[m], ph);
+                        if (m > kOne) ph2 = fma(cv[m], phi[m], ph2);
+                    }
+                    ph += ph2;
+                    ph -= 2.0 * kPi * rint(ph * (0.5 / kPi));
+                    T sn, cs;
+                    if constexpr (sizeof(T) == 8) {
+                        sincos(ph, &sn, &cs);
+                    } else {
+                        sincosf((float)ph, &sn, &cs);
+                    }
+                    const T amp = (T)(iu3 * w3);                             // f^(-7/6)
+                    // q = conj(h) D = amp e^{+i ph} D
+                    const T hr = amp * cs, hi2 = amp * sn;
+                    const double qr = (double)(hr * (T)dk.x - hi2 * (T)dk.y);
+                    const double qi = (double)(hr * (T)dk.y + hi2 * (T)dk.x);
+#pragma unroll
+                    for (int m = 0; m < kNM; ++m) {
+                        s[2 * m] = fma(qr, phi[m], s[2 * m]);
+                        s[2 * m + 1] = fma(qi, phi[m], s[2 * m + 1]);
+                    }
+                }
+                // lane x ends with the warp's sum of s[x]: each exchange halves the values a lane holds
+                double v[16];
+                {
+                    const bool up = lane & 16;
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) {
+                        const double a = s[x], b = x + 16 < kNS ? s[x + 16 < kNS ? x + 16 : 0] : 0.0;
+                        v[x] = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+                    }
+                }
+#pragma unroll
+                for (int h = 8; h >= 1; h >>= 1) {
+                    const bool up = lane & h;
+#pragma unroll
+                    for (int x = 0; x < h; ++x)
+                        v[x] = (up ? v[x + h] : v[x]) + __shfl_xor_sync(0xffffffffu, up ? v[x] : v[x + h], h);
+                }
+                if (lane < kNS) seg[warp + j][lane] = v[0];
+                if (lane == 0) owner[warp + j] = j;
+            }
         }
-        const double dabs = az > 0.0 ? (zr * dzr + zi * dzi) / az : 0.0;
-        const double dsnr = dabs / sg;
-        const double dchi = ((double)nb * dpw - 2.0 * az * dabs) / sig2;
-        o[7 + p] = dsnr;
-        o[7 + kNP + p] = dsnr * g + snr * gp * dchi / (double)dof;
-        o[7 + 2 * kNP + p] = dchi;
+        __syncthreads();
+        // per (bin, value): the bin's runs in band order, then the contraction with dC / dtheta
+        const double c4 = 4.0 * df;
+        for (int x = tid; x < nb * (1 + kNP); x += kGT) {
+            const int j = x / (1 + kNP), p = x % (1 + kNP) - 1;
+            double re = 0.0, im = 0.0;
+            for (int w = 0; w < kWarps; ++w) {
+                if (owner[j + w] != j) continue;
+                const double* M = seg[j + w];
+                if (p < 0) {
+                    re += M[2 * kOne];
+                    im += M[2 * kOne + 1];
+                } else if (p < kNI) {
+#pragma unroll
+                    for (int m = 0; m < kNF; ++m) {
+                        re = fma(-C[m][1 + p], M[2 * m + 1], re);
+                        im = fma(C[m][1 + p], M[2 * m], im);
+                    }
+                } else {
+                    const int m = p == 5 ? kNF : kOne;
+                    const double g = p == 5 ? 2.0 * kPi : -1.0;
+                    re -= g * M[2 * m + 1];
+                    im += g * M[2 * m];
+                }
+            }
+            acc[j][2 * (p + 1)] = c4 * re;
+            acc[j][2 * (p + 1) + 1] = c4 * im;
+        }
+        __syncthreads();
+        if (tid < kNP) {                               // thread p: the outputs of parameter p (thread 0: the values too)
+            const int p = tid;
+            const double sig2 = c4 * tot;
+            double zr = 0.0, zi = 0.0, pw = 0.0, dzr = 0.0, dzi = 0.0, dpw = 0.0;
+            for (int j = 0; j < nb; ++j) {
+                const double ar = acc[j][0], ai = acc[j][1], br = acc[j][2 + 2 * p], bi = acc[j][3 + 2 * p];
+                zr += ar;
+                zi += ai;
+                pw += ar * ar + ai * ai;
+                dzr += br;
+                dzi += bi;
+                dpw += 2.0 * (ar * br + ai * bi);
+            }
+            const double az = sqrt(zr * zr + zi * zi), sg = sqrt(sig2);
+            const double snr = az / sg;
+            const double chisq = ((double)nb * pw - az * az) / sig2;
+            const int dof = 2 * nb - 2;
+            const double rc = chisq / (double)dof;
+            double ns = snr, g = 1.0, gp = 0.0;
+            if (rc > 1.0) {
+                const double base = (1.0 + rc * rc * rc) / 2.0;
+                g = pow(base, -1.0 / 6.0);
+                gp = -1.0 / 6.0 * pow(base, -7.0 / 6.0) * 1.5 * rc * rc;   // d g / d rc
+                ns = snr * g;
+            }
+            double* o = out + (long long)i * ldout;
+            if (p == 0) {
+                o[0] = snr;
+                o[1] = ns;
+                o[2] = chisq;
+                o[3] = sig2;
+                o[4] = zr;
+                o[5] = zi;
+                o[6] = (double)k1;
+            }
+            const double dabs = az > 0.0 ? (zr * dzr + zi * dzi) / az : 0.0;
+            const double dsnr = dabs / sg;
+            const double dchi = ((double)nb * dpw - 2.0 * az * dabs) / sig2;
+            o[7 + p] = dsnr;
+            o[7 + kNP + p] = dsnr * g + snr * gp * dchi / (double)dof;
+            o[7 + 2 * kNP + p] = dchi;
+        }
+        __syncthreads();                               // the next trigger's sums go over this one's
     }
 }
 
@@ -662,11 +666,15 @@ int gwb_snr_grad(const double* params, int n, const float* D, long long ldd, con
                   GWB_ERR_SHAPE, "snr_grad: n=%d flen=%d kmin=%d nbins=%d ldout=%lld", n, flen, kmin, nbins, ldout);
     cudaStream_t s = (cudaStream_t)stream;
     const float2* d = reinterpret_cast<const float2*>(D);
+    const int grid = std::min(n, 2 * num_sms());           // two CTAs per SM
+    const size_t smem = kTab * sizeof(double2);
+    GWB_CUDA(cudaFuncSetAttribute(fp64 ? snr_grad_kernel<double> : snr_grad_kernel<float>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (fp64)
-        snr_grad_kernel<double><<<n, kThreads, 0, s>>>(params, n, d, ldd, IP, ldip, flen, df, kmin, f_ecc, nbins,
+        snr_grad_kernel<double><<<grid, kGT, smem, s>>>(params, n, d, ldd, IP, ldip, flen, df, kmin, f_ecc, nbins,
                                                         out, ldout);
     else
-        snr_grad_kernel<float><<<n, kThreads, 0, s>>>(params, n, d, ldd, IP, ldip, flen, df, kmin, f_ecc, nbins, out,
+        snr_grad_kernel<float><<<grid, kGT, smem, s>>>(params, n, d, ldd, IP, ldip, flen, df, kmin, f_ecc, nbins, out,
                                                        ldout);
     GWB_LAUNCH_CHECK("snr_grad_kernel");
     return GWB_OK;
