@@ -260,6 +260,38 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)
           "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
         : "r"(taddr));
 }
+// maximum of |z|^2 over 32 samples and its first index: four chains of eight, merged in order (strictly larger wins, so
+// the first index stays); samples at or past `valid` count as -1
+template <bool FULL>
+__device__ __forceinline__ void best_of_32(const uint32_t (&re)[32], const uint32_t (&im)[32], int valid, int base,
+                                           float& best, int& bi) {
+    float b[4];
+    int x[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        b[c] = -1.f;
+        x[c] = 0;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float r = __uint_as_float(re[8 * c + j]), i = __uint_as_float(im[8 * c + j]);
+            float p = fmaf(r, r, i * i);
+            if (!FULL && 8 * c + j >= valid) p = -1.f;
+            if (p > b[c]) {
+                b[c] = p;
+                x[c] = base + 8 * c + j;
+            }
+        }
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (b[c] > best) {
+            best = b[c];
+            bi = x[c];
+        }
+}
+
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }

@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
-            mbar_init(&tempty[b], kEpiWarps);
+            mbar_init(&tempty[b], kEpiWarps / 2);
         }
         mbar_init(barA, 1);
         mbar_init(done, 1);
@@ -368,115 +368,124 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
         }
         __syncwarp();
     } else {
-        const int ew = warp - 2, q = warp & 3, hh = ew >> 2;
+        // two groups of four warps: group g takes the items of accumulator buffer g (with two M blocks, always M block g),
+        // so a group has two items' time for one, and with one M block the two meet once per output window, not per tile
+        const int q = warp & 3, g = (warp - 2) >> 2;
         const int rl = 32 * q + lane;
-        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-        float wb0 = -1.f, wb1 = -1.f;
-        int wi0 = 0, wi1 = 0;
-        for (int i = 0; i < ntl; ++i) {
-            const int t = t_begin + i;
-            const long long col0 = (long long)t * kTile;
-            const bool full_tile = col0 + kTile <= args.Tn;
-#pragma unroll
-            for (int mb = 0; mb < 2; ++mb) {
-                if (mb >= MBe) break;
-                const int j = i * MBe + mb, b = j & 1;
-                const uint32_t u = (uint32_t)(j >> 1);
-                float best = -1.f;
-                int bi = 0;
-                if (*abort_flag || !mbar_wait_bounded(&tfull[b], u & 1)) {
-                    record_error(args.err, GWB_ERR_TIMEOUT, 205, blockIdx.x, i);
-                    *abort_flag = 1;
-                } else {
-                    tc_fence_after();
-#pragma unroll
-                    for (int c = 0; c < 64; c += 32) {
-                        uint32_t re[32], im[32];
-                        tmem_ld_32x32b_x32(lane_base + (uint32_t)(b * 256 + hh * 64 + c), re);
-                        tmem_ld_32x32b_x32(lane_base + (uint32_t)(b * 256 + 128 + hh * 64 + c), im);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int jj = 0; jj < 32; ++jj) asm volatile("" : "+r"(re[jj]), "+r"(im[jj]));
-                        const int cb = hh * 64 + c;
-                        // best of this 32-column chunk first (index as an immediate), then merged: 2 FMA-pipe and 3
-                        // ALU instructions per element
-                        float lb = -1.f;
-                        int lj = 0;
-                        if (full_tile) {
-#pragma unroll
-                            for (int jj = 0; jj < 32; ++jj) {
-                                const float xr = __uint_as_float(re[jj]), xm = __uint_as_float(im[jj]);
-                                const float p = fmaf(xr, xr, xm * xm);
-                                if (p > lb) {
-                                    lb = p;
-                                    lj = jj;
-                                }
-                            }
-                        } else {
-                            const int valid = (int)min((long long)32, max(0ll, args.Tn - (col0 + cb)));
-#pragma unroll
-                            for (int jj = 0; jj < 32; ++jj) {
-                                const float xr = __uint_as_float(re[jj]), xm = __uint_as_float(im[jj]);
-                                const float p = jj < valid ? fmaf(xr, xr, xm * xm) : -1.f;
-                                if (p > lb) {
-                                    lb = p;
-                                    lj = jj;
-                                }
-                            }
-                        }
-                        if (lb > best) {
-                            best = lb;
-                            bi = cb + lj;
-                        }
-                    }
-                }
+        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(g * 256);
+        const int G = args.group;
+        // maximum of item j (tile t): waits for the accumulators, frees them once they are in registers; the next 32
+        // samples are in flight while these are compared
+        auto item = [&](int j, int t, float& best, int& bi) {
+            best = -1.f;
+            bi = 0;
+            if (*abort_flag || !mbar_wait_bounded(&tfull[g], (uint32_t)((j >> 1) & 1))) {
+                record_error(args.err, GWB_ERR_TIMEOUT, 205, blockIdx.x, j);
+                *abort_flag = 1;
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&tempty[b]);
-                if (hh == 1) {
-                    xv[(j & 1) * 128 + rl] = best;
-                    xi[(j & 1) * 128 + rl] = bi;
+                if (lane == 0) mbar_arrive(&tempty[g]);
+                return;
+            }
+            tc_fence_after();
+            const long long left = args.Tn - (long long)t * kTile;     // samples of the tile inside the row
+            uint32_t re[2][32], im[2][32];
+            tmem_ld_32x32b_x32(lane_base, re[0]);
+            tmem_ld_32x32b_x32(lane_base + 128, im[0]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                tmem_ld_wait();
+                // tie every value to the wait so no use is scheduled above it
+#pragma unroll
+                for (int jj = 0; jj < 32; ++jj) asm volatile("" : "+r"(re[c & 1][jj]), "+r"(im[c & 1][jj]));
+                if (c < 3) {
+                    tmem_ld_32x32b_x32(lane_base + 32 * (c + 1), re[(c + 1) & 1]);
+                    tmem_ld_32x32b_x32(lane_base + 128 + 32 * (c + 1), im[(c + 1) & 1]);
+                } else {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&tempty[g]);
                 }
-                named_bar_sync(1, 32 * kEpiWarps);
-                if (hh == 0) {
-                    const float ob = xv[(j & 1) * 128 + rl];
-                    const int oi = xi[(j & 1) * 128 + rl];
-                    if (ob > best) {
-                        best = ob;
-                        bi = oi;
-                    }
-                    const int gi = (int)(col0 + bi);
-                    const bool first = (t % args.group) == 0 || t == t_begin;
-                    const bool last = ((t + 1) % args.group) == 0 || t == args.ntiles - 1 || t == t_end - 1;
-                    float& wb = (mb == 0) ? wb0 : wb1;
-                    int& wi = (mb == 0) ? wi0 : wi1;
-                    if (first || best > wb) {
+                if (left >= kTile)
+                    best_of_32<true>(re[c & 1], im[c & 1], 32, 32 * c, best, bi);
+                else
+                    best_of_32<false>(re[c & 1], im[c & 1], (int)min(32ll, max(0ll, left - 32 * c)), 32 * c, best, bi);
+            }
+            bi += t * kTile;
+        };
+        // the maximum of the part of window o that this CTA's range holds, of M block mb
+        auto put = [&](int o, int mb, float wb, int wi) {
+            const int row = m0 + mb * 128 + rl;
+            if (row >= args.M) return;
+            const int w0 = o * G;
+            const int w1 = (int)min((long long)w0 + G, (long long)args.ntiles);
+            if (args.pv && (t_begin > w0 || t_end < w1)) {
+                const long long pidx = ((long long)row * gridDim.x + blockIdx.x) * 2 + (t_begin > w0 ? 0 : 1);
+                args.pv[pidx] = wb;
+                args.pi[pidx] = wi;
+            } else {
+                float vo = wb;
+                if (args.rowscale) {
+                    const float rs = args.rowscale[row];
+                    vo = wb * rs * rs;
+                }
+                args.V[(long long)row * args.ldv + o] = vo;
+                args.I[(long long)row * args.ldv + o] = wi;
+            }
+        };
+        float wb = -2.f;                                   // below any tile's maximum (at least -1)
+        int wi = 0;
+        if (MBe == 2) {
+            for (int i = 0; i < ntl; ++i) {
+                const int t = t_begin + i;
+                float best;
+                int bi;
+                item(2 * i + g, t, best, bi);
+                if (best > wb) {
+                    wb = best;
+                    wi = bi;
+                }
+                if ((t + 1) % G == 0 || t + 1 == t_end) {
+                    put(t / G, g, wb, wi);
+                    wb = -2.f;
+                }
+            }
+        } else {
+            int par = 0;
+            for (int t = t_begin; t < t_end;) {
+                const int o = t / G, ts = t, te = (int)min((long long)(o + 1) * G, (long long)t_end);
+                wb = -2.f;
+                wi = 0;
+                for (; t < te; ++t) {
+                    const int i = t - t_begin;
+                    if ((i & 1) != g) continue;
+                    float best;
+                    int bi;
+                    item(i, t, best, bi);
+                    if (best > wb) {
                         wb = best;
-                        wi = gi;
-                    }
-                    if (last) {
-                        const int row = m0 + mb * 128 + rl;
-                        if (row < args.M) {
-                            const long long o = t / args.group;
-                            const int w0 = (int)(o * args.group);
-                            const int w1 = (int)min((long long)w0 + args.group, (long long)args.ntiles);
-                            if (args.pv && (t_begin > w0 || t_end < w1)) {
-                                const long long pidx = ((long long)row * gridDim.x + blockIdx.x) * 2 +
-                                                       (t_begin > w0 ? 0 : 1);
-                                args.pv[pidx] = wb;
-                                args.pi[pidx] = wi;
-                            } else {
-                                float vo = wb;
-                                if (args.rowscale) {
-                                    const float rs = args.rowscale[row];
-                                    vo = wb * rs * rs;
-                                }
-                                args.V[(long long)row * args.ldv + o] = vo;
-                                args.I[(long long)row * args.ldv + o] = wi;
-                            }
-                        }
+                        wi = bi;
                     }
                 }
+                if (te - ts == 1) {                        // one tile: its group has the maximum
+                    if (((ts - t_begin) & 1) == g) put(o, 0, wb, wi);
+                    continue;
+                }
+                if (g == 1) {
+                    xv[par * 128 + rl] = wb;
+                    xi[par * 128 + rl] = wi;
+                }
+                named_bar_sync(1, 32 * kEpiWarps);         // the slots take turns: written again two outputs on
+                if (g == 0) {
+                    const float ob = xv[par * 128 + rl];
+                    const int oi = xi[par * 128 + rl];
+                    if (ob > wb || (ob == wb && oi < wi)) {
+                        wb = ob;
+                        wi = oi;
+                    }
+                    put(o, 0, wb, wi);
+                }
+                par ^= 1;
             }
         }
     }
@@ -567,7 +576,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
-            mbar_init(&tempty[b], 2 * kEpiWarps);
+            mbar_init(&tempty[b], kEpiWarps);              // four warps of each CTA
         }
         mbar_init(barA, 1);
         mbar_init(done, 1);
@@ -792,89 +801,103 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         __syncwarp();
     } else if (ntl > 0) {
-        const int q = warp & 3, hh = (warp - 2) >> 2;
+        // two groups of four warps take the two accumulator buffers in turn, as in the one-CTA kernel
+        const int q = warp & 3, g = (warp - 2) >> 2;
         const int rl = 32 * q + lane;
-        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-        const uint32_t tempty_l0 = mapa_shared(smem_u32(&tempty[0]), 0);
-        const uint32_t tempty_l1 = mapa_shared(smem_u32(&tempty[1]), 0);
-        float wb = -1.f;
-        int wi = 0;
-        for (int i = 0; i < ntl; ++i) {
-            const int t = t_begin + i;
-            const long long col0 = (long long)t * kTile;
-            const bool full_tile = col0 + kTile <= args.Tn;
-            const int b = i & 1;
-            const uint32_t u = (uint32_t)(i >> 1);
-            float best = -1.f;
-            int bi = 0;
-            if (*abort_flag || !mbar_wait_bounded(&tfull[b], u & 1)) {
-                record_error(args.err, GWB_ERR_TIMEOUT, 215, tr, i);
+        const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(g * 256);
+        const uint32_t tempty_l = mapa_shared(smem_u32(&tempty[g]), 0);
+        const int G = args.group;
+        // maximum of item j (tile t): waits for the accumulators, frees them once they are in registers; the next 32
+        // samples are in flight while these are compared
+        auto item = [&](int j, int t, float& best, int& bi) {
+            best = -1.f;
+            bi = 0;
+            if (*abort_flag || !mbar_wait_bounded(&tfull[g], (uint32_t)((j >> 1) & 1))) {
+                record_error(args.err, GWB_ERR_TIMEOUT, 215, tr, j);
                 abort_pair();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_cluster(tempty_l);
+                return;
+            }
+            tc_fence_after();
+            const long long left = args.Tn - (long long)t * kTile;     // samples of the tile inside the row
+            uint32_t re[2][32], im[2][32];
+            tmem_ld_32x32b_x32(lane_base, re[0]);
+            tmem_ld_32x32b_x32(lane_base + 128, im[0]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                tmem_ld_wait();
+                // tie every value to the wait so no use is scheduled above it
+#pragma unroll
+                for (int jj = 0; jj < 32; ++jj) asm volatile("" : "+r"(re[c & 1][jj]), "+r"(im[c & 1][jj]));
+                if (c < 3) {
+                    tmem_ld_32x32b_x32(lane_base + 32 * (c + 1), re[(c + 1) & 1]);
+                    tmem_ld_32x32b_x32(lane_base + 128 + 32 * (c + 1), im[(c + 1) & 1]);
+                } else {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(tempty_l);
+                }
+                if (left >= kTile)
+                    best_of_32<true>(re[c & 1], im[c & 1], 32, 32 * c, best, bi);
+                else
+                    best_of_32<false>(re[c & 1], im[c & 1], (int)min(32ll, max(0ll, left - 32 * c)), 32 * c, best, bi);
+            }
+            bi += t * kTile;
+        };
+        auto put = [&](int o, int, float wb, int wi) {
+            const int row = m0 + rl;
+            if (row >= args.M) return;
+            const int w0 = o * G;
+            const int w1 = (int)min((long long)w0 + G, (long long)args.ntiles);
+            if (args.pv && (t_begin > w0 || t_end < w1)) {
+                const long long pidx = ((long long)row * gridDim.y + tr) * 2 + (t_begin > w0 ? 0 : 1);
+                args.pv[pidx] = wb;
+                args.pi[pidx] = wi;
             } else {
-                tc_fence_after();
-#pragma unroll
-                for (int c = 0; c < 64; c += 32) {
-                    uint32_t re[32], im[32];
-                    tmem_ld_32x32b_x32(lane_base + (uint32_t)(b * 256 + hh * 64 + c), re);
-                    tmem_ld_32x32b_x32(lane_base + (uint32_t)(b * 256 + 128 + hh * 64 + c), im);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) asm volatile("" : "+r"(re[jj]), "+r"(im[jj]));
-                    const int cb = hh * 64 + c;
-                    const int valid = full_tile ? 32 : (int)min((long long)32, max(0ll, args.Tn - (col0 + cb)));
-                    float lb = -1.f;
-                    int lj = 0;
-#pragma unroll
-                    for (int jj = 0; jj < 32; ++jj) {
-                        const float xr = __uint_as_float(re[jj]), xm = __uint_as_float(im[jj]);
-                        const float p = jj < valid ? fmaf(xr, xr, xm * xm) : -1.f;
-                        if (p > lb) {
-                            lb = p;
-                            lj = jj;
-                        }
-                    }
-                    if (lb > best) {
-                        best = lb;
-                        bi = cb + lj;
-                    }
-                }
+                args.V[(long long)row * args.ldv + o] = wb;
+                args.I[(long long)row * args.ldv + o] = wi;
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(b ? tempty_l1 : tempty_l0);
-            if (hh == 1) {
-                xv[b * 128 + rl] = best;
-                xi[b * 128 + rl] = bi;
-            }
-            named_bar_sync(1, 32 * kEpiWarps);
-            if (hh == 0) {
-                const float ob = xv[b * 128 + rl];
-                const int oi = xi[b * 128 + rl];
-                if (ob > best) {
-                    best = ob;
-                    bi = oi;
-                }
-                const int gi = (int)(col0 + bi);
-                const bool first = (t % args.group) == 0 || t == t_begin;
-                const bool last = ((t + 1) % args.group) == 0 || t == args.ntiles - 1 || t == t_end - 1;
-                if (first || best > wb) {
-                    wb = best;
-                    wi = gi;
-                }
-                const int row = m0 + rl;
-                if (last && row < args.M) {
-                    const long long o = t / args.group;
-                    const int w0 = (int)(o * args.group);
-                    const int w1 = (int)min((long long)w0 + args.group, (long long)args.ntiles);
-                    if (args.pv && (t_begin > w0 || t_end < w1)) {
-                        const long long pidx = ((long long)row * gridDim.y + tr) * 2 + (t_begin > w0 ? 0 : 1);
-                        args.pv[pidx] = wb;
-                        args.pi[pidx] = wi;
-                    } else {
-                        args.V[(long long)row * args.ldv + o] = wb;
-                        args.I[(long long)row * args.ldv + o] = wi;
+        };
+        float wb;
+        int wi;
+        {
+            int par = 0;
+            for (int t = t_begin; t < t_end;) {
+                const int o = t / G, ts = t, te = (int)min((long long)(o + 1) * G, (long long)t_end);
+                wb = -2.f;
+                wi = 0;
+                for (; t < te; ++t) {
+                    const int i = t - t_begin;
+                    if ((i & 1) != g) continue;
+                    float best;
+                    int bi;
+                    item(i, t, best, bi);
+                    if (best > wb) {
+                        wb = best;
+                        wi = bi;
                     }
                 }
+                if (te - ts == 1) {                        // one tile: its group has the maximum
+                    if (((ts - t_begin) & 1) == g) put(o, 0, wb, wi);
+                    continue;
+                }
+                if (g == 1) {
+                    xv[par * 128 + rl] = wb;
+                    xi[par * 128 + rl] = wi;
+                }
+                named_bar_sync(1, 32 * kEpiWarps);         // the slots take turns: written again two outputs on
+                if (g == 0) {
+                    const float ob = xv[par * 128 + rl];
+                    const int oi = xi[par * 128 + rl];
+                    if (ob > wb || (ob == wb && oi < wi)) {
+                        wb = ob;
+                        wi = oi;
+                    }
+                    put(o, 0, wb, wi);
+                }
+                par ^= 1;
             }
         }
     }
