@@ -147,8 +147,11 @@ __global__ void __launch_bounds__(256) simt_absmax_kernel(const float* __restric
 //  - a window is shared out over a cluster of SPL CTAs (each walks its part of the blocks; rank 0 merges the maxima
 //    in block order through distributed shared memory), so that the last wave is a quarter of a window long.
 // Sums run over k in order with one rounding per FMA, so results are bit-identical to the kernel above.
-// Measured, 248 x 192 by 192 x 458,700, 1 s windows: 2,526 -> 1,759 us (49.7 TFLOP/s; 1,935 with pairs along samples, 16
-// duplicated A values per k); 64 templates x 118 rows of K by 475,136 samples: 855 -> 338 us (half the rows were padding).
+// Measured, 248 x 192 by 192 x 458,700, 1 s windows: 2,526 -> 1,728 us (50.6 TFLOP/s; 1,759 with each copy's address
+// taken anew from its step; 1,935 with pairs along samples, 16 duplicated A values per k; 1,915 with no duplicated value
+// but pairs (row, sample), (row + 1, sample + 1) and the crossed ones: three operands of 64 bits each then need more than
+// the register file reads in the two cycles of an instruction); 64 templates x 118 rows of K by 475,136 samples: 855 ->
+// 338 us (half the rows were padding). The FMA pipe is 78 % busy.
 // Pairs run along rows: A lies k-major in shared memory (4-byte copies), so a pair of rows is one register pair as read,
 // and only the 8 samples of a k are duplicated, not 16 A values. Thread (tx, ty) owns rows 8 ty .. 8 ty + 7 and samples
 // 4 tx + j, 64 + 4 tx + j (j < 4): a warp's A reads are two broadcast float4, its Z reads two runs of 256 bytes.
@@ -200,31 +203,50 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
     const int t0 = min(w0 + rank * share, w1), t1 = min(t0 + share, w1);
     const int nk = (K + BK - 1) / BK;
     const int nsteps = (t1 - t0) * nk;
-    auto load = [&](int step) {
-        float* sAr = smf + (step % AS_ST) * AS_STAGE;
-        float* sAi = sAr + AS_LD * BK;
-        float* sZ = sAi + AS_LD * BK;
-        const int t = t0 + step / nk, k0 = (step % nk) * BK;
-        constexpr int E = VEC ? 4 : 1;           // elements per copy
+    // Copies of the next step's tiles: (lt, lk) is its block and its place along K, ls its stage. A thread copies one k of
+    // the rows row0 + 8 r (rows past M are read as the last one: nothing is written for them) and samples zc .. of the
+    // k's zk + ZS r; pointers go on by a constant, and k's past K or samples past Tn are zero-filled.
+    constexpr int E = VEC ? 4 : 1, ZT = BN / E, ZS = AS_NT / ZT;  // samples per copy; threads and k's per round of copies
+    const int ak = tid % BK, row0 = tid / BK, rows = M - m0;
+    const int zk = tid / ZT, zc = tid % ZT * E;
+    const float* a_re = Are + (long long)(m0 + min(row0, rows - 1)) * lda;
+    const float* a_im = Aim + (long long)(m0 + min(row0, rows - 1)) * lda;
+    int lt = t0, lk = 0, ls = 0;
+    auto load = [&]() {
+        float* sA = smf + ls * AS_STAGE;
+        const int k0 = lk * BK;
+        {
+            const int kc = min(k0 + ak, K - 1), nb = k0 + ak < K ? 4 : 0;
+            const float* pr = a_re + kc;
+            const float* pi = a_im + kc;
+            float* d = sA + ak * AS_LD + row0;
 #pragma unroll
-        for (int r = 0; r < AS_BM * BK / AS_NT; ++r) {           // A: 64 rows x 16 k, transposed
-            const int e = tid + AS_NT * r;
-            const int row = e / BK, kk = e % BK;
-            const int gr = m0 + row, gk = k0 + kk;
-            const bool ok = gr < M && gk < K;
-            const long long off = ok ? (long long)gr * lda + gk : 0;
-            cp_async_zfill<4>(sAr + kk * AS_LD + row, Are + off, ok ? 4 : 0);
-            cp_async_zfill<4>(sAi + kk * AS_LD + row, Aim + off, ok ? 4 : 0);
+            for (int r = 0; r < AS_BM * BK / AS_NT; ++r) {       // A: 64 rows x 16 k, transposed
+                cp_async_zfill<4>(d + 8 * r, pr, nb);
+                cp_async_zfill<4>(d + 8 * r + AS_LD * BK, pi, nb);
+                if (row0 + 8 * (r + 1) < rows) {
+                    pr += 8 * lda;
+                    pi += 8 * lda;
+                }
+            }
         }
+        {
+            const long long gc = (long long)lt * BN + zc;
+            const int nc = gc < Tn ? (int)min((long long)(4 * E), (Tn - gc) * 4) : 0;
+            const float* pz = Z + (nc ? (long long)(k0 + zk) * ldz + gc : 0);
+            float* d = sA + 2 * AS_LD * BK + zk * BN + zc;
 #pragma unroll
-        for (int r = 0; r < BK * BN / E / AS_NT; ++r) {          // Z: 16 k x 128 samples
-            const int e = tid + AS_NT * r;
-            const int kk = e / (BN / E), cq = e % (BN / E) * E;
-            const int gk = k0 + kk;
-            const long long gc = (long long)t * BN + cq;
-            const int nb = (gk < K && gc < Tn) ? (int)min((long long)(4 * E), (Tn - gc) * 4) : 0;
-            cp_async_zfill<4 * E>(sZ + kk * BN + cq, Z + (nb ? (long long)gk * ldz + gc : 0), nb);
+            for (int r = 0; r < BK / ZS; ++r) {                  // Z: 16 k x 128 samples
+                const int nb = k0 + zk + ZS * r < K ? nc : 0;
+                cp_async_zfill<4 * E>(d + ZS * r * BN, nb ? pz : Z, nb);
+                pz += ZS * ldz;
+            }
         }
+        if (++lk == nk) {
+            lk = 0;
+            ++lt;
+        }
+        ls = ls + 1 == AS_ST ? 0 : ls + 1;
     };
     float wb[8];
     int wi[8];
@@ -240,17 +262,19 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
         for (int j = 0; j < 8; ++j) ar[i][j] = ai[i][j] = 0ull;
 #pragma unroll
     for (int s = 0; s < AS_ST - 1; ++s) {
-        if (s < nsteps) load(s);
+        if (s < nsteps) load();
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
+    int t = t0, k = 0, st = 0;                   // this step's block, place along K and stage
     for (int step = 0; step < nsteps; ++step) {
         asm volatile("cp.async.wait_group %0;" ::"n"(AS_ST - 2) : "memory");
         __syncthreads();                         // this step's tiles are in; every thread is done with step - 1's
-        if (step + AS_ST - 1 < nsteps) load(step + AS_ST - 1);
+        if (step + AS_ST - 1 < nsteps) load();
         asm volatile("cp.async.commit_group;" ::: "memory");
-        const float* sAr = smf + (step % AS_ST) * AS_STAGE;
+        const float* sAr = smf + st * AS_STAGE;
         const float* sAi = sAr + AS_LD * BK;
         const float* sZ = sAi + AS_LD * BK;
+        st = st + 1 == AS_ST ? 0 : st + 1;
 #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
             const float4 z0 = *reinterpret_cast<const float4*>(sZ + kk * BN + 4 * tx);
@@ -269,10 +293,9 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
                 }
             }
         }
-        if (step % nk == nk - 1) {
+        if (++k == nk) {
             // |z|^2, max and first index per row over this thread's 8 samples (increasing order), then over the 16
             // threads of the row; then the running window maximum
-            const int t = t0 + step / nk;
             const long long c0 = (long long)t * BN;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -304,6 +327,8 @@ __global__ void __launch_bounds__(AS_NT, 2) simt_absmax_packed_kernel(
             for (int i = 0; i < 4; ++i)
 #pragma unroll
                 for (int j = 0; j < 8; ++j) ar[i][j] = ai[i][j] = 0ull;
+            k = 0;
+            ++t;
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
