@@ -158,7 +158,8 @@ int gwb_filter_step(const GwbTile* tiles, int ntiles, const float* H, long long 
     GWB_CUDA(cudaMemsetAsync(w.Z, 0, 2ll * s.K * s.ldz, st));
     if (w.Zlo) GWB_CUDA(cudaMemsetAsync(w.Zlo, 0, 2ll * s.K * s.ldz, st));
     // template norms (float64) and every segment's D isw in four-step order
-    GWB_TRY(gwb_sigma2_band(H, ldh, M, kmax, IP, ldip, nseg, kmin, flen, df, w.part, gwb_sigma2_part_elems(M, nseg), sig, nseg, st));
+    // (over whole rows: kmax is where the chi-squared band ends, and the caller's templates may go on)
+    GWB_TRY(gwb_sigma2(H, ldh, M, IP, ldip, nseg, kmin, flen, df, w.part, gwb_sigma2_part_elems(M, nseg), sig, nseg, st));
     GWB_TRY(gwb_fourstep_order(D, ldd, nseg, isw, flen, tlen, w.Dp, s.ldp, st));
     GWB_TRY(gwb_fft_twiddles(tlen, w.tw, st));
     const float thr2 = (float)((double)cfg->snr_threshold * (1.0 - cfg->margin) *
