@@ -176,7 +176,8 @@ class FusedBasisWorkspace:
         self.ring = bool(ring)
         self.nfirst = 2 if ring is None and tlen == RING_N else RB      # rows behind the scale
         assert not self.ring or tlen == RING_N, 'the ring form is for tlen = 2^20'
-        self.wrows = rows if wrows is None else max(min(2, rows) if ring is None else 1, min(int(wrows), rows))
+        least = min(2, rows) if self.nfirst < RB else 1    # the scale's two rows are of one batch
+        self.wrows = rows if wrows is None else max(least, min(int(wrows), rows))
         lib = _lib.load()
         wr = lib.gwb_basis_ring_rows() if self.ring else self.wrows
         self.W = torch.empty((wr, tlen), dtype=torch.complex64, device=device)
@@ -233,8 +234,7 @@ class BasisWorkspace:
 class SeriesWorkspace:
     """Device buffers of the reference's basis series through the fused passes (gwb_basis_series, power-of-two tlen in
     [FUSED_MIN, FUSED_MAX]): a batch of basis filters and the data in four-step order, and the batch's transform between
-    the passes. 100 rows of 2^20, fp16 Z: 1,517 us a call through premul,
-    cuFFT and pack, 958 so."""
+    the passes. 100 rows of 2^20, fp16 Z: 1,517 us a call through premul, cuFFT and pack, 958 so."""
 
     def __init__(self, tlen, flen, rows=RB, device='cuda'):
         self.tlen, self.flen, self.rows = tlen, flen, rows
