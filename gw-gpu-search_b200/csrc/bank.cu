@@ -27,8 +27,8 @@ double* g_scratch_ptr[64] = {nullptr};
 // Split-k partial sums of sig for a block of 64 rows x 8 NT segments on the float64 matrix instruction
 // (mma.m8n8k4.f64: products and sums in float64, as an FMA chain). Four warps, each 16 rows (two A fragments) x all
 // 8 NT segments; a chunk is 32 bins. A warp loads its rows' H one chunk ahead, 32 consecutive bins of a row per load
-// (loads in fragment order, 8 rows x 4 bins, reached 2.4 TB/s: 440 us at 16 segments, now 216, 5.0 TB/s), forms |H|^2 in float64 (exact from complex64) and
-// turns it to fragment order through its own shared tile; IP goes through shared memory once per chunk, converted to
+// (loads in fragment order, 8 rows x 4 bins, reached 2.4 TB/s: 440 us at 16 segments, now 215, 5.0 TB/s), forms |H|^2
+// in float64 (exact from complex64) and turns it to fragment order through its own shared tile; IP goes through shared memory once per chunk, converted to
 // float64 for all four warps (row stride 36 doubles: a fragment read hits 16 distinct bank pairs per half-warp).
 // Templates end at f_ISCO, so most chunks of a row are zero: a warp whose 16 x 32 values are all zero multiplies
 // nothing, unless the chunk's IP holds a value that is not finite (then 0 * inf must give the NaN it always gave).

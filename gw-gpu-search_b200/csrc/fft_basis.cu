@@ -1670,7 +1670,9 @@ int gwb_basis_series(const float* Vh, long long ldv, int rows, const float* D, c
             case 128: st = launch_pass1<128>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
             case 256: st = launch_pass1<256>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
             case 512: st = launch_pass1<512>(v, ldvp, nr, d, n, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, s); break;
-            default: st = launch_pass1_w(v, ldvp, nr, d, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, n / 2 + 1, nullptr, s); break;
+            default:
+                st = launch_pass1_w(v, ldvp, nr, d, N2, t, w, 0, nullptr, nullptr, nullptr, nullptr, n / 2 + 1, nullptr, s);
+                break;
         }
         if (st) break;
         switch (N2) {

@@ -202,8 +202,9 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
             }
         }
     } else if (warp == 1) {
-        // the whole warp runs the loop and one elected lane issues, so that descriptors, TMEM addresses and loop state stay
-        // in the uniform registers that tcgen05.mma reads
+        // the whole warp runs the loop and one elected lane issues, so that descriptors, TMEM addresses and loop state
+        // stay in the uniform registers that tcgen05.mma reads (in a one-lane branch each MMA's operands were moved
+        // there first: the C2 step's fp16 launches 861 -> 793 ms, split bf16 at Kh = 128 449 -> 395 us a launch)
         {
             const bool el = elect_lane();
             const uint32_t tm = (uint32_t)warp_uniform((int)tmem);
@@ -219,8 +220,8 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
             // the MMAs of one item (M block mb) on one Z chunk. One-product forms: every descriptor of the chunk is
             // formed first (base descriptors plus offsets), then the MMAs go out back to back in the same order (sk,
             // four real products), so the one issuing thread spends no address arithmetic between them (measured
-            // 0.266 -> 0.253 ms at n = 256, r = 128, fp16). The split form keeps descriptors and MMAs interleaved (the burst measured slower there:
-            // one K step per chunk when A lo is streamed).
+            // 0.266 -> 0.253 ms at n = 256, r = 128, fp16). The split form keeps descriptors and MMAs interleaved (the
+            // burst measured slower there: one K step per chunk when A lo is streamed).
             auto issue = [&](int kc, int mb, int b, uint32_t st) {
                 if constexpr (C::NPROD == 1) {
                     constexpr int MAXS = 4;                      // K steps per chunk: KC / KSTEP (64/16, 128/32)
@@ -368,8 +369,10 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
         }
         __syncwarp();
     } else {
-        // two groups of four warps: group g takes the items of accumulator buffer g (with two M blocks, always M block g),
-        // so a group has two items' time for one, and with one M block the two meet once per output window, not per tile
+        // two groups of four warps: group g takes the items of accumulator buffer g (with two M blocks, always M block
+        // g), so a group has two items' time for one, and with one M block the two meet once per output window, not per
+        // tile (all eight warps on every tile, halves merged across a barrier: the C2 step's fp16 launches 793 ms, now
+        // 697; split bf16 1,342, now 1,318)
         const int q = warp & 3, g = (warp - 2) >> 2;
         const int rl = 32 * q + lane;
         const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(g * 256);

@@ -149,9 +149,10 @@ __global__ void __launch_bounds__(256) simt_absmax_kernel(const float* __restric
 // Sums run over k in order with one rounding per FMA, so results are bit-identical to the kernel above.
 // Measured, 248 x 192 by 192 x 458,700, 1 s windows: 2,526 -> 1,728 us (50.6 TFLOP/s; 1,759 with each copy's address
 // taken anew from its step; 1,935 with pairs along samples, 16 duplicated A values per k; 1,915 with no duplicated value
-// but pairs (row, sample), (row + 1, sample + 1) and the crossed ones: three operands of 64 bits each then need more than
-// the register file reads in the two cycles of an instruction); 64 templates x 118 rows of K by 475,136 samples: 855 ->
-// 338 us (half the rows were padding). The FMA pipe is 78 % busy.
+// but pairs (row, sample), (row + 1, sample + 1) and the crossed ones: three operands of 64 bits an instruction, which the
+// register file presumably does not read in its two cycles); 64 templates x 118 rows of K by 475,136 samples: 855 ->
+// 326 us (half the rows were padding). The FMA pipe is 78 % busy while a CTA runs; the waits of two warps per scheduler
+// for each other's operand steps and the last wave are the rest.
 // Pairs run along rows: A lies k-major in shared memory (4-byte copies), so a pair of rows is one register pair as read,
 // and only the 8 samples of a k are duplicated, not 16 A values. Thread (tx, ty) owns rows 8 ty .. 8 ty + 7 and samples
 // 4 tx + j, 64 + 4 tx + j (j < 4): a warp's A reads are two broadcast float4, its Z reads two runs of 256 bytes.
@@ -424,7 +425,8 @@ extern "C" int gwb_fused_peaks_f32(const float* Are, const float* Aim, long long
         // windows are shared out over clusters while whole windows would leave the last of few waves nearly empty
         // (two CTAs per SM; from 32 waves on it is a thirty-second at most) and a part still holds two blocks
         const long long items = nout * cdiv(M, AS_BM);
-        const int spl = items >= 32ll * 2 * num_sms() || nout * AS_MAXSPL >= (1ll << 31) ? 1 : group >= 8 ? 4 : group >= 4 ? 2 : 1;
+        const bool whole = items >= 32ll * 2 * num_sms() || nout * AS_MAXSPL >= (1ll << 31);
+        const int spl = whole ? 1 : group >= 8 ? 4 : group >= 4 ? 2 : 1;
         auto go = [&](auto v) {
             constexpr bool VEC = decltype(v)::value;
             cudaStream_t st = (cudaStream_t)stream;
