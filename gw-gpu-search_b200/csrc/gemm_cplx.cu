@@ -950,18 +950,31 @@ __global__ void window_merge_kernel(int M, int ntiles, int group, int nout, int 
     I[(long long)row * ldv + o] = bi;
 }
 
-// Launch configuration per (form, Kh) from the autotuner's table (gwb_gemm_set_config). Defaults: CTA pairs for
-// fp16 / bf16, the deepest Z ring that fits, the MMA order 0.
+// Launch configuration per (form, Kh) from the autotuner's table (gwb_gemm_set_config), else by size. Every choice here
+// gives the same bits. Times are ms at Tn = 917,504 (pair against one CTA per M block).
+// - A pair works on two M blocks, so an odd count pays for one of zeros. One block: one CTA (fp16 at Kh = 128 0.210
+//   against 0.139, split bf16 0.401 against 0.303, fp16 with split A 0.288 against 0.198). Three or five blocks: one CTA
+//   as long as it is slower per block by less than the padding, which holds up to a product of blocks and Kh (three
+//   blocks, Kh = 128: fp16 0.404 / 0.378; split bf16 at 32 0.372 / 0.283 but at 64 0.438 / 0.462; fp16 with split A at 96
+//   0.478 / 0.457 but at 128 0.601 / 0.634).
+// - fp16 with split A on even counts: pairs from Kh = 64 on (two blocks: 0.217 / 0.218 at 64, 0.309 / 0.397 at 128,
+//   0.464 / 0.745 at 192; 0.186 / 0.179 at 32).
+// - Order of the split forms' pairs (1: K chunks of 64): split bf16 order 1 where A lo stays resident (Kh = 64: 0.272 ->
+//   0.238) and from 192 on (equal), between them order 0, whose chunks of 32 leave more stages beside the streamed A lo
+//   (Kh = 144: 0.672 -> 0.550, 160: 0.611 -> 0.544); fp16 with split A order 1 up to 160 (0.415 -> 0.397 there).
 struct GemmTune {
     int form, kh, pair, stages, order;
 };
 
-GemmTune gemm_tune(int form, int kh) {
-    // without a table entry: CTA pairs, except for fp16 with split A (one CTA per M block: measured 0.368 against
-    // 0.404 ms at n = 256, Kh = 128; the pair is faster at Kh = 192, 0.569 against 0.616, where the autotuner picks
-    // it); split bf16 with order 1, K chunks of 64 where A hi and lo stay resident (0.526 -> 0.488 ms at Kh = 128)
-    GemmTune t{form, kh, form == 6 ? 0 : 1, 0, form == 2 ? 1 : 0};
-    tune_lookup(form, kh, &t.pair, &t.stages, &t.order);
+// one_ok: the workspace is large enough for one CTA per M block
+GemmTune gemm_tune(int form, int kh, int M, bool one_ok) {
+    GemmTune t{form, kh, 1, 0, 0};
+    if (tune_lookup(form, kh, &t.pair, &t.stages, &t.order)) return t;
+    const int blocks = (M + 127) / 128;
+    const int padding_pays = form == 2 ? 96 : form == 6 ? 320 : 384;
+    const bool one = blocks == 1 || (blocks % 2 == 1 && (long long)blocks * kh <= padding_pays) || (form == 6 && kh < 64);
+    t.pair = one && one_ok ? 0 : 1;
+    if (t.pair) t.order = form == 2 ? (kh <= 128 || kh >= 192) : form == 6 ? kh <= 160 : 0;
     return t;
 }
 
@@ -1117,7 +1130,7 @@ int launch_cplx(const void* const* A, const void* const* Zp, long long lda, long
     // 128, Tn = 917,504; the second M group's Z reads hit L2), with the TMEM double buffer spanning tiles. The kernel
     // also runs two M blocks per CTA (each Z tile read once for both) when MB = 2.
     const int MB = 1;
-    const GemmTune tune = gemm_tune(FORM, Kh);
+    const GemmTune tune = gemm_tune(FORM, Kh, M, work_bytes >= 16ll * M * std::max(1, num_sms() / (int)cdiv(M, 128)));
     int stages = most_stages(MB);
     if (tune.stages >= 2 && stages >= 2) stages = std::min(stages, tune.stages);
     // split A beyond Kh = 128: A hi + lo no longer fit beside the Z ring, so A lo is streamed with it
