@@ -81,6 +81,7 @@ class Bank:
             r0 += len(ids)
         self.kmax = torch.from_numpy(km).to(device)
         self.kmax_h = km
+        self.ends = self.kmax.clone()       # where the templates end, whatever becomes of the chi-squared bands
         self.nbins = torch.full((M,), cfg.nbins, dtype=torch.int32, device=device)
         self.svd = []
         for t, ids in enumerate(self.tiles):
@@ -111,12 +112,6 @@ class MatchedFilter:
         self.compact = self.form != 'f32'
         self.fp8 = self.form == 'fp8'
         rmax = max(s['r'] for s in bank.svd)
-        # where the templates end, read from the templates themselves (the norms stop there)
-        self.ends = torch.empty(bank.M, dtype=torch.int32, device=device)
-        for t, ids in enumerate(bank.tiles):
-            rows = slice(bank.row0[t], bank.row0[t] + len(ids))
-            nz = bank.H[rows] != 0
-            self.ends[rows] = torch.where(nz.any(1), bank.flen - nz.flip(1).to(torch.uint8).argmax(1), 0).int()
         # the fused two-pass basis series (premul and pack folded into the transform passes) where the length allows,
         # else premul + cuFFT + pack
         self.fused = fp_filter.FUSED_MIN <= tlen <= fp_filter.FUSED_MAX
@@ -295,9 +290,9 @@ class MatchedFilter:
         sig = torch.empty((b.M, nseg), dtype=torch.float64, device=IP.device)
         part_elems = _lib.load().gwb_sigma2_part_elems(b.M, nseg)
         part = torch.empty(part_elems, dtype=torch.float64, device=IP.device)
-        _lib.call('gwb_sigma2_band', _lib.ptr(b.H), b.H.stride(0), b.M, _lib.ptr(self.ends), _lib.ptr(IP),
-                  _lib.row_stride(IP), nseg, b.kmin, b.flen, float(b.df), _lib.ptr(part), part_elems, _lib.ptr(sig),
-                  sig.stride(0), _lib.stream_ptr())
+        _lib.call('gwb_sigma2_band', _lib.ptr(b.H), b.H.stride(0), b.M, _lib.ptr(getattr(b, 'ends', None)),
+                  _lib.ptr(IP), _lib.row_stride(IP), nseg, b.kmin, b.flen, float(b.df), _lib.ptr(part), part_elems,
+                  _lib.ptr(sig), sig.stride(0), _lib.stream_ptr())
         self.kernel_launches += 2
         return sig
 
