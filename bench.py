@@ -432,11 +432,11 @@ def run_c2(a):
             split[name] = a_.elapsed_time(b_)
         split['total'] = ec[0].elapsed_time(ep)
         split = {k: round(v, 3) for k, v in split.items()}
-        # algorithmic HBM bytes of one basis-series call (both passes): Vp read (tlen/2 + 1 complex per row), W
-        # written and read back (tlen complex per row), Z written (re + im over Tn, one or two 16-bit planes, fp32 or
-        # fp8)
+        # algorithmic HBM bytes of one basis-series call (both passes), the mean over the tiles (each runs once per
+        # chunk): Vp read (complex, up to the bin where the tile's templates end), W written and read back (tlen complex
+        # per row), Z written (re + im over Tn, one or two 16-bit planes, fp32 or fp8)
         zb = {'bf16x3': 8, 'f16': 4, 'f16x2': 4, 'bf16': 4, 'f32': 8, 'fp8': 2}[form]
-        b_bytes = [r * (8 * (mf.tlen // 2 + 1) + 16 * mf.tlen + zb * mf.Tn) for e, n, r, kp in L]
+        b_bytes = [t['r'] * (8 * min(k, mf.tlen // 2 + 1) + 16 * mf.tlen + zb * mf.Tn) for t, k in zip(B.svd, mf.kend)]
         useful = [8.0 * n * r * mf.Tn for e, n, r, kp in L]
         nprod = {'bf16x3': 3, 'f16x2': 2}.get(form, 1)
         issued = [nprod * 4.0 * n * kp * mf.Tn for e, n, r, kp in L]
