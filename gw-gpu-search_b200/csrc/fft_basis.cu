@@ -302,16 +302,24 @@ constexpr int RC = 8;   // rows per pass-1 CTA of the warp-per-column form
 // A of a column's 16 runs of 32 bins are live (k1 < 32 A holds every k < kend): the others are neither loaded nor
 // multiplied, and the first DFT starts from A inputs. The outputs are those of the full kernel bit for bit (up to the
 // sign of exact zeros) as long as D is finite from kend on; where it is not (*last_bad >= kend), 0 * D puts a NaN into
-// every output, and so does this kernel. 122 rows of 2^20 at A = 1: 315 -> 240 us (W's
-// store is 157 at the measured copy rate).
+// every output, and so does this kernel. At A = 1 the exchange between the two DFTs shrinks to the warp's 32 inputs, which
+// every lane reads as broadcasts. 122 rows of 2^20 at A = 1: 315 -> 204 us (242 with the general exchange, whose waits on
+// shared memory were the largest stall; 229 at three CTAs per SM, 80 registers with spills; W's store is 157 at the
+// measured copy rate).
+// float2 of shared memory per warp: exchange, TH, basis-filter segment
+template <int A>
+struct Pass1Shared {
+    static constexpr int Y = A == 1 ? 32 : 32 * 33, V = A == 1 ? 32 : 512, TOTAL = Y + 32 + V;
+};
+
 template <int N2, int A>
 __global__ void __launch_bounds__(256, 2) basis_pass1_w(
     const float2* __restrict__ Vp, long long ldvp, int rows, const float2* __restrict__ Dp,
     const float2* __restrict__ tw, float2* __restrict__ W, int nfirst, double* __restrict__ partials,
     unsigned int* __restrict__ ticket, float* __restrict__ scale_out, float* __restrict__ rowpart, int kend,
     const int* __restrict__ last_bad) {
-    constexpr int N1 = 1024, N = N1 * N2, R = 32, H = N1 / 2, NW = 8, YS = R * (R + 1);
-    constexpr int WS = YS + R + H;                          // per warp: Y tile, TH, basis-filter segment
+    constexpr int N1 = 1024, N = N1 * N2, R = 32, H = N1 / 2, NW = 8, YS = Pass1Shared<A>::Y;
+    constexpr int WS = Pass1Shared<A>::TOTAL;
     static_assert(A >= 1 && A <= R / 2, "live runs");
     extern __shared__ float2 sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -375,15 +383,28 @@ __global__ void __launch_bounds__(256, 2) basis_pass1_w(
                 if (lane == 0) rowpart[(long long)j * N2 + k2] = ps;
             }
         }
-        if constexpr (A == R / 2) dft_reg_upper_zero<R>(x); // q is zero for k1 > N1 / 2
-        else dft_reg_zero_from<A, R>(x);
-        static_for<R>([&](auto U) {
-            constexpr int u = decltype(U)::value;
-            Yw[lane * (R + 1) + u] = cmul(x[brev(u, ilog2(R))], tw2[u * R + lane]);
-        });
-        __syncwarp();
+        if constexpr (A == 1) {
+            // one input: the first DFT's 32 outputs are all q_b, so lane u reads the warp's 32 q_b (broadcasts) and
+            // twiddles them itself (tw2 is symmetric): the same products without the exchange of 1,024 values
+            Yw[lane] = x[0];
+            __syncwarp();
 #pragma unroll
-        for (int bb = 0; bb < R; ++bb) x[bb] = Yw[bb * (R + 1) + lane];
+            for (int bb = 0; bb < R; bb += 2) {
+                const float4 q2 = *reinterpret_cast<const float4*>(Yw + bb);
+                x[bb] = cmul(make_float2(q2.x, q2.y), tw2[bb * R + lane]);
+                x[bb + 1] = cmul(make_float2(q2.z, q2.w), tw2[(bb + 1) * R + lane]);
+            }
+        } else {
+            if constexpr (A == R / 2) dft_reg_upper_zero<R>(x); // q is zero for k1 > N1 / 2
+            else dft_reg_zero_from<A, R>(x);
+            static_for<R>([&](auto U) {
+                constexpr int u = decltype(U)::value;
+                Yw[lane * (R + 1) + u] = cmul(x[brev(u, ilog2(R))], tw2[u * R + lane]);
+            });
+            __syncwarp();
+#pragma unroll
+            for (int bb = 0; bb < R; ++bb) x[bb] = Yw[bb * (R + 1) + lane];
+        }
         __syncwarp();
         dft_reg<R>(x);
         // t1 = lane + 32 v: W block t1 / 8 = 4 v + lane / 8, position lane % 8
@@ -1266,7 +1287,7 @@ template <int N2, int A>
 int launch_pass1_wa(const float2* Vp, long long ldvp, int rows, const float2* Dp, const float2* tw, float2* W, int nfirst,
                     double* partials, unsigned* ticket, float* scale_out, float* rowpart, int kend, const int* last_bad,
                     cudaStream_t s) {
-    const size_t smem = (size_t)(1024 + 8 * (32 * 33 + 32 + 512)) * sizeof(float2);
+    const size_t smem = (size_t)(1024 + 8 * Pass1Shared<A>::TOTAL) * sizeof(float2);
     auto k = basis_pass1_w<N2, A>;
     GWB_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k<<<dim3(N2 / 8, (rows + RC - 1) / RC), 256, smem, s>>>(Vp, ldvp, rows, Dp, tw, W, nfirst, partials, ticket,
