@@ -1387,6 +1387,11 @@ int launch_pass2_w(const float2* W, int N, int N1, int rows, const float2* tw, i
 // (basis_pass2_p, or the per-row kernel for the split form)
 std::atomic<int> g_pass2_cols[5] = {{16}, {16}, {16}, {16}, {16}};
 
+// whether launch_pass2 takes a kernel that copies W to shared memory 16 bytes at a time
+bool pass2_copies16(int N2, int form) {
+    return N2 == 1024 ? form != 2 || g_pass2_cols[form].load() == 16 : N2 >= 512 && form != 2;
+}
+
 template <int N2>
 int launch_pass2(int form, const float2* W, int N, int N1, int rows, const float2* tw, int a0, int Tn,
                  const float* scale, void* Z, void* Zlo, long long ldz, int im_off, int row0, cudaStream_t s) {
@@ -1615,6 +1620,7 @@ int gwb_basis_fused_band(const float* Vp, long long ldvp, int rows, const float*
                   "basis_fused: scale partials need %lld entries", need);
     GWB_CHECK_ARG(N1 != 1024 || ((uintptr_t)Vp % 16 == 0 && ldvp % 2 == 0), GWB_ERR_ALIGN,
                   "basis_fused: Vp and its row stride must be 16-byte aligned");
+    GWB_CHECK_ARG(!pass2_copies16(N2, form) || aligned(W, 16), GWB_ERR_ALIGN, "basis_fused: W must be 16-byte aligned");
     // fp8: per-row partial sums of |q|^2 (P per row) and one scale per row
     const int P = N1 == 1024 ? N2 : N2 / TB;
     const long long pneed = (long long)std::min(rows, wrows) * P;
@@ -1675,6 +1681,10 @@ int gwb_basis_series(const float* Vh, long long ldv, int rows, const float* D, c
                   rows <= im_off, GWB_ERR_SHAPE, "basis_series: rows=%d wrows=%d a0=%lld Tn=%lld", rows, wrows, a0, Tn);
     const int N1 = 1 << ((log2i(N) + 1) / 2), N2 = (int)(N / N1);
     const long long ldvp = N / 2 + 2;                      // even: 16-byte aligned rows
+    GWB_CHECK_ARG(N1 != 1024 || aligned(Vp, 16), GWB_ERR_ALIGN, "basis_series: Vp must be 16-byte aligned");
+    // the power form of pass 2 at N2 = 1024 copies W as its row-chunk form does, whatever the Z encoding
+    GWB_CHECK_ARG(!(N2 == 1024 || pass2_copies16(N2, form)) || aligned(W, 16), GWB_ERR_ALIGN,
+                  "basis_series: W must be 16-byte aligned");
     cudaStream_t s = (cudaStream_t)stream;
     const float2* t = reinterpret_cast<const float2*>(tw);
     const float2* v = reinterpret_cast<const float2*>(Vp);

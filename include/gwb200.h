@@ -348,7 +348,8 @@ GWB_API int gwb_basis_set_pass2_pairs(int on);
  * that span (written to scale). Both are reordered (gwb_fourstep_order) and go through the two fused passes in batches
  * of wrows rows; the first batch's second pass runs once more to sum its power. Vp: wrows x (N / 2 + 2) complex, Dp:
  * N / 2 + 2, W: wrows x N, partials: wrows x 128 doubles. isw may be NULL (D already divided). form: 0-3 as
- * gwb_basis_pack. */
+ * gwb_basis_pack. Vp (from N = 2^19 on) and W (from N = 2^18 on; for form 2 at N = 2^20) are copied 16 bytes at a time:
+ * GWB_ERR_ALIGN where they do not lie on such a boundary, as from gwb_basis_fused. */
 GWB_API int gwb_basis_series(const float* Vh, long long ldv, int rows, const float* D, const float* isw, long long flen,
                              long long N, const float* tw, float* Vp, float* Dp, float* W, int wrows, long long a0,
                              long long Tn, int form, void* Z, void* Zlo, long long ldz, int im_off, double* partials,
