@@ -28,8 +28,9 @@ double* g_scratch_ptr[64] = {nullptr};
 // (mma.m8n8k4.f64: products and sums in float64, as an FMA chain). Four warps, each 16 rows (two A fragments) x all
 // 8 NT segments; a chunk is 32 bins. A warp loads its rows' H one chunk ahead, 32 consecutive bins of a row per load
 // (loads in fragment order, 8 rows x 4 bins, reached 2.4 TB/s: 440 us at 16 segments, now 215, 5.0 TB/s), forms |H|^2
-// in float64 (exact from complex64) and turns it to fragment order through its own shared tile; IP goes through shared memory once per chunk, converted to
-// float64 for all four warps (row stride 36 doubles: a fragment read hits 16 distinct bank pairs per half-warp).
+// in float64 (exact from complex64) and turns it to fragment order through its own shared tile; IP goes through shared
+// memory once per chunk, converted to float64 for all four warps (row stride 36 doubles: a fragment read hits 16 distinct
+// bank pairs per half-warp).
 // Templates end at f_ISCO, so most chunks of a row are zero: a warp whose 16 x 32 values are all zero multiplies
 // nothing, unless the chunk's IP holds a value that is not finite (then 0 * inf must give the NaN it always gave).
 // NT is the smallest of 1, 2, 4, 8 that covers the segments: 64-wide blocks for one or a few segments did up to 64
@@ -184,6 +185,34 @@ __global__ void __launch_bounds__(512) sigma2_reduce_kernel(const double* __rest
 int sigma2_splits(int n, int nseg) {
     const long long blocks = cdiv(n, kSR) * cdiv(nseg, 64);
     return (int)std::max(16ll, std::min(512ll, 8ll * 148 / blocks));
+}
+
+// Where each row ends: one past its last value that is not zero (a NaN is not), 0 for a row of zeros. A CTA per row looks
+// from the end, so only the zeros behind a template are read. Once per filter object: no figure.
+__global__ void __launch_bounds__(1024) row_ends_kernel(const float2* __restrict__ H, long long ldh, int flen,
+                                                        int32_t* __restrict__ ends) {
+    const float2* h = H + (long long)blockIdx.x * ldh;
+    __shared__ int s_end;
+    if (threadIdx.x == 0) s_end = 0;
+    constexpr int U = 4;
+    for (int hi = flen; hi > 0; hi -= U * 1024) {
+        int e = 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = hi - 1 - u * 1024 - (int)threadIdx.x;
+            if (k >= 0) {
+                const float2 v = __ldg(h + k);
+                if (v.x != 0.f || v.y != 0.f) e = max(e, k + 1);
+            }
+        }
+        if (__syncthreads_or(e > 0)) {
+            e = __reduce_max_sync(0xffffffffu, e);
+            if (threadIdx.x % 32 == 0 && e > 0) atomicMax(&s_end, e);
+            break;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) ends[blockIdx.x] = s_end;
 }
 
 constexpr int kG = 32;   // Gram block: 32 x 32 outputs
@@ -384,6 +413,16 @@ int gwb_sigma2_band(const float* H, long long ldh, int n, const int32_t* kmax, c
     sigma2_reduce_kernel<<<(unsigned)cdiv((long long)n * nseg, 32), 512, 0, s>>>(part, nsplit, n, nseg, 4.0 * df, sig,
                                                                                 ldsig);
     GWB_LAUNCH_CHECK("sigma2_reduce_kernel");
+    return GWB_OK;
+}
+
+int gwb_row_ends(const float* H, long long ldh, int n, int flen, int32_t* ends, void* stream) {
+    using namespace gwb;
+    GWB_CHECK_ARG(H && ends, GWB_ERR_ARG, "row_ends: null pointer");
+    GWB_CHECK_ARG(n > 0 && flen > 0 && flen < (1 << 30) && ldh >= flen, GWB_ERR_SHAPE, "row_ends: n=%d flen=%d ldh=%lld",
+                  n, flen, ldh);
+    row_ends_kernel<<<n, 1024, 0, (cudaStream_t)stream>>>(reinterpret_cast<const float2*>(H), ldh, flen, ends);
+    GWB_LAUNCH_CHECK("row_ends_kernel");
     return GWB_OK;
 }
 

@@ -37,6 +37,15 @@ def derive_sw(IPall):
     return sw, isw
 
 
+def row_ends(H, out=None):
+    """Per row of H (n, flen) complex64 one past its last bin that is not zero (int32; 0 for a row of zeros)."""
+    _lib.require_cuda(H)
+    n, flen = H.shape
+    out = torch.empty(n, dtype=torch.int32, device=H.device) if out is None else out
+    _lib.call('gwb_row_ends', _lib.ptr(H), _lib.row_stride(H), n, flen, _lib.ptr(out), _lib.stream_ptr(H.device))
+    return out
+
+
 def sigma2(H, IPall, df, kmin=0):
     """Template norms (fp_filter.py:710-714) in float64: sig (n, nseg) = 4 df |H|^2 @ IP^T; norm = 4 df / sqrt(sig)."""
     _lib.require_cuda(H, IPall)

@@ -81,7 +81,6 @@ class Bank:
             r0 += len(ids)
         self.kmax = torch.from_numpy(km).to(device)
         self.kmax_h = km
-        self.ends = self.kmax.clone()       # where the templates end, whatever becomes of the chi-squared bands
         self.nbins = torch.full((M,), cfg.nbins, dtype=torch.int32, device=device)
         self.svd = []
         for t, ids in enumerate(self.tiles):
@@ -95,7 +94,8 @@ class Bank:
 
 
 class MatchedFilter:
-    """Runs steps of the batched filter for one bank and one segment geometry (tlen, analysed span)."""
+    """Runs steps of the batched filter for one bank and one segment geometry (tlen, analysed span), for the templates
+    and the basis filters that the bank holds when the object is made (they may be a caller's own)."""
 
     def __init__(self, bank: Bank, tlen, a0, Tn, cfg: FilterConfig, device='cuda'):
         self.bank, self.cfg = bank, cfg
@@ -127,6 +127,10 @@ class MatchedFilter:
             ends = torch.empty(len(bank.svd), dtype=torch.int32, device=device)
             self.vp = [fp_filter.fourstep_order(s['Vh'], tlen, last_nz=ends[t:t + 1]) for t, s in enumerate(bank.svd)]
             self.kend = [int(e) + 1 for e in ends.cpu()]
+            # and where each tile's templates end, for the norms of a step
+            self.ends = fp_filter.row_ends(bank.H)
+            for r0, ids in zip(bank.row0, bank.tiles):
+                self.ends[r0:r0 + len(ids)] = self.ends[r0:r0 + len(ids)].max()
             self.last_bad = None
             self.Dp = None
         else:
@@ -283,14 +287,15 @@ class MatchedFilter:
             self.kernel_launches += 2 * nb + 4  # premul and pack per batch; scale, stacked A, GEMM, selection
             self.fft_launches += nb
 
-    def norms(self, IP):
-        """Template norms for every (row, segment): sig (M, S) float64 = 4 df sum |H|^2 IP (fp_filter.py:710-714)."""
+    def norms(self, IP, ends=None):
+        """Template norms for every (row, segment): sig (M, S) float64 = 4 df sum |H|^2 IP (fp_filter.py:710-714). ends:
+        the bins from which the rows are zero (int32, on the device), which are then not read; None: whole rows."""
         b = self.bank
         nseg = IP.shape[0]
         sig = torch.empty((b.M, nseg), dtype=torch.float64, device=IP.device)
         part_elems = _lib.load().gwb_sigma2_part_elems(b.M, nseg)
         part = torch.empty(part_elems, dtype=torch.float64, device=IP.device)
-        _lib.call('gwb_sigma2_band', _lib.ptr(b.H), b.H.stride(0), b.M, _lib.ptr(getattr(b, 'ends', None)),
+        _lib.call('gwb_sigma2_band', _lib.ptr(b.H), b.H.stride(0), b.M, _lib.ptr(ends),
                   _lib.ptr(IP), _lib.row_stride(IP), nseg, b.kmin, b.flen, float(b.df), _lib.ptr(part), part_elems,
                   _lib.ptr(sig), sig.stride(0), _lib.stream_ptr())
         self.kernel_launches += 2
@@ -354,7 +359,7 @@ class MatchedFilter:
         if prof is not None:
             e_n = (ev(), ev())
             e_n[0].record()
-        sig = self.norms(IP)
+        sig = self.norms(IP, self.ends if self.fused else None)
         if prof is not None:
             e_n[1].record()
             prof.setdefault('parts', []).append(('norms', e_n))

@@ -236,6 +236,9 @@ GWB_API int gwb_sigma2(const float* H, long long ldh, int n, const float* IP, lo
 GWB_API int gwb_sigma2_band(const float* H, long long ldh, int n, const int32_t* kmax, const float* IP, long long ldip,
                             int nseg, int kmin, int flen, double df, double* part, long long part_elems, double* sig,
                             long long ldsig, void* stream);
+/* ends[i] = one past the last bin of row i (flen complex values) that is not zero, 0 for a row of zeros: gwb_sigma2_band's
+ * kmax from the templates themselves. */
+GWB_API int gwb_row_ends(const float* H, long long ldh, int n, int flen, int32_t* ends, void* stream);
 /* Template norms as gwb_sigma2, for callers that must not allocate device memory: no counterpart in the reference.
  * Some callers cannot let a library call cudaMalloc: a host program (for example a Go or Java service over the C ABI)
  * whose own pool owns every byte of device memory, code that runs between stream-capture begin and end, where an
