@@ -122,7 +122,7 @@ class MatchedFilter:
             bt = self.tuning['basis']['best'] if self.tuning and self.tuning['basis'] else {}
             self.fws = fp_filter.FusedBasisWorkspace(tlen, bank.flen, rmax, device, wrows=bt.get('wrows'),
                                                      ring=bt.get('ring'))
-            # basis filters in the four-step order of the transform, once per tile; D isw per step (self.Dp)
+            # basis filters in the four-step order of the transform, once per tile; D isw per step (order_data)
             # and, read from the filters themselves, the bin from which each tile's are zero (its last f_ISCO)
             ends = torch.empty(len(bank.svd), dtype=torch.int32, device=device)
             self.vp = [fp_filter.fourstep_order(s['Vh'], tlen, last_nz=ends[t:t + 1]) for t, s in enumerate(bank.svd)]
@@ -131,8 +131,8 @@ class MatchedFilter:
             self.ends = fp_filter.row_ends(bank.H)
             for r0, ids in zip(bank.row0, bank.tiles):
                 self.ends[r0:r0 + len(ids)] = self.ends[r0:r0 + len(ids)].max()
-            self.last_bad = None
-            self.Dp = None
+            self._Dp = self._last_bad = None
+            self._paired = False                # _last_bad is of the data in _Dp
         else:
             self.ws = fp_filter.BasisWorkspace(tlen, bank.flen, fp_filter.RB, device)
         assert self.fused or not self.fp8, 'the fp8 form needs the fused basis series (tlen in [2^12, 2^20])'
@@ -234,6 +234,29 @@ class MatchedFilter:
                 for a, b in spans:
                     Zp[a:b].zero_()
 
+    def order_data(self, D, isw):
+        """D isw of every segment in four-step order, shared by all tiles, with each segment's last bin that is not
+        finite: what tile_segment's basis series reads on the fused path."""
+        S = D.shape[0]
+        if self._Dp is None or self._Dp.shape[0] != S:
+            self._Dp = torch.empty((S, self.tlen // 2 + 1), dtype=torch.complex64, device=D.device)
+        if self._last_bad is None or self._last_bad.shape[0] != S:
+            self._last_bad = torch.empty(S, dtype=torch.int32, device=D.device)
+        fp_filter.fourstep_order(D, self.tlen, isw, out=self._Dp, last_bad=self._last_bad)
+        self._paired = True
+        self.kernel_launches += 1
+
+    @property
+    def Dp(self):
+        """The ordered data. Whoever takes or sets it may change what it holds, so the first pass then goes over the full
+        band until order_data writes the data and its last bad bins together again."""
+        self._paired = False
+        return self._Dp
+
+    @Dp.setter
+    def Dp(self, Dp):
+        self._Dp, self._paired = Dp, False
+
     def tile_segment(self, t, D, isw, sig, seg):
         """Basis series, stacked A, fused GEMM and window selection of tile t against segment seg (row of D)."""
         b = self.bank
@@ -248,9 +271,9 @@ class MatchedFilter:
             e[0].record()
         im_off = Kh if self.compact else r
         if self.fused:
-            scale = fp_filter.basis_series_fused(self.fws, self.vp[t], self.Dp[seg], self.a0, self.Tn, self.Z,
-                                                 self.Zlo, self.form, im_off=im_off, kend=self.kend[t],
-                                                 last_bad=None if self.last_bad is None else self.last_bad[seg:seg + 1])
+            band = dict(kend=self.kend[t], last_bad=self._last_bad[seg:seg + 1]) if self._paired else {}
+            scale = fp_filter.basis_series_fused(self.fws, self.vp[t], self._Dp[seg], self.a0, self.Tn, self.Z,
+                                                 self.Zlo, self.form, im_off=im_off, **band)
         else:
             scale = fp_filter.basis_series_into(self.ws, sv['Vh'], D[seg], isw, self.a0, self.Tn, self.Z,
                                                 self.Zlo, self.form, im_off=im_off)
@@ -366,12 +389,7 @@ class MatchedFilter:
             e_f = (ev(), ev())
             e_f[0].record()
         if self.fused:
-            # every segment's D isw in four-step order, shared by all tiles
-            if self.Dp is None or self.Dp.shape[0] != D.shape[0]:
-                self.Dp = torch.empty((D.shape[0], self.tlen // 2 + 1), dtype=torch.complex64, device=D.device)
-                self.last_bad = torch.empty(D.shape[0], dtype=torch.int32, device=D.device)
-            fp_filter.fourstep_order(D, self.tlen, isw, out=self.Dp, last_bad=self.last_bad)
-            self.kernel_launches += 1
+            self.order_data(D, isw)
         if prof is not None:
             e_f[1].record()
             prof.setdefault('parts', []).append(('fourstep', e_f))

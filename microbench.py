@@ -377,7 +377,7 @@ def form_window_snr(mf, t, D, isw, sig, seg):
     """Window maxima of the SNR (n, nw) and their samples from the fused GEMM of mf's form, for tile t against
     segment seg (rows of D). Resets mf's candidate counters (the diagnostic call's candidates are not kept)."""
     if mf.fused:
-        mf.Dp = fp_filter.fourstep_order(D, mf.tlen, isw)
+        mf.order_data(D, isw)
     mf.counters.zero_()
     mf.tile_segment(t, D, isw, sig, seg)
     torch.cuda.synchronize()
