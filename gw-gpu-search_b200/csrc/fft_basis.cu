@@ -545,9 +545,15 @@ __global__ void rowscale_kernel(const float* __restrict__ rowpart, int P, float*
     }
 }
 
-// FORM 5 of the pass-2 kernels stores nothing and sums |z|^2 over the analysed samples (unscaled): one double per CTA,
-// added up in a fixed order by power_scale_kernel. The reference's scale is that rms over its first batch of rows.
+// FORM 5 of the pass-2 kernels stores nothing and sums |z|^2 over the analysed samples (unscaled), in float64 from the
+// squares on as gwb_basis_scale does (the conversions, 16 a clock and SM, make it 25 us of a call of 100 rows of 2^20 against
+// float32 partial sums, whose squares leave float32's range where the samples are below 1e-19 or above 1e19): one double
+// per CTA, added up in a fixed order by power_scale_kernel. The reference's scale is that rms over its first batch of rows.
 constexpr int kPower = 5;
+__device__ __forceinline__ double add_power(float2 z, double s) {
+    const double x = z.x, y = z.y;
+    return fma(x, x, fma(y, y, s));
+}
 template <int NT>
 __device__ __forceinline__ void power_partial(double acc, double* __restrict__ partials) {
     __shared__ double red[NT / 32];
@@ -619,7 +625,7 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT) basis_pass2(
     const int row = blockIdx.y, t10 = blockIdx.x * TB, tid = threadIdx.x;
     const int stride = N / N2;
     const float inv = FORM == kPower ? 1.0f : 1.0f / (FORM == 4 ? scale[row] : *scale);
-    float power = 0.f;
+    double power = 0.0;
     const float tsc = kFold<N2, FORM> ? inv : 1.f, zsc = kFold<N2, FORM> ? 1.f : inv;
     for (int m = tid; m < N2; m += NT) {
         const float2 w = tw[m * stride];
@@ -660,13 +666,13 @@ __global__ void __launch_bounds__(Split<N2, 2>::NT) basis_pass2(
             const int t = t0 + N1 * (R1 * vv);
             if (t >= 0 && t < Tn) {
                 const float2 z = y[brev(vv, ilog2(R2))];
-                if constexpr (FORM == kPower) power = fmaf(z.x, z.x, fmaf(z.y, z.y, power));
+                if constexpr (FORM == kPower) power = add_power(z, power);
                 else if constexpr (!kFold<N2, FORM>) store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x * zsc, z.y * zsc);
                 else store_z<FORM>(Zr, Zi, Zlr, Zli, t, z.x, z.y);
             }
         });
     }
-    if constexpr (FORM == kPower) power_partial<NT>((double)power, partials);
+    if constexpr (FORM == kPower) power_partial<NT>(power, partials);
 }
 
 // pass 2 over row chunks: CTA = (TB consecutive t1, RC consecutive rows). One shared buffer holds the W tile of a row
@@ -901,13 +907,13 @@ __global__ void __launch_bounds__(SplitW<N2>::NT, 1) basis_pass2_w(
                 ps.template store<K>(z.x * inv, z.y * inv, ph, pl, (vmask >> vv) & 1u);
             });
         } else if constexpr (FORM == kPower) {
-            float pj = 0.f;
+            double pj = 0.0;                     // a chain per row
             static_for<R2>([&](auto V) {
                 constexpr int vv = decltype(V)::value;
                 const float2 z = y[brev(vv, ilog2(R2))];
-                if ((vmask >> vv) & 1u) pj = fmaf(z.x, z.x, fmaf(z.y, z.y, pj));
+                if ((vmask >> vv) & 1u) pj = add_power(z, pj);
             });
-            power += (double)pj;
+            power += pj;
         } else {
             const long long re_off = (long long)(row0 + j) * ldz * ES, im_off_b = (long long)(im_off + row0 + j) * ldz * ES;
             void* Zr = zb + re_off;

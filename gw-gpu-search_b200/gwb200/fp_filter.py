@@ -243,7 +243,7 @@ class BasisWorkspace:
 class SeriesWorkspace:
     """Device buffers of the reference's basis series through the fused passes (gwb_basis_series, power-of-two tlen in
     [FUSED_MIN, FUSED_MAX]): a batch of basis filters and the data in four-step order, and the batch's transform between
-    the passes. 100 rows of 2^20, fp16 Z: 1,517 us a call through premul, cuFFT and pack, 958 so."""
+    the passes. 100 rows of 2^20, fp16 Z: 1,531 us a call through premul, cuFFT and pack, 991 so."""
 
     def __init__(self, tlen, flen, rows=RB, device='cuda'):
         self.tlen, self.flen, self.rows = tlen, flen, rows
