@@ -173,40 +173,46 @@ __device__ __forceinline__ int kmax_of(double Ms, double df, int flen) {
 
 // ---- SNR and its gradient ----
 // In f alone the phase is linear in ten functions of frequency, whose coefficients hold all of theta: with u = f^(1/3),
-//   Psi(f) = sum_m C_m(theta) phi_m(f),  phi = u^-5, u^-3, u^-2, u^-1, 1, log f, u, u log f, u^2, u^(-34/3).
+//   Psi(f) = sum_m C_m(theta) phi_m(f),  phi = u^-5, u^-3, u^-2, u^-1, 1, l, u, u l, u^2, u^(-34/3),  l = log(f / kF0).
 // So dPsi/dtheta_p = sum_m dC_m/dtheta_p phi_m, and the sums over bins that the gradient needs are the moments
 // M_m = sum_k q_k phi_m(f_k), one per function (and one of f for t_c), contracted with dC_m/dtheta_p once per
-// chi-squared bin instead of a dual-number phase per (bin, parameter). All phi are products of w = f^(-1/18).
+// chi-squared bin instead of a dual-number phase per (bin, parameter).
+// Errors: every power is within a few roundings of its value, since each one is multiplied by up to 1e4 rad. A power taken
+// as exp(x log a) carries the error of x log a, and a product of n equal factors n times the factor's, so the coefficients
+// come from pi Ms and its cube root and the float64 form's phi from f, 1 / f and f^(-1/3) (u^-5 = f^-1 f^(-2/3)). Largest /
+// rms error of Psi against 64-bit mantissas, 20 to 1,024 Hz, 150 triggers, rad: Mc = 1.2 9.7e-12 / 3.1e-13, 5 1.0e-12 /
+// 4.5e-14, 25 7.9e-14 / 1.7e-14 (exponentials of the logarithm per term, as psi_at: 5.7e-11 / 1.7e-12, 4.1e-12 / 2.1e-13,
+// 1.8e-13 / 2.3e-14; products of w = f^(-1/18): 9.7e-11 / 2.9e-12, 7.5e-12 / 4.0e-13, 4.1e-13 / 4.6e-14). The float32
+// form rounds the reduced phase to 24 bits and keeps the products of w, which cost it no division or root per bin. l is
+// centred so that the constant and the logarithmic terms, which cancel, stay small.
 constexpr int kNF = 10;                  // phase functions
 constexpr int kNM = kNF + 1;             // moments: the phase functions, then f
 constexpr int kOne = 4;                  // phi = 1: the moment is the bin's z
 constexpr int kGT = 256;                 // threads per trigger of snr_grad_kernel
 constexpr int kWarps = kGT / 32;
-constexpr int kTab = 6016;               // bins from kmin on whose log f and w a CTA keeps for all its triggers (94 KB)
+constexpr int kTab = 6016;               // bins from kmin on whose l and root of f a CTA keeps for all its triggers (94 KB)
+constexpr double kF0 = 128.0;            // a power of two: f / kF0 and kF0 pi Ms are exact
 
-// C_m and its derivatives for m = lane: pre times a^x times a polynomial in (eta, chi), with every power of pi Ms (and the
-// eccentric term's v0^(19/3)) in one exponential whose exponent is the lane's own; only logarithms of Mc, eta and f_ecc
-// come before it, side by side. (Through pow by pow, the CTA waited for this chain longer than for the sums over bins.)
-__device__ __forceinline__ Dual phase_function_coef(const double* th, double f_ecc, int m) {
+// C_m and its derivatives for m = lane: pre times a^x times a polynomial in (eta, chi), a = (pi Ms)^(1/3), so that
+// a^-5 = 1 / (pi Ms a^2), and one division gives every lane its power. The eccentric term's a^(-34/3) v0^(19/3) is
+// (pi Ms)^(-34/9 + 19/9) f_ecc^(19/9) = a^-5 ecc0. Ms: the trigger's (its pow is shared with the band's end).
+__device__ __forceinline__ Dual phase_function_coef(const double* th, double Ms, double ecc0, int m) {
     Dual q = dc(th[1]), c1 = dc(th[2]), c2 = dc(th[3]);
     q.d[1] = 1.0;
     c1.d[2] = 1.0;
     c2.d[3] = 1.0;
     const Dual one_q = 1.0 + q, iq = dc(1.0) / one_q, qi = q * iq;
     const Dual eta = qi * iq;
-    // log(pi Ms) = log(pi Msun) + log Mc - 0.6 log eta
     const double ieta = 1.0 / eta.v;
-    Dual lms = dc(log(kPi * kMsun) + log(th[0]) - 0.6 * log(eta.v));
-    lms.d[0] = 1.0 / th[0];
-    lms.d[1] = -0.6 * ieta * eta.d[1];
-    const Dual la = (1.0 / 3.0) * lms;                                // log a, v = a u
-    // a^x; the eccentric term's a^(-34/3) v0^(19/3) is (pi Ms)^(-34/9 + 19/9) f_ecc^(19/9)
-    const double expo[kNF] = {-5.0, -3.0, -2.0, -1.0, 0.0, 0.0, 1.0, 1.0, 2.0, -5.0};
-    double ex = 0.0;
-#pragma unroll
-    for (int i = 0; i < kNF; ++i) ex = m == i ? expo[i] : ex;
+    const double X = kPi * Ms, a = cbrt(X), a2 = a * a;
+    Dual la = dc((1.0 / 3.0) * log(kF0 * X));                         // log(a kF0^(1/3)), v = a u
+    la.d[0] = 1.0 / (3.0 * th[0]);
+    la.d[1] = -0.2 * ieta * eta.d[1];
+    const double num = m == 9 ? ecc0 : m == 8 ? a2 : m >= 6 ? a : 1.0;
+    const double den = m == 0 || m == 9 ? X * a2 : m == 1 ? X : m == 2 ? a2 : m == 3 ? a : 1.0;
+    const double ex = m == 0 || m == 9 ? -5.0 : m == 1 ? -3.0 : m == 2 ? -2.0 : m == 3 ? -1.0 : m == 8 ? 2.0 : m >= 6 ? 1.0 : 0.0;
     Dual pw;
-    pw.v = exp(ex * la.v + (m == kNF - 1 ? 19.0 / 9.0 * log(f_ecc) : 0.0));
+    pw.v = num / den;
 #pragma unroll
     for (int i = 0; i < kNI; ++i) pw.d[i] = pw.v * ex * la.d[i];
     const Dual e2 = eta * eta;
@@ -241,28 +247,54 @@ __device__ __forceinline__ Dual phase_function_coef(const double* th, double f_e
     return pre * pw * c;
 }
 
-// f^(-1/18) from log f; w^42 = f^(-7/3)
-__device__ __forceinline__ double root18(double lf) { return exp(lf * (-1.0 / 18.0)); }
-__device__ __forceinline__ double w_to_73(double w) {
-    const double w3 = w * w * w, iu = w3 * w3, iu3 = iu * iu * iu;
-    return iu3 * iu3 * iu;
+// What a CTA keeps per bin: l = log(f / kF0) and a root of f, f^(-1/3) for the float64 form, w = f^(-1/18) for the float32
+// form.
+template <typename T>
+__device__ __forceinline__ double2 log_root(double f) {
+    const double l = log(f * (1.0 / kF0));
+    if constexpr (sizeof(T) == 8) return make_double2(l, rcbrt(f));
+    else return make_double2(l, exp((l + 4.852030263919617) * (-1.0 / 18.0)));        // + log kF0
 }
-
+template <typename T>
 __device__ __forceinline__ double2 log_root(const double2* tab, int kmin, int k, double df) {
-    if (k - kmin < kTab) return tab[k - kmin];
-    const double lf = log((double)k * df);
-    return make_double2(lf, root18(lf));
+    return k - kmin < kTab ? tab[k - kmin] : log_root<T>((double)k * df);
+}
+// 1 / f from iu = f^(-1/3): the cube's relative error (8 roundings) squared by one Newton step
+__device__ __forceinline__ double inverse(double f, double iu) {
+    const double r = iu * iu * iu;
+    return fma(r, fma(-f, r, 1.0), r);
+}
+// f^(-1/N) from a float32 estimate y0 (good to 1e-6): with y0^N f = 1 - d, y0 (1 - d)^(-1/N) by its binomial series
+template <int N>
+__device__ __forceinline__ double minus_root(double f, double y0) {
+    const double y2 = y0 * y0, y4 = y2 * y2, yn = N == 6 ? y4 * y2 : N == 9 ? y4 * y4 * y0 : 0.0;
+    static_assert(N == 6 || N == 9, "powers written out");
+    const double d = fma(-yn, f, 1.0);
+    return fma(y0 * d, fma(d, (N + 1) / (2.0 * N * N), 1.0 / N), y0);
+}
+// f^(-7/3)
+template <typename T>
+__device__ __forceinline__ double root_to_73(double root, double f) {
+    if constexpr (sizeof(T) == 8) {
+        const double r = inverse(f, root);
+        return root * r * r;
+    }
+    const double w3 = root * root * root, iu = w3 * w3, iu3 = iu * iu * iu;
+    return iu3 * iu3 * iu;
 }
 
 // Equal-power edges of w_k = f^-7/3 IP_k over [kmin, k1): edge j = first k whose inclusive cumulative sum exceeds
 // (j / nb) total (the pipeline's edges, offset mode 0). Threads take contiguous ranges; float64 sums, warp and block
 // scans, and one walk per thread over its range that sets the edges inside it.
+template <typename T>
 __device__ void block_edges(const float* __restrict__ ip, double df, int kmin, int k1, int nb, int* e, double* tot_out,
                             double* scan, const double2* tab) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int len = k1 - kmin, chunk = (len + kGT - 1) / kGT;
     const int a = min(kmin + tid * chunk, k1), b = min(a + chunk, k1);
-    auto weight = [&](int k) { return w_to_73(log_root(tab, kmin, k, df).y) * (double)ip[k]; };
+    auto weight = [&](int k) {
+        return root_to_73<T>(log_root<T>(tab, kmin, k, df).y, (double)k * df) * (double)ip[k];
+    };
     double s = 0.0;
 #pragma unroll 4
     for (int k = a; k < b; ++k) s += weight(k);
@@ -310,15 +342,17 @@ __device__ void block_edges(const float* __restrict__ ip, double df, int kmin, i
 // out row layout (doubles): snr, newsnr, chisq, sigma2, z_re, z_im, kmax, dsnr[7], dnewsnr[7], dchisq[7]
 constexpr int kOut = 7 + 3 * kNP;
 
-// CTAs of eight warps, two per SM, stay for all their triggers (blockIdx.x, + gridDim.x, ...), so that log f and
-// f^(-1/18) of the first kTab bins are computed once per CTA, as far as the longest band of its triggers. Per trigger, the
+// CTAs of eight warps, two per SM, stay for all their triggers (blockIdx.x, + gridDim.x, ...), so that log_root of the
+// first kTab bins is computed once per CTA, as far as the longest band of its triggers. Per trigger, the
 // band is cut into one contiguous run per warp; a lane's bins are 32 apart (coalesced D and IP), and at every chi-squared
 // edge the warp adds its 22 sums over the lanes (a halving exchange: 31 shuffles of a double, against 110 for 22 trees)
 // and stores them with the edge bin they belong to. Bound: the chain of a trigger (coefficients, edges, runs, final sums)
 // with two of them per SM, and the float64 pipe. The former kernel took a barrier and a block reduction per chi-squared
 // bin, in which 256 threads share the 20 to 200 bins of 16 s of data, and a dual-number phase with three exp and two pow
 // per frequency bin: 803 us for 2,048 triggers of 16 s, float32, now 159. (A CTA per trigger without the table 194, four
-// warps per trigger and four CTAs per SM 192, a warp per trigger 291: it waits for the longest band.)
+// warps per trigger and four CTAs per SM 192, a warp per trigger 291: it waits for the longest band.) The float64 form's
+// more exact powers cost it 5%: 333 us a call for 2,048 triggers of 16 s, Mc 4 to 34, 316 with products of w and 1,372 with
+// the former kernel (float32 form 303, 304 and 1,320); divided and rooted by the library functions it took 385.
 template <typename T>
 __global__ void __launch_bounds__(kGT, 2) snr_grad_kernel(const double* __restrict__ params, int n,
                                                              const float2* __restrict__ D, long long ldd,
@@ -345,16 +379,15 @@ __global__ void __launch_bounds__(kGT, 2) snr_grad_kernel(const double* __restri
         atomicMax(&s_top, kmax_of(kMsun * (th[0] * pow(eta, -0.6)), df, flen));
     }
     __syncthreads();
-    for (int k = tid; k < min(kTab, s_top - kmin); k += kGT) {
-        const double lf = log((double)(kmin + k) * df);
-        tab[k] = make_double2(lf, root18(lf));
-    }
+    for (int k = tid; k < min(kTab, s_top - kmin); k += kGT) tab[k] = log_root<T>((double)(kmin + k) * df);
+    const double ecc0 = f_ecc * f_ecc * pow(f_ecc, 1.0 / 9.0);
     __syncthreads();
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         const double* th = params + (long long)i * kNP;
         // the end bin from the same operations as phase_coef's value of Ms
         const double q1 = 1.0 + th[1], eta = th[1] / (q1 * q1);
-        const int k1 = kmax_of(kMsun * (th[0] * pow(eta, -0.6)), df, flen);
+        const double Ms = kMsun * (th[0] * pow(eta, -0.6));
+        const int k1 = kmax_of(Ms, df, flen);
         if (k1 <= kmin + 256) {           // no band above kmin (f_ISCO below the low cut): nothing to filter
             if (tid < kOut) out[(long long)i * ldout + tid] = 0.0;
             continue;
@@ -363,14 +396,14 @@ __global__ void __launch_bounds__(kGT, 2) snr_grad_kernel(const double* __restri
         const float2* d = D + (long long)i * ldd;
         if (tid < kSeg) owner[tid] = -1;
         if (warp == kWarps - 1) {
-            const Dual c = phase_function_coef(th, f_ecc, min(lane, kNF - 1));
+            const Dual c = phase_function_coef(th, Ms, ecc0, min(lane, kNF - 1));
             if (lane < kNF) {
                 C[lane][0] = c.v;
 #pragma unroll
                 for (int p = 0; p < kNI; ++p) C[lane][1 + p] = c.d[p];
             }
         }
-        block_edges(ip, df, kmin, k1, nb, e, &tot, scan, tab);   // ends with a barrier
+        block_edges<T>(ip, df, kmin, k1, nb, e, &tot, scan, tab);   // ends with a barrier
         {
             double cv[kNF];
 #pragma unroll
@@ -390,11 +423,28 @@ __global__ void __launch_bounds__(kGT, 2) snr_grad_kernel(const double* __restri
                     const float2 dk = dn;
                     if (k + 32 < hi) dn = d[k + 32];
                     const double f = (double)k * df;
-                    const double2 t = log_root(tab, kmin, k, df);
-                    const double lf = t.x, w = t.y;
-                    const double w2 = w * w, w3 = w2 * w, iu = w3 * w3, iu2 = iu * iu, iu3 = iu2 * iu, iu5 = iu3 * iu2;
+                    const double2 t = log_root<T>(tab, kmin, k, df);
+                    const double lf = t.x;
+                    double iu, iu2, i3, i5, i34, amp64;                      // u^-1, u^-2, u^-3, u^-5, u^(-34/3), f^(-7/6)
+                    if constexpr (sizeof(T) == 8) {
+                        iu = t.y;
+                        iu2 = iu * iu;
+                        i3 = inverse(f, iu);
+                        i5 = iu2 * i3;
+                        const float lg = log2f((float)f);
+                        i34 = i5 * (i3 * i3) * minus_root<9>(f, exp2f(lg * (-1.f / 9.f)));
+                        amp64 = i3 * minus_root<6>(f, exp2f(lg * (-1.f / 6.f)));
+                    } else {
+                        const double w = t.y, w2 = w * w, w3 = w2 * w;
+                        iu = w3 * w3;
+                        iu2 = iu * iu;
+                        i3 = iu2 * iu;
+                        i5 = i3 * iu2;
+                        i34 = i5 * i5 * iu * w2;
+                        amp64 = i3 * w3;
+                    }
                     const double u = f * iu2;
-                    const double phi[kNM] = {iu5, iu3, iu2, iu, 1.0, lf, u, u * lf, f * iu, iu5 * iu5 * iu * w2, f};
+                    const double phi[kNM] = {i5, i3, iu2, iu, 1.0, lf, u, u * lf, f * iu, i34, f};
                     double ph = cv[kOne], ph2 = wtc * f;                     // two chains
 #pragma unroll
                     for (int m = 0; m < kNF; ++m) {
@@ -409,7 +459,7 @@ __global__ void __launch_bounds__(kGT, 2) snr_grad_kernel(const double* __restri
                     } else {
                         sincosf((float)ph, &sn, &cs);
                     }
-                    const T amp = (T)(iu3 * w3);                             // f^(-7/6)
+                    const T amp = (T)amp64;
                     // q = conj(h) D = amp e^{+i ph} D
                     const T hr = amp * cs, hi2 = amp * sn;
                     const double qr = (double)(hr * (T)dk.x - hi2 * (T)dk.y);
