@@ -170,9 +170,9 @@ def fourstep_order(X, N, isw=None, out=None, last_nz=None, last_bad=None):
 
 
 RING_N = 1 << 20   # the transform length of the persistent ring form (gwb_basis_fused_ring)
-# rows of W by default at 2^20, where the default was once the ring's few: 2.1 GB at most, and no slower than W for all rows
-# (128 rows in batches of 64 take 5.8 us each against 5.2 in one)
-W_ROWS = 256
+# rows of W by default at 2^20, where the default was once the ring's few: 5.4 GB at most, and no batches up
+# to the GEMM's widest forms (they cost 2 to 7%: 512 rows 5.30 us each, in batches of 256 5.47, of 128 5.68)
+W_ROWS = 640
 
 
 class FusedBasisWorkspace:

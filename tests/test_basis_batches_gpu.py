@@ -6,7 +6,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize('rows', [1, 2, 300])
+@pytest.mark.parametrize('rows', [1, 2, 700])
 def test_default_workspace(rows):
     from gwb200 import fp_filter
     N = 1 << 20
@@ -18,7 +18,7 @@ def test_default_workspace(rows):
     for kw in ({}, dict(wrows=rows), dict(ring=True)):
         ws = fp_filter.FusedBasisWorkspace(N, N // 2 + 1, rows, **kw)
         if not kw:
-            assert ws.W.shape[0] == min(rows, 256)
+            assert ws.W.shape[0] == min(rows, 640)
         Z = torch.zeros((2 * rows, Tn), dtype=torch.float16, device='cuda')
         s = fp_filter.basis_series_fused(ws, Vp, Dp, a0, Tn, Z, form='f16')
         out.append((Z, s.clone()))
