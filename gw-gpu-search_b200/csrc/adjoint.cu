@@ -179,12 +179,13 @@ __device__ __forceinline__ int kmax_of(double Ms, double df, int flen) {
 // chi-squared bin instead of a dual-number phase per (bin, parameter).
 // Errors: every power is within a few roundings of its value, since each one is multiplied by up to 1e4 rad. A power taken
 // as exp(x log a) carries the error of x log a, and a product of n equal factors n times the factor's, so the coefficients
-// come from pi Ms and its cube root and the float64 form's phi from f, 1 / f and f^(-1/3) (u^-5 = f^-1 f^(-2/3)). Largest /
-// rms error of Psi against 64-bit mantissas, 20 to 1,024 Hz, 150 triggers, rad: Mc = 1.2 9.7e-12 / 3.1e-13, 5 1.0e-12 /
-// 4.5e-14, 25 7.9e-14 / 1.7e-14 (exponentials of the logarithm per term, as psi_at: 5.7e-11 / 1.7e-12, 4.1e-12 / 2.1e-13,
-// 1.8e-13 / 2.3e-14; products of w = f^(-1/18): 9.7e-11 / 2.9e-12, 7.5e-12 / 4.0e-13, 4.1e-13 / 4.6e-14). The float32
-// form rounds the reduced phase to 24 bits and keeps the products of w, which cost it no division or root per bin. l is
-// centred so that the constant and the logarithmic terms, which cancel, stay small.
+// come from pi Ms and its cube root and the float64 form's phi from f, 1 / f and f^(-1/3) (u^-5 = f^-1 f^(-2/3)). Error of
+// Psi against 80-bit arithmetic, 4,096 (trigger, bin) pairs from 20 Hz on, largest / rms in rad: Mc = 1.2 1.1e-11 /
+// 1.9e-12, 5 1.4e-12 / 1.8e-13, 25 6.6e-14 / 1.8e-14 (an exponential of the logarithm per term, as psi_at: 3.5e-11 /
+// 7.5e-12, 3.3e-12 / 6.5e-13, 1.9e-13 / 3.4e-14; products of w = f^(-1/18): 6.4e-11 / 1.2e-11, 5.2e-12 / 9.2e-13, 3.3e-13 /
+// 5.3e-14); amplitude 3.3 / 0.8 units of 2^-53 (6.8 / 3.6; 36 / 9.6). The float32 form rounds the reduced phase to 24 bits
+// and keeps the products of w, which cost it no root per bin. l is centred so that the constant and the logarithmic terms,
+// which cancel, stay small.
 constexpr int kNF = 10;                  // phase functions
 constexpr int kNM = kNF + 1;             // moments: the phase functions, then f
 constexpr int kOne = 4;                  // phi = 1: the moment is the bin's z
