@@ -1533,6 +1533,15 @@ int gwb_basis_set_pass2_pairs(int on) {
     return GWB_OK;
 }
 
+int gwb_basis_ring_get_config(int* pc, int* nslot, int* look) {
+    using namespace gwb;
+    GWB_CHECK_ARG(pc && nslot && look, GWB_ERR_ARG, "basis_ring_get_config: null pointer");
+    *pc = g_ring_pc.load();
+    *nslot = g_ring_nslot.load();
+    *look = g_ring_look.load();
+    return GWB_OK;
+}
+
 int gwb_basis_ring_rows(void) { return gwb::g_ring_pc.load() * gwb::g_ring_nslot.load(); }
 
 int gwb_basis_ring_sync_ints(int rows) {

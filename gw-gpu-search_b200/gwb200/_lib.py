@@ -59,6 +59,7 @@ SIGNATURES = {
                              _LL, _P, _LL, _P],
     'gwb_basis_series': [_P, _LL, _I, _P, _P, _LL, _LL, _P, _P, _P, _P, _I, _LL, _LL, _I, _P, _P, _LL, _I, _P, _LL, _P, _P],
     'gwb_basis_ring_set_config': [_I, _I, _I],
+    'gwb_basis_ring_get_config': [_P, _P, _P],
     'gwb_basis_ring_rows': [],
     'gwb_basis_set_pass2_columns': [_I, _I],
     'gwb_basis_pass2_columns': [_I],

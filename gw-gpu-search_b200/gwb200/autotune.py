@@ -11,14 +11,17 @@ MatchedFilter of the same shapes reuses it without timing. The candidates comput
 of the fp32 accumulation differs between MMA orders (identical V and I where the sums are exact, as in the tests;
 otherwise the last bits of V and, at near-ties, I), so tuning changes speed, not precision.
 """
+import ctypes
+
 import torch
 
 from . import _lib, fp_filter
 
 FORM_CODE = {'f16': 0, 'bf16': 1, 'bf16x3': 2, 'fp8': 3, 'f16x2': 6}
 # the persistent basis series' (rows per chunk, W slots, lookahead): W in L2 holds rows x slots rows of 8 MB at 2^20
-# (lookahead 0: split roles, half the CTAs on each pass)
-RING_CONFIGS = [(2, 3, 1), (2, 4, 2), (4, 2, 1), (2, 3, 0), (2, 2, 0), (4, 2, 0), (1, 4, 0)]
+# (lookahead 0: split roles, half the CTAs on each pass). The scale comes from the first chunk, so all have the default's
+# two rows: the choice then leaves Z as it is
+RING_CONFIGS = [(2, 3, 1), (2, 4, 2), (2, 3, 0), (2, 2, 0)]
 _CACHE = {}
 
 
@@ -93,11 +96,14 @@ def tune_gemm(form, n, Kh, Tn, group=16, reps=3, device='cuda'):
     return best, res
 
 
-def tune_basis(tlen, r, form='f16', reps=2, device='cuda'):
+def tune_basis(tlen, r, form='f16', reps=2, device='cuda', kend=None):
     """Times the basis-series forms for r rows of length tlen: the ring (tlen = 2^20, RING_CONFIGS) and two passes with
     W for all rows or in batches of 32, with 8 or 16 columns per pass-2 CTA (16 at tlen = 2^20 only); sets the fastest
-    and returns (best: dict(ring, wrows, ring_config, pass2_cols), {candidate: ms})."""
-    key = (torch.cuda.get_device_name(device), 'basis', int(tlen), int(r), form)
+    and returns (best: dict(ring, wrows, ring_config, pass2_cols), {candidate: ms}). kend: the filters are zero from this
+    bin on, as the run's are (the two-pass form stops there, the ring does not). ring is True or None, so that a workspace
+    made from the choice gives the default's Z whichever form it is. The ring configuration, which is process-wide, stays
+    as it was unless a ring is chosen."""
+    key = (torch.cuda.get_device_name(device), 'basis', int(tlen), int(r), form, kend)
     if key in _CACHE:
         out = _CACHE[key]
         _apply_basis(out[0], form)
@@ -107,25 +113,33 @@ def tune_basis(tlen, r, form='f16', reps=2, device='cuda'):
     Vh = torch.randn((r, flen), generator=g, device=device, dtype=torch.complex64)
     D = torch.randn(flen, generator=g, device=device, dtype=torch.complex64)
     isw = torch.rand(flen, generator=g, device=device) + 0.5
+    kend = flen if kend is None else min(int(kend), flen)
+    Vh[:, kend:] = 0
     a0, Tn = tlen * 3 // 32, tlen * 28 // 32
     Kh = fp_filter.kh_of(r, form)
     Z = torch.zeros((2 * Kh, -(-Tn // 16) * 16), dtype=fp_filter._z_dtype(form), device=device)
     Zlo = torch.zeros_like(Z) if form == 'bf16x3' else None
     Vp = fp_filter.fourstep_order(Vh, tlen)
-    Dp = fp_filter.fourstep_order(D, tlen, isw)
-    cands = [(False, None, None, 16), (False, 32, None, 16)]
+    bad = torch.empty(1, dtype=torch.int32, device=device)
+    Dp = fp_filter.fourstep_order(D, tlen, isw, last_bad=bad)
+    cands = [(None, None, None, 16), (None, 32, None, 16)]
     if tlen == fp_filter.RING_N:
         cands = ([(True, None, rc, 16) for rc in RING_CONFIGS] + cands +
-                 [(False, None, None, 8), (False, 32, None, 8)])
+                 [(None, None, None, 8), (None, 32, None, 8)])
     res, best = {}, None
+    was = (ctypes.c_int * 3)()
+    _lib.call('gwb_basis_ring_get_config', *(ctypes.byref(was, 4 * i) for i in range(3)))
     for ring, wrows, rc, cols in cands:
         _apply_basis(dict(ring_config=rc, pass2_cols=cols), form)
         ws = fp_filter.FusedBasisWorkspace(tlen, flen, r, device=device, wrows=wrows, ring=ring)
-        ms = _events_ms(lambda: fp_filter.basis_series_fused(ws, Vp, Dp, a0, Tn, Z, Zlo, form, im_off=Kh), reps)
+        ms = _events_ms(lambda: fp_filter.basis_series_fused(ws, Vp, Dp, a0, Tn, Z, Zlo, form, im_off=Kh, kend=kend,
+                                                             last_bad=bad), reps)
         res[(ring, wrows, rc, cols)] = ms
         if best is None or ms < res[best]:
             best = (ring, wrows, rc, cols)
         del ws
+    if not best[0]:
+        _lib.call('gwb_basis_ring_set_config', *was)
     out = (dict(ring=best[0], wrows=best[1], ring_config=best[2], pass2_cols=best[3]), res)
     _apply_basis(out[0], form)
     _CACHE[key] = out
@@ -150,7 +164,8 @@ def tune_filter(bank, tlen, Tn, form, group, device='cuda'):
             best, res = tune_gemm(form, nmax, kh, Tn, group, device=device)
             rep['gemm'][kh] = dict(best=best, ms={str(k): v for k, v in res.items()})
     if fp_filter.FUSED_MIN <= tlen <= fp_filter.FUSED_MAX:
-        rmax = max(s['r'] for s in bank.svd)
-        best, res = tune_basis(tlen, rmax, form, device=device)
+        wide = max(bank.svd, key=lambda s: s['r'])
+        kend = int(fp_filter.row_ends(wide['Vh']).max())
+        best, res = tune_basis(tlen, wide['r'], form, device=device, kend=kend)
         rep['basis'] = dict(best=best, ms={str(k): v for k, v in res.items()})
     return rep

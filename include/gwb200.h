@@ -368,6 +368,8 @@ GWB_API int gwb_basis_series(const float* Vh, long long ldv, int rows, const flo
  * gwb_basis_ring_set_config sets (pc in 1..4, nslot > look, look >= 0; 0 splits the grid into pass-1 and pass-2
  * CTAs) process-wide (default 2, 3, 1; the autotuner times the choices); gwb_basis_ring_rows and gwb_basis_ring_sync_ints size W and sync for the current one. */
 GWB_API int gwb_basis_ring_set_config(int pc, int nslot, int look);
+/* The present configuration (three ints out). */
+GWB_API int gwb_basis_ring_get_config(int* pc, int* nslot, int* look);
 GWB_API int gwb_basis_ring_rows(void);
 GWB_API int gwb_basis_ring_sync_ints(int rows);
 GWB_API int gwb_basis_fused_ring(const float* Vp, long long ldvp, int rows, const float* Dp, long long N,
