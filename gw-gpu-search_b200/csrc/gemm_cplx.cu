@@ -34,7 +34,7 @@ struct __align__(64) CplxArgs {
     const float* rowscale;   // form 3: per-row scale of A (V is multiplied by its square); else null
     long long ldv;
     long long Tn;
-    int M, Kh, ntiles, group, nout, stages, MB, KC;
+    int M, Kh, ntiles, group, nout, stages, KC;
     // split bf16 with Kh > 128: A hi resident, A lo streamed with the Z ring (16 K rows per stage, 32-byte swizzle)
     int lo_stream;
     int order;   // CTA-pair kernel: order of the complex products' MMAs (0-3, see the kernel)
@@ -70,10 +70,10 @@ struct Layout {
     uint32_t a_tiles, a_bytes, z_off, stage_bytes, x_off, bar_off, total;
 };
 
-__host__ __device__ inline Layout layout_of(int nha, int nhz, int MB, int Kh, int KC, int stages, int rowel = 64) {
+__host__ __device__ inline Layout layout_of(int nha, int nhz, int Kh, int KC, int stages, int rowel = 64) {
     Layout L;
     L.a_tiles = (uint32_t)((2 * Kh + rowel - 1) / rowel);
-    L.a_bytes = (uint32_t)MB * nha * L.a_tiles * kATile;
+    L.a_bytes = (uint32_t)nha * L.a_tiles * kATile;
     L.z_off = L.a_bytes;
     // (re, im) x (hi, lo) x the 128-sample tile as 128-byte rows (two 64-sample halves for 16-bit, one for 8-bit)
     L.stage_bytes = 2u * nhz * (uint32_t)(128 / rowel) * (uint32_t)KC * 128u;
@@ -103,10 +103,10 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
     using C = Cfg<FORM>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    const int Kh = args.Kh, KC = args.KC, S = args.stages, MB = args.MB;
-    const bool los = C::SPLIT_A && args.lo_stream != 0;   // A lo streamed (MB = 1, KC = 16 or 32)
+    const int Kh = args.Kh, KC = args.KC, S = args.stages;
+    const bool los = C::SPLIT_A && args.lo_stream != 0;   // A lo streamed (KC = 16 or 32)
     const int nres = los ? 1 : C::NHA;                    // resident copies of A
-    const Layout L = los ? layout_split_stream(Kh, KC, S, C::NHZ) : layout_of(C::NHA, C::NHZ, MB, Kh, KC, S, C::ROWEL);
+    const Layout L = los ? layout_split_stream(Kh, KC, S, C::NHZ) : layout_of(C::NHA, C::NHZ, Kh, KC, S, C::ROWEL);
     const uint32_t zst_bytes = 2u * C::NHZ * C::HALVES * (uint32_t)KC * 128u;   // the Z part of a stage
     const int nkc = (Kh + KC - 1) / KC;
     uint8_t* sA = smem;
@@ -124,8 +124,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
-    const int m0 = blockIdx.y * 128 * MB;
-    const int MBe = min(MB, (args.M - m0 + 127) / 128);
+    const int m0 = blockIdx.y * 128;
     int t_begin, t_end;
     if (args.pv) {
         t_begin = (int)((long long)blockIdx.x * args.ntiles / gridDim.x);
@@ -137,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
         t_end = (int)min(o1 * (long long)args.group, (long long)args.ntiles);
     }
     const int ntl = t_end - t_begin;
-    if (ntl <= 0 || MBe <= 0) return;
+    if (ntl <= 0) return;
     const int nfill = ntl * nkc;   // Z stages consumed by this CTA
 
     if (threadIdx.x == 0) {
@@ -167,12 +166,10 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
         if (lane == 0) {
             for (int h = 0; h < C::NHA; ++h) prefetch_tmap(&args.tA[h]);
             for (int h = 0; h < C::NHZ; ++h) prefetch_tmap(&args.tZ[h]);
-            mbar_arrive_expect_tx(barA, (uint32_t)(MBe * nres * L.a_tiles * kATile));
-            for (int mb = 0; mb < MBe; ++mb)
-                for (int h = 0; h < nres; ++h)
-                    for (int a = 0; a < (int)L.a_tiles; ++a)
-                        tma_load_2d(sA + ((mb * nres + h) * L.a_tiles + a) * kATile, &args.tA[h], barA,
-                                    a * C::ROWEL, m0 + mb * 128);
+            mbar_arrive_expect_tx(barA, (uint32_t)(nres * L.a_tiles * kATile));
+            for (int h = 0; h < nres; ++h)
+                for (int a = 0; a < (int)L.a_tiles; ++a)
+                    tma_load_2d(sA + (h * L.a_tiles + a) * kATile, &args.tA[h], barA, a * C::ROWEL, m0);
             for (int f = 0; f < nfill; ++f) {
                 const int s = f % S;
                 const uint32_t n = (uint32_t)(f / S);
@@ -217,20 +214,19 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                 *abort_flag = 1;
             }
             tc_fence_after();
-            // the MMAs of one item (M block mb) on one Z chunk. One-product forms: every descriptor of the chunk is
+            // the MMAs of one item on one Z chunk. One-product forms: every descriptor of the chunk is
             // formed first (base descriptors plus offsets), then the MMAs go out back to back in the same order (sk,
             // four real products), so the one issuing thread spends no address arithmetic between them (measured
             // 0.266 -> 0.253 ms at n = 256, r = 128, fp16). The split form keeps descriptors and MMAs interleaved (the
             // burst measured slower there: one K step per chunk when A lo is streamed).
-            auto issue = [&](int kc, int mb, int b, uint32_t st) {
+            auto issue = [&](int kc, int b, uint32_t st) {
                 if constexpr (C::NPROD == 1) {
                     constexpr int MAXS = 4;                      // K steps per chunk: KC / KSTEP (64/16, 128/32)
                     const uint32_t dre = tm + (uint32_t)(b * 256), dim = dre + 128;
                     const int nsteps = min(KC, Kh - kc * KC) / C::KSTEP;
-                    const uint32_t abase = a_base + mb * L.a_tiles * kATile;
                     // base descriptors of the chunk plus byte offsets >> 4 (the start-address field, bits 0-13;
                     // shared-memory addresses stay below 2^18, so it does not carry)
-                    const uint64_t ad = smem_desc(abase, 16, 1024, 2);
+                    const uint64_t ad = smem_desc(a_base, 16, 1024, 2);
                     const uint64_t zd = smem_desc(st, (uint32_t)KC * 128u, 1024, 2);
                     uint64_t dAre[MAXS], dAim[MAXS], dZre[MAXS], dZim[MAXS];
 #pragma unroll
@@ -268,7 +264,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                         const int k = kc * KC + sk * C::KSTEP;
                         for (int pr = 0; pr < C::NPROD; ++pr) {
                             const int ha = C::ha(pr), hz = C::hz(pr);
-                            const uint32_t abase = a_base + (mb * nres + ha) * L.a_tiles * kATile;
+                            const uint32_t abase = a_base + ha * L.a_tiles * kATile;
                             const uint32_t are = abase + (k / C::ROWEL) * kATile + (k % C::ROWEL) * C::ES;
                             const uint32_t aim = abase + ((Kh + k) / C::ROWEL) * kATile + ((Kh + k) % C::ROWEL) * C::ES;
                             // K step = KSTEP rows of 128 bytes (2048 bytes for 16-bit, 4096 for 8-bit)
@@ -311,9 +307,9 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                 }
             };
             // this item's accumulators must have been read out by the epilogue
-            auto wait_tempty = [&](int i, int j) {
-                const uint32_t u = (uint32_t)(j >> 1);
-                if (!mbar_wait_warp(&tempty[j & 1], (u & 1) ^ 1)) {
+            auto wait_tempty = [&](int i) {
+                const uint32_t u = (uint32_t)(i >> 1);
+                if (!mbar_wait_warp(&tempty[i & 1], (u & 1) ^ 1)) {
                     record_error(args.err, GWB_ERR_TIMEOUT, 204, blockIdx.x, i);
                     *abort_flag = 1;
                     return false;
@@ -330,37 +326,15 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                 tc_fence_after();
                 return true;
             };
-            // Two M blocks: when the Z ring holds a whole tile, M block 0 runs through all chunks before M block 1,
-            // so block 0's MMAs overlap the epilogue of the previous tile's block 1 and block 1's the epilogue of
-            // this tile's block 0. Otherwise both blocks go chunk by chunk.
-            const bool mb_outer = MBe == 2 && S >= nkc;
             for (int i = 0; i < ntl && ok; ++i) {
-                if (mb_outer) {
-                    for (int mb = 0; mb < MBe && ok; ++mb) {
-                        const int j = i * MBe + mb;
-                        for (int kc = 0; kc < nkc && ok; ++kc) {
-                            const int f = i * nkc + kc;
-                            if (mb == 0 && !(ok = wait_full(f))) break;
-                            if (kc == 0 && !(ok = wait_tempty(i, j))) break;
-                            issue(kc, mb, j & 1, z_base + (f % S) * L.stage_bytes);
-                            if (mb == MBe - 1 && el) umma_commit(&empty[f % S]);
-                        }
-                        if (ok && el) umma_commit(&tfull[j & 1]);
-                    }
-                } else {
-                    for (int kc = 0; kc < nkc && ok; ++kc) {
-                        const int f = i * nkc + kc;
-                        if (!(ok = wait_full(f))) break;
-                        for (int mb = 0; mb < MBe && ok; ++mb) {
-                            const int j = i * MBe + mb;
-                            if (kc == 0 && !(ok = wait_tempty(i, j))) break;
-                            issue(kc, mb, j & 1, z_base + (f % S) * L.stage_bytes);
-                        }
-                        if (el) umma_commit(&empty[f % S]);
-                    }
-                    if (ok && el)
-                        for (int mb = 0; mb < MBe; ++mb) umma_commit(&tfull[(i * MBe + mb) & 1]);
+                for (int kc = 0; kc < nkc && ok; ++kc) {
+                    const int f = i * nkc + kc;
+                    if (!(ok = wait_full(f))) break;
+                    if (kc == 0 && !(ok = wait_tempty(i))) break;
+                    issue(kc, i & 1, z_base + (f % S) * L.stage_bytes);
+                    if (el) umma_commit(&empty[f % S]);
                 }
+                if (ok && el) umma_commit(&tfull[i & 1]);
             }
             __syncwarp();
             if (el) umma_commit(done);
@@ -369,10 +343,9 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
         }
         __syncwarp();
     } else {
-        // two groups of four warps: group g takes the items of accumulator buffer g (with two M blocks, always M block
-        // g), so a group has two items' time for one, and with one M block the two meet once per output window, not per
-        // tile (all eight warps on every tile, halves merged across a barrier: the C2 step's fp16 launches 793 ms, now
-        // 697; split bf16 1,342, now 1,318)
+        // two groups of four warps: group g takes the items of accumulator buffer g, so a group has two items' time for one,
+        // and the two meet once per output window, not per tile (all eight warps on every tile, halves merged across a
+        // barrier: the C2 step's fp16 launches 793 ms, now 697; split bf16 1,342, now 1,318)
         const int q = warp & 3, g = (warp - 2) >> 2;
         const int rl = 32 * q + lane;
         const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(g * 256);
@@ -416,9 +389,9 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
             }
             bi += t * kTile;
         };
-        // the maximum of the part of window o that this CTA's range holds, of M block mb
-        auto put = [&](int o, int mb, float wb, int wi) {
-            const int row = m0 + mb * 128 + rl;
+        // the maximum of the part of window o that this CTA's range holds
+        auto put = [&](int o, float wb, int wi) {
+            const int row = m0 + rl;
             if (row >= args.M) return;
             const int w0 = o * G;
             const int w1 = (int)min((long long)w0 + G, (long long)args.ntiles);
@@ -436,60 +409,41 @@ __global__ void __launch_bounds__(kThreads, 1) umma_cplx_kernel(const __grid_con
                 args.I[(long long)row * args.ldv + o] = wi;
             }
         };
-        float wb = -2.f;                                   // below any tile's maximum (at least -1)
-        int wi = 0;
-        if (MBe == 2) {
-            for (int i = 0; i < ntl; ++i) {
-                const int t = t_begin + i;
+        int par = 0;
+        for (int t = t_begin; t < t_end;) {
+            const int o = t / G, ts = t, te = (int)min((long long)(o + 1) * G, (long long)t_end);
+            float wb = -2.f;                               // below any tile's maximum (at least -1)
+            int wi = 0;
+            for (; t < te; ++t) {
+                const int i = t - t_begin;
+                if ((i & 1) != g) continue;
                 float best;
                 int bi;
-                item(2 * i + g, t, best, bi);
+                item(i, t, best, bi);
                 if (best > wb) {
                     wb = best;
                     wi = bi;
                 }
-                if ((t + 1) % G == 0 || t + 1 == t_end) {
-                    put(t / G, g, wb, wi);
-                    wb = -2.f;
-                }
             }
-        } else {
-            int par = 0;
-            for (int t = t_begin; t < t_end;) {
-                const int o = t / G, ts = t, te = (int)min((long long)(o + 1) * G, (long long)t_end);
-                wb = -2.f;
-                wi = 0;
-                for (; t < te; ++t) {
-                    const int i = t - t_begin;
-                    if ((i & 1) != g) continue;
-                    float best;
-                    int bi;
-                    item(i, t, best, bi);
-                    if (best > wb) {
-                        wb = best;
-                        wi = bi;
-                    }
-                }
-                if (te - ts == 1) {                        // one tile: its group has the maximum
-                    if (((ts - t_begin) & 1) == g) put(o, 0, wb, wi);
-                    continue;
-                }
-                if (g == 1) {
-                    xv[par * 128 + rl] = wb;
-                    xi[par * 128 + rl] = wi;
-                }
-                named_bar_sync(1, 32 * kEpiWarps);         // the slots take turns: written again two outputs on
-                if (g == 0) {
-                    const float ob = xv[par * 128 + rl];
-                    const int oi = xi[par * 128 + rl];
-                    if (ob > wb || (ob == wb && oi < wi)) {
-                        wb = ob;
-                        wi = oi;
-                    }
-                    put(o, 0, wb, wi);
-                }
-                par ^= 1;
+            if (te - ts == 1) {                        // one tile: its group has the maximum
+                if (((ts - t_begin) & 1) == g) put(o, wb, wi);
+                continue;
             }
+            if (g == 1) {
+                xv[par * 128 + rl] = wb;
+                xi[par * 128 + rl] = wi;
+            }
+            named_bar_sync(1, 32 * kEpiWarps);         // the slots take turns: written again two outputs on
+            if (g == 0) {
+                const float ob = xv[par * 128 + rl];
+                const int oi = xi[par * 128 + rl];
+                if (ob > wb || (ob == wb && oi < wi)) {
+                    wb = ob;
+                    wi = oi;
+                }
+                put(o, wb, wi);
+            }
+            par ^= 1;
         }
     }
     __syncthreads();
@@ -849,7 +803,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
             bi += t * kTile;
         };
-        auto put = [&](int o, int, float wb, int wi) {
+        auto put = [&](int o, float wb, int wi) {
             const int row = m0 + rl;
             if (row >= args.M) return;
             const int w0 = o * G;
@@ -883,7 +837,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     }
                 }
                 if (te - ts == 1) {                        // one tile: its group has the maximum
-                    if (((ts - t_begin) & 1) == g) put(o, 0, wb, wi);
+                    if (((ts - t_begin) & 1) == g) put(o, wb, wi);
                     continue;
                 }
                 if (g == 1) {
@@ -898,7 +852,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                         wb = ob;
                         wi = oi;
                     }
-                    put(o, 0, wb, wi);
+                    put(o, wb, wi);
                 }
                 par ^= 1;
             }
@@ -1059,7 +1013,6 @@ int launch_pair(CplxArgs args, const void* const* A, const void* const* Zp, long
                   work_bytes, 16ll * M * gx);
     args.stages = stages;
     args.KC = KC;
-    args.MB = 1;
     args.pv = static_cast<float*>(work);
     args.pi = reinterpret_cast<int32_t*>(static_cast<char*>(work) + 8ll * M * gx);
     const uint32_t smem = layout_pair(args.Kh, KC, stages, los ? 1 : C::NHA, C::NHZ, los).total + 1024;
@@ -1118,20 +1071,11 @@ int launch_cplx(const void* const* A, const void* const* Zp, long long lda, long
     GWB_CHECK_ARG(ldv >= nout, GWB_ERR_SHAPE, "fused_peaks_cplx: ldv=%lld < outputs per row %lld", ldv, nout);
     const uint32_t max_smem = 227 * 1024;
     int KC = FORM == 2 ? 32 : (C::F8 ? 128 : 64);          // K rows per Z stage (32 KB per stage in every form)
-    auto fits = [&](int mb, int st) {
-        return layout_of(C::NHA, C::NHZ, mb, Kh, KC, st, C::ROWEL).total + 1024 <= max_smem;
-    };
-    auto most_stages = [&](int mb) {
-        int st = 6;
-        while (st > 0 && !fits(mb, st)) --st;
-        return st;
-    };
-    // one M block per CTA: measured faster than two per CTA sharing each Z tile (0.285 vs 0.292 ms at n = 256, Kh =
-    // 128, Tn = 917,504; the second M group's Z reads hit L2), with the TMEM double buffer spanning tiles. The kernel
-    // also runs two M blocks per CTA (each Z tile read once for both) when MB = 2.
-    const int MB = 1;
+    // one M block per CTA (two that shared each Z tile were no faster: the second M group's Z reads hit L2), with the TMEM
+    // double buffer spanning tiles
     const GemmTune tune = gemm_tune(FORM, Kh, M, work_bytes >= 16ll * M * std::max(1, num_sms() / (int)cdiv(M, 128)));
-    int stages = most_stages(MB);
+    int stages = 6;
+    while (stages > 0 && layout_of(C::NHA, C::NHZ, Kh, KC, stages, C::ROWEL).total + 1024 > max_smem) --stages;
     if (tune.stages >= 2 && stages >= 2) stages = std::min(stages, tune.stages);
     // split A beyond Kh = 128: A hi + lo no longer fit beside the Z ring, so A lo is streamed with it
     const bool los = C::SPLIT_A && stages < 2;
@@ -1180,12 +1124,11 @@ int launch_cplx(const void* const* A, const void* const* Zp, long long lda, long
     args.group = group;
     args.nout = (int)nout;
     args.stages = stages;
-    args.MB = MB;
     args.KC = KC;
     args.lo_stream = los ? 1 : 0;
     args.err = device_error_ptr();
     const uint32_t smem = (los ? layout_split_stream(Kh, KC, stages, C::NHZ)
-                               : layout_of(C::NHA, C::NHZ, MB, Kh, KC, stages, C::ROWEL)).total + 1024;
+                               : layout_of(C::NHA, C::NHZ, Kh, KC, stages, C::ROWEL)).total + 1024;
     auto kern = umma_cplx_kernel<FORM>;
     GWB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if constexpr (!C::F8) {
@@ -1193,7 +1136,7 @@ int launch_cplx(const void* const* A, const void* const* Zp, long long lda, long
             return launch_pair<FORM>(args, A, Zp, lda, ldz, M, ntiles, nout, group, V, I, ldv, work, work_bytes, tune,
                                      stream);
     }
-    const int mgroups = (M + 128 * MB - 1) / (128 * MB);
+    const int mgroups = (M + 127) / 128;
     const long long per = (long long)std::max(1, num_sms() / mgroups);
     // with a workspace the CTA ranges are tile-granular (balanced to one tile; split windows merged afterwards),
     // without one they are whole windows (up to one window of imbalance)
