@@ -1,9 +1,11 @@
 // Plain-fp32 form of the reconstruction GEMM with fused |z|^2 and blocked argmax, on the fp32 pipe.
 //
 // Same contract as gwb_fused_peaks_f16 (pipeline/fp_gemm.py:14-44 semantics) with fp32 operands: the reference only
-// has an fp16 GEMM, so this is the full-precision form that the mixed forms are compared against. CTA = 128 template
-// rows x one output group of `group` 128-sample blocks, walked block by block; 256 threads as 16 x 16, each thread
-// owning 8 rows x 8 samples for re and im (128 accumulators). K is staged through shared memory 16 at a time.
+// has an fp16 GEMM, so this is the full-precision form that the mixed forms are compared against. Two kernels with the same
+// sums: simt_absmax_packed_kernel, which runs (64 template rows x part of an output group of `group` 128-sample blocks per
+// CTA of 128 threads, paired FMAs, asynchronous copies), and simt_absmax_kernel, which runs where gwb_f32_set_async(0) asks
+// for it or there are more than 65,535 blocks of 64 rows (128 rows x one output group per CTA of 256 threads as 16 x 16).
+// In both a thread owns 8 rows x 8 samples for re and im, and K is staged through shared memory 16 at a time.
 #include <cooperative_groups.h>
 
 #include <atomic>

@@ -125,10 +125,10 @@ __global__ void __launch_bounds__(kT, P2 > 32 ? 2 : 3) welch_median_kernel(const
     }
 }
 
+// Mean of up to MAXN frames, or the median of 65 to 256 (up to 64 welch_median_kernel takes it, past 256 the one below)
 template <int MAXN>
 __global__ void welch_avg_kernel(const float2* __restrict__ X, long long ldx, int rows, int nfr, int nbin, float dt,
-                                 int median, float bias32, double bias64, int wide, float fac, float* __restrict__ psd,
-                                 long long ldp) {
+                                 int median, float bias32, float fac, float* __restrict__ psd, long long ldp) {
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= (long long)rows * nbin) return;
     const int r = (int)(e / nbin), k = (int)(e % nbin);
@@ -141,7 +141,7 @@ __global__ void welch_avg_kernel(const float2* __restrict__ X, long long ldx, in
         v[s] = p;
     }
     float q;
-    if (median) {
+    if (MAXN > 64 && median) {
         for (int i = 1; i < nfr; ++i) {   // insertion sort, nfr is small
             const float t = v[i];
             int j = i - 1;
@@ -152,10 +152,6 @@ __global__ void welch_avg_kernel(const float2* __restrict__ X, long long ldx, in
             v[j + 1] = t;
         }
         q = (nfr & 1) ? v[nfr / 2] : __fdiv_rn(__fadd_rn(v[nfr / 2 - 1], v[nfr / 2]), 2.f);
-        if (wide) {
-            psd[(long long)r * ldp + k] = (float)(((double)q / bias64) * (double)fac);
-            return;
-        }
         q = __fdiv_rn(q, bias32);
     } else {
         float s = 0.f;
@@ -465,11 +461,9 @@ int gwb_welch_avg(const float* X, long long ldx, int rows, int nfr, int nbin, fl
         return GWB_OK;
     }
     if (nfr <= 64)
-        welch_avg_kernel<64><<<blocks_for(n), kT, 0, s>>>(x2, ldx, rows, nfr, nbin, dt, median, (float)bias, bias, wide,
-                                                          fac, psd, ldp);
+        welch_avg_kernel<64><<<blocks_for(n), kT, 0, s>>>(x2, ldx, rows, nfr, nbin, dt, median, (float)bias, fac, psd, ldp);
     else
-        welch_avg_kernel<256><<<blocks_for(n), kT, 0, s>>>(x2, ldx, rows, nfr, nbin, dt, median, (float)bias, bias, wide,
-                                                           fac, psd, ldp);
+        welch_avg_kernel<256><<<blocks_for(n), kT, 0, s>>>(x2, ldx, rows, nfr, nbin, dt, median, (float)bias, fac, psd, ldp);
     GWB_LAUNCH_CHECK("welch_avg_kernel");
     return GWB_OK;
 }

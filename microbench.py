@@ -90,9 +90,13 @@ def basis(a):
     Kh = fp_filter.kh_of(r, a.form)
     Z = torch.zeros((2 * Kh, Tn), dtype=fp_filter._z_dtype(a.form), device='cuda')
     Zlo = torch.zeros_like(Z) if a.form == 'bf16x3' else None
-    Dp = fp_filter.fourstep_order(D, tlen, isw)
+    kend = a.kend or flen
+    Vh[:, kend:] = 0
+    bad = torch.empty(1, dtype=torch.int32, device='cuda')
+    Dp = fp_filter.fourstep_order(D, tlen, isw, last_bad=bad)
     Vp = fp_filter.fourstep_order(Vh, tlen)
-    out = dict(kernel='basis_series', form=a.form, r=r, tlen=tlen)
+    band = dict(kend=kend, last_bad=bad) if a.kend else {}
+    out = dict(kernel='basis_series', form=a.form, r=r, tlen=tlen, kend=kend)
     if a.form != 'fp8':            # the cuFFT path has no fp8 pack
         ms = _time(lambda: fp_filter.basis_series_into(ws, Vh, D, isw, a0, Tn, Z, Zlo, a.form, im_off=Kh), a.reps)
         out.update(ms_cufft_path=ms, us_per_row_cufft=ms * 1e3 / r)
@@ -105,11 +109,12 @@ def basis(a):
         _lib.call('gwb_basis_set_pass2_pairs', pairs)
         for wr in [int(x) for x in a.wrows.split(',')]:
             fws = fp_filter.FusedBasisWorkspace(tlen, flen, r, wrows=wr or None, ring=False)
-            msf = _time(lambda: fp_filter.basis_series_fused(fws, Vp, Dp, a0, Tn, Z, Zlo, a.form, im_off=Kh), a.reps)
+            msf = _time(lambda: fp_filter.basis_series_fused(fws, Vp, Dp, a0, Tn, Z, Zlo, a.form, im_off=Kh, **band),
+                        a.reps)
             tag = f'w{fws.wrows}_c{cols}' + ('' if pairs else '_unpaired')
             # HBM bytes of the fused form when W stays in L2: Vh read and Z written (D isw stays in L2)
             out['us_per_row_fused_' + tag] = msf * 1e3 / r
-            out['hbm_gbs_' + tag] = r * (8 * flen + zb) / msf / 1e6
+            out['hbm_gbs_' + tag] = r * (8 * min(kend, flen) + zb) / msf / 1e6
             got = [Z.clone()] + ([Zlo.clone()] if Zlo is not None else [])
             if first is None:
                 first = got
@@ -579,6 +584,8 @@ def main():
     ap.add_argument('--groups', type=int, default=512)
     ap.add_argument('--peaks', type=int, default=1)
     ap.add_argument('--reps', type=int, default=10)
+    ap.add_argument('--kend', type=int, default=0,
+                    help='basis: filters zero from this bin on, and the first pass told so (0: full band)')
     ap.add_argument('--wrows', default='0', help='basis: comma list of W row batches (0: all rows at once)')
     ap.add_argument('--pass2-cols', default='16,8', help='basis: comma list of columns per pass-2 CTA (8, 16)')
     ap.add_argument('--pass2-pairs', default='1,0',
