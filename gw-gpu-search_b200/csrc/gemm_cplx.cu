@@ -906,16 +906,18 @@ __global__ void window_merge_kernel(int M, int ntiles, int group, int nout, int 
 
 // Launch configuration per (form, Kh) from the autotuner's table (gwb_gemm_set_config), else by size. Every choice here
 // gives the same bits. Times are ms at Tn = 917,504 (pair against one CTA per M block).
-// - A pair works on two M blocks, so an odd count pays for one of zeros. One block: one CTA (fp16 at Kh = 128 0.210
-//   against 0.139, split bf16 0.401 against 0.303, fp16 with split A 0.288 against 0.198). Three or five blocks: one CTA
-//   as long as it is slower per block by less than the padding, which holds up to a product of blocks and Kh (three
-//   blocks, Kh = 128: fp16 0.404 / 0.378; split bf16 at 32 0.372 / 0.283 but at 64 0.438 / 0.462; fp16 with split A at 96
-//   0.478 / 0.457 but at 128 0.601 / 0.634).
-// - fp16 with split A on even counts: pairs from Kh = 64 on (two blocks: 0.217 / 0.218 at 64, 0.309 / 0.397 at 128,
-//   0.464 / 0.745 at 192; 0.186 / 0.179 at 32).
-// - Order of the split forms' pairs (1: K chunks of 64): split bf16 order 1 where A lo stays resident (Kh = 64: 0.272 ->
-//   0.238) and from 192 on (equal), between them order 0, whose chunks of 32 leave more stages beside the streamed A lo
-//   (Kh = 144: 0.672 -> 0.550, 160: 0.611 -> 0.544); fp16 with split A order 1 up to 160 (0.415 -> 0.397 there).
+// - A pair reads Z once for two M blocks and keeps the tensor pipe fuller on long tiles; a CTA per block has no partner to
+//   wait for at every chunk and pays for no block of zeros where their count is odd. One block: one CTA (fp16 at Kh = 128
+//   0.216 against 0.120, split bf16 0.440 / 0.302, fp16 with split A 0.291 / 0.183). Even counts: one CTA up to a Kh (two and
+//   eight blocks: fp16 0.203 / 0.181 and 0.750 / 0.682 at 96, 0.221 / 0.219 and 0.888 / 0.871 at 128, six blocks 0.626 /
+//   0.654; split bf16 0.226 / 0.190 and 0.693 / 0.576 at 32, 0.243 / 0.298 and 0.912 / 1.184 at 64; fp16 with split A 0.228 /
+//   0.199 and 0.751 / 0.717 at 64, 0.263 / 0.272 and 1.030 / 1.166 at 96). Odd counts: as long as the padding costs more
+//   (fp16, three and nine blocks, 0.584 / 0.468 and 1.559 / 1.432 at 192; split bf16, three, 0.430 / 0.402 at 64, 0.605 /
+//   0.643 at 96, five and nine 0.734 / 0.776 and 1.141 / 1.276 at 64, nine 0.868 / 0.634 at 32; fp16 with split A, three and
+//   five, 0.598 / 0.545 and 0.969 / 0.897 at 128, three 0.707 / 0.745 at 144, nine 1.540 / 1.688 at 128).
+// - Order of the split forms' pairs (1: K chunks of 64): split bf16 order 1 where A lo stays resident (Kh = 64: 0.265 ->
+//   0.243) and from 192 on (equal), between them order 0, whose chunks of 32 leave more stages beside the streamed A lo
+//   (Kh = 144: 0.670 -> 0.555, 160: 0.675 -> 0.582); fp16 with split A order 1 up to 160 (0.378 -> 0.360 at 144).
 struct GemmTune {
     int form, kh, pair, stages, order;
 };
@@ -925,8 +927,9 @@ GemmTune gemm_tune(int form, int kh, int M, bool one_ok) {
     GemmTune t{form, kh, 1, 0, 0};
     if (tune_lookup(form, kh, &t.pair, &t.stages, &t.order)) return t;
     const int blocks = (M + 127) / 128;
-    const int padding_pays = form == 2 ? 96 : form == 6 ? 320 : 384;
-    const bool one = blocks == 1 || (blocks % 2 == 1 && (long long)blocks * kh <= padding_pays) || (form == 6 && kh < 64);
+    const int even = form == 2 ? 32 : form == 6 ? 64 : 112;
+    const int odd = form == 2 ? std::max(32, 192 / blocks) : form == 6 ? std::max(64, std::min(128, 640 / blocks)) : 192;
+    const bool one = blocks == 1 || kh <= (blocks % 2 ? odd : even);
     t.pair = one && one_ok ? 0 : 1;
     if (t.pair) t.order = form == 2 ? (kh <= 128 || kh >= 192) : form == 6 ? kh <= 160 : 0;
     return t;
