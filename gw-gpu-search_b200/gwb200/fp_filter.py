@@ -140,12 +140,20 @@ _TWIDDLES = {}
 
 
 def twiddles(N, device='cuda'):
-    """e^{2 pi i m / N}, m < N, complex64 on the device (cached per (N, device))."""
-    key = (int(N), str(torch.device(device)))
+    """e^{2 pi i m / N}, m < N, complex64 on the device (cached per (N, device index); complete before any other stream or
+    thread can take it from the cache)."""
+    d = torch.device(device)
+    if d.type != 'cuda':
+        raise ValueError('twiddles are made on a CUDA device, not on %s' % d)
+    key = (int(N), torch.cuda.current_device() if d.index is None else d.index)
     t = _TWIDDLES.get(key)
     if t is None:
-        t = torch.empty(N, dtype=torch.complex64, device=device)
-        _lib.call('gwb_fft_twiddles', int(N), _lib.ptr(t), _lib.stream_ptr(t.device))
+        with torch.cuda.device(key[1]):
+            t = torch.empty(N, dtype=torch.complex64, device='cuda')
+            _lib.call('gwb_fft_twiddles', int(N), _lib.ptr(t), _lib.stream_ptr(t.device))
+            if torch.cuda.is_current_stream_capturing():
+                return t                    # filled by the graph alone: not for others
+            torch.cuda.current_stream().synchronize()
         _TWIDDLES[key] = t
     return t
 
@@ -330,7 +338,8 @@ def make_closures(kmin, flen, tlen, sw, eps_b, dev='cuda', form='f16'):
     object with svd_tile(H), basis_series(Vh, Dws, a0, Tn) and stacked_A(A, nrm_s, scale, Kp), same arguments and
     results as the reference (CUDA tensors; scale a Python float, as the reference returns)."""
     # the fused passes where the length allows, else premul + cuFFT + pack
-    fused = FUSED_MIN <= tlen <= FUSED_MAX and tlen & (tlen - 1) == 0 and flen <= tlen // 2 + 1 and form != 'fp8'
+    fused = (FUSED_MIN <= tlen <= FUSED_MAX and tlen & (tlen - 1) == 0 and flen <= tlen // 2 + 1 and form != 'fp8' and
+             torch.device(dev).type == 'cuda')
     ws = SeriesWorkspace(tlen, flen, RB, dev) if fused else BasisWorkspace(tlen, flen, RB, dev)
 
     def _svd_tile(H):
