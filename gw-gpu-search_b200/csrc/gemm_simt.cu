@@ -422,6 +422,7 @@ extern "C" int gwb_fused_peaks_f32(const float* Are, const float* Aim, long long
     const long long nout = cdiv(ntiles, group);
     GWB_CHECK_ARG(ldv >= nout, GWB_ERR_SHAPE, "fused_peaks_f32: ldv=%lld < outputs per row %lld", ldv, nout);
     GWB_CHECK_ARG(nout < (1ll << 31), GWB_ERR_SHAPE, "fused_peaks_f32: too many outputs");
+    group = (int)std::min<long long>(group, ntiles);        // one output at most: the kernels' sums of it stay in range
     if (g_f32_async.load() && cdiv(M, AS_BM) <= 65535) {
         const bool vec = ldz % 4 == 0 && aligned(Z, 16);        // 16-byte copies of Z
         // windows are shared out over clusters while whole windows would leave the last of few waves nearly empty
