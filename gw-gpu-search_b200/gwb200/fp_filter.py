@@ -51,7 +51,7 @@ def sigma2(H, IPall, df, kmin=0):
     _lib.require_cuda(H, IPall)
     n, flen = H.shape
     nseg = IPall.shape[0]
-    part_elems = _lib.load().gwb_sigma2_part_elems(n, nseg)
+    part_elems = max(0, _lib.load().gwb_sigma2_part_elems(n, nseg))     # (an empty shape is refused by the call)
     part = torch.empty(part_elems, dtype=torch.float64, device=H.device)
     sig = torch.empty((n, nseg), dtype=torch.float64, device=H.device)
     _lib.call('gwb_sigma2', _lib.ptr(H), H.stride(0), n, _lib.ptr(IPall), _lib.row_stride(IPall), nseg, int(kmin), flen,
