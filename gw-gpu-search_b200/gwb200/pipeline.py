@@ -122,15 +122,16 @@ class MatchedFilter:
             bt = self.tuning['basis']['best'] if self.tuning and self.tuning['basis'] else {}
             self.fws = fp_filter.FusedBasisWorkspace(tlen, bank.flen, rmax, device, wrows=bt.get('wrows'),
                                                      ring=bt.get('ring'))
-            # basis filters in the four-step order of the transform, once per tile; D isw per step (order_data)
-            # and, read from the filters themselves, the bin from which each tile's are zero (its last f_ISCO)
-            ends = torch.empty(len(bank.svd), dtype=torch.int32, device=device)
-            self.vp = [fp_filter.fourstep_order(s['Vh'], tlen, last_nz=ends[t:t + 1]) for t, s in enumerate(bank.svd)]
-            self.kend = [int(e) + 1 for e in ends.cpu()]
-            # and where each tile's templates end, for the norms of a step
+            # where each tile's templates end, for the norms of a step
             self.ends = fp_filter.row_ends(bank.H)
             for r0, ids in zip(bank.row0, bank.tiles):
                 self.ends[r0:r0 + len(ids)] = self.ends[r0:r0 + len(ids)].max()
+            # basis filters in the four-step order of the transform, once per tile; D isw per step (order_data)
+            # and, read from the filters themselves, the bin from which each tile's are zero (its last f_ISCO). The copy
+            # waits for all of these, so that a step may run on any stream
+            ends = torch.empty(len(bank.svd), dtype=torch.int32, device=device)
+            self.vp = [fp_filter.fourstep_order(s['Vh'], tlen, last_nz=ends[t:t + 1]) for t, s in enumerate(bank.svd)]
+            self.kend = [int(e) + 1 for e in ends.cpu()]
             self._Dp = self._last_bad = None
             self._paired = False                # _last_bad is of the data in _Dp
         else:
