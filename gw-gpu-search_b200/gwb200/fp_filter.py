@@ -220,7 +220,8 @@ class FusedBasisWorkspace:
 def basis_series_fused(ws, Vp, Dp, a0, Tn, Z, Zlo=None, form='f16', im_off=None, kend=None, last_bad=None):
     """Same Z as basis_series_into in two fused passes (gwb_basis_fused), from the basis filters Vp (r, tlen/2 + 1) and
     one segment's D isw Dp (tlen/2 + 1,), both in four-step order (fourstep_order). The scale is the whole-series rms
-    of the first min(RB, wrows) rows by Parseval instead of the analysed-span rms (it cancels between Z and A).
+    of the first min(ws.nfirst, wrows) rows (two by default at 2^20, else RB; the ring's first chunk) by Parseval instead of
+    the analysed-span rms (it cancels between Z and A).
     Returns the device scale; for form 'fp8' Z row j holds z_j / ws.rowscale[j] in e4m3 instead. kend: Vp is zero from
     this bin on, with last_bad (device int32) the data's last non-finite bin (gwb_basis_fused_band)."""
     r = Vp.shape[0]
