@@ -15,6 +15,7 @@
 //
 // The phase metric (the quadratic form of the phase-maximised match, 1 - m ~ dtheta^T g dtheta / 2): with |h|
 // independent of theta, g_ij = Cov_w(dPhi/dtheta_i, dPhi/dtheta_j), w_k = |h_k|^2 IP_k; the phi_c row is zero.
+#include <cmath>
 #include "common.cuh"
 
 namespace gwb {
@@ -352,13 +353,13 @@ constexpr int kOut = 7 + 3 * kNP;
 // bin, in which 256 threads share the 20 to 200 bins of 16 s of data, and a dual-number phase with three exp and two pow
 // per frequency bin: 803 us for 2,048 triggers of 16 s, float32, now 159. (A CTA per trigger without the table 194, four
 // warps per trigger and four CTAs per SM 192, a warp per trigger 291: it waits for the longest band.) The float64 form's
-// more exact powers cost it 5%: 333 us a call for 2,048 triggers of 16 s, Mc 4 to 34, 316 with products of w and 1,372 with
+// more exact powers cost it 5%: 330 us a call for 2,048 triggers of 16 s, Mc 4 to 34, 316 with products of w and 1,372 with
 // the former kernel (float32 form 303, 304 and 1,320); divided and rooted by the library functions it took 385.
 template <typename T>
 __global__ void __launch_bounds__(kGT, 2) snr_grad_kernel(const double* __restrict__ params, int n,
                                                              const float2* __restrict__ D, long long ldd,
                                                              const float* __restrict__ IP, long long ldip, int flen,
-                                                             double df, int kmin, double f_ecc, int nb,
+                                                             double df, int kmin, double ecc0, int nb,
                                                              double* __restrict__ out, long long ldout) {
     constexpr int kNS = 2 * kNM;
     constexpr int kSeg = kMaxBins + kWarps;            // (warp, bin) runs: warp + bin never repeats along the band
@@ -381,7 +382,6 @@ __global__ void __launch_bounds__(kGT, 2) snr_grad_kernel(const double* __restri
     }
     __syncthreads();
     for (int k = tid; k < min(kTab, s_top - kmin); k += kGT) tab[k] = log_root<T>((double)(kmin + k) * df);
-    const double ecc0 = f_ecc * f_ecc * pow(f_ecc, 1.0 / 9.0);
     __syncthreads();
     for (int i = blockIdx.x; i < n; i += gridDim.x) {
         const double* th = params + (long long)i * kNP;
@@ -719,13 +719,14 @@ int gwb_snr_grad(const double* params, int n, const float* D, long long ldd, con
     const float2* d = reinterpret_cast<const float2*>(D);
     const int grid = std::min(n, 2 * num_sms());           // two CTAs per SM
     const size_t smem = kTab * sizeof(double2);
+    const double ecc0 = f_ecc * f_ecc * std::pow(f_ecc, 1.0 / 9.0);       // f_ecc^(19/9)
     GWB_CUDA(cudaFuncSetAttribute(fp64 ? snr_grad_kernel<double> : snr_grad_kernel<float>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (fp64)
-        snr_grad_kernel<double><<<grid, kGT, smem, s>>>(params, n, d, ldd, IP, ldip, flen, df, kmin, f_ecc, nbins,
+        snr_grad_kernel<double><<<grid, kGT, smem, s>>>(params, n, d, ldd, IP, ldip, flen, df, kmin, ecc0, nbins,
                                                         out, ldout);
     else
-        snr_grad_kernel<float><<<grid, kGT, smem, s>>>(params, n, d, ldd, IP, ldip, flen, df, kmin, f_ecc, nbins, out,
+        snr_grad_kernel<float><<<grid, kGT, smem, s>>>(params, n, d, ldd, IP, ldip, flen, df, kmin, ecc0, nbins, out,
                                                        ldout);
     GWB_LAUNCH_CHECK("snr_grad_kernel");
     return GWB_OK;
